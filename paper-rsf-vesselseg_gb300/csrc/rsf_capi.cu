@@ -458,6 +458,7 @@ StepConst make_const(const rsf_params *p, int k, const float *taps, rsf_dtype dt
     for (int i = 0; i < k; i++) sy = std::fma(sx, taps[i], sy);
     for (int i = 0; i < k; i++) s3 = std::fma(sy, taps[i], s3);
     c.s3 = s3;
+    rsf::set_pair_const(c.pk, c.eps, c.dt, c.nu, c.mu);
     c.gdelta = 0;
     return c;
 }

@@ -4,6 +4,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "rsf_pair.cuh"
+
 namespace rsf {
 
 constexpr int MAXK = 128;  // largest supported tap count (sigma up to ~18)
@@ -68,6 +70,7 @@ struct StepConst {
     int full_data;  // box or gauss: the z-pass stores the fits, the data factor of every voxel follows them
     float s3;       // gauss: the valid correlation of ones, K*1
     ptrdiff_t gdelta;  // gauss: offset (floats) of the scratch G from xb
+    PairConst pk;   // the packed arithmetic's constants
     const void *ymaps;  // per sub-volume TMA map of the y-pass pair planes (TMAP_BYTES each), or null
 };
 

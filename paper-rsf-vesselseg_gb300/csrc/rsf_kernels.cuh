@@ -28,10 +28,7 @@
 
 #include "rsf_arith.cuh"
 #include "rsf_internal.h"
-
-#ifndef RSF_F32X2
-#define RSF_F32X2 1
-#endif
+#include "rsf_pair.cuh"
 
 namespace rsf {
 
@@ -50,22 +47,6 @@ __device__ __forceinline__ int find_sv(const int *__restrict__ pre, int n, int b
 __device__ __forceinline__ float load_img(const void *img, size_t i, int f32) {
     return f32 ? __ldg(static_cast<const float *>(img) + i)
                : (float)__ldg(static_cast<const unsigned char *>(img) + i);
-}
-
-// d = a * b + c on both lanes, each rounded once (IEEE fma).
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-#if RSF_F32X2
-    unsigned long long ua, ub, uc, ud;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(ua) : "f"(a.x), "f"(a.y));
-    asm("mov.b64 %0, {%1, %2};" : "=l"(ub) : "f"(b.x), "f"(b.y));
-    asm("mov.b64 %0, {%1, %2};" : "=l"(uc) : "f"(c.x), "f"(c.y));
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(ud) : "l"(ua), "l"(ub), "l"(uc));
-    float2 d;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(ud));
-    return d;
-#else
-    return make_float2(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y));
-#endif
 }
 
 __device__ __forceinline__ float2 ld2(const float *p) { return __ldg(reinterpret_cast<const float2 *>(p)); }
@@ -253,7 +234,7 @@ __device__ __forceinline__ void cp_async8(float2 *smem_dst, const float *gsrc) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(gsrc) : "memory");
 }
-__device__ __forceinline__ void cp_async4(unsigned *smem_dst, const void *gsrc) {
+__device__ __forceinline__ void cp_async4(void *smem_dst, const void *gsrc) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(gsrc) : "memory");
 }
@@ -867,11 +848,6 @@ struct StencilCtx {
     bool need_x, need_y;
     ptrdiff_t xoff, yoff;   // offsets of the extra neighbour loads
     size_t col;
-    // fast path (stencil_step_f): rows of the y neighbours in the shared
-    // rings, and the x face rules of the thread's voxel
-    int urow, drow;         // phi rows above / below (Pb, ST_WARPS + 2 rows)
-    int gwl, gwr;           // gradient rows above / below (Gb)
-    bool xl_self, xr_self;  // the x - 1 / x + 1 neighbour is the voxel itself
 };
 
 // nx, gx, nz, gz of a plane (ny, gy live in the shared rows)
@@ -911,7 +887,7 @@ __device__ __forceinline__ float st_data(const StencilCtx &k, const StepConst &c
     return data_factor(e, e, c.l1, c.l2, c.lam_equal != 0);
 }
 
-template <int C, Arith A, bool DEBUG>
+template <int C, Arith A>
 __device__ __forceinline__ void stencil_step(const StencilCtx &k, const StepConst &c, StencilState &S, int rel,
                                              float (*Pb)[ST_WARPS + 2][32], float2 (*Gb)[ST_WARPS][32],
                                              unsigned *flag, const DebugOut &dbg) {
@@ -973,23 +949,21 @@ __device__ __forceinline__ void stencil_step(const StencilCtx &k, const StepCons
         const size_t vi = (size_t)sc * k.WH + k.col;
         k.phi_out[vi] = out;
         if (!isfinite(out)) atomicOr(flag, kFlagNonFinite);
-        if constexpr (DEBUG) {
-            const bool inside = k.inside_xy && sc >= k.r && sc < k.L - k.r;
-            if (!inside) {
-                dbg.f[0 * dbg.n + vi] = 1.0f;
-                dbg.f[1 * dbg.n + vi] = 1.0f;
-                if (!c.full_data) {  // else the data-term kernels wrote e everywhere
-                    const float I = load_img(k.s->img, vi, c.img_f32);
-                    const float d = __fsub_rn(I, 1.0f);
-                    dbg.f[2 * dbg.n + vi] = __fmul_rn(d, d);
-                    dbg.f[3 * dbg.n + vi] = __fmul_rn(d, d);
-                }
+        const bool inside = k.inside_xy && sc >= k.r && sc < k.L - k.r;
+        if (!inside) {
+            dbg.f[0 * dbg.n + vi] = 1.0f;
+            dbg.f[1 * dbg.n + vi] = 1.0f;
+            if (!c.full_data) {  // else the data-term kernels wrote e everywhere
+                const float I = load_img(k.s->img, vi, c.img_f32);
+                const float d = __fsub_rn(I, 1.0f);
+                dbg.f[2 * dbg.n + vi] = __fmul_rn(d, d);
+                dbg.f[3 * dbg.n + vi] = __fmul_rn(d, d);
             }
-            dbg.f[4 * dbg.n + vi] = dh;
-            dbg.f[5 * dbg.n + vi] = kap;
-            dbg.f[6 * dbg.n + vi] = lap;
-            dbg.f[7 * dbg.n + vi] = grad_mag(gc.gx, Gb[C][k.w][k.lane].y, gc.gz);
         }
+        dbg.f[4 * dbg.n + vi] = dh;
+        dbg.f[5 * dbg.n + vi] = kap;
+        dbg.f[6 * dbg.n + vi] = lap;
+        dbg.f[7 * dbg.n + vi] = grad_mag(gc.gx, Gb[C][k.w][k.lane].y, gc.gz);
     }
     S.P[C] = p3;    // plane rel+3
     S.EX[C] = exn;  // plane rel+3
@@ -1003,119 +977,6 @@ __device__ __forceinline__ float border_data(const unsigned char *ip, const Step
     const float d = __fsub_rn(I, 1.0f);
     const float e = __fmul_rn(d, d);
     return data_factor(e, e, c.l1, c.l2, c.lam_equal != 0);
-}
-
-// Fast step: the same arithmetic as stencil_step with every boundary rule
-// that depends on the thread's voxel decided once per thread (rows of the
-// y neighbours in the shared rings, x face flags) and phi, the output, the
-// data factor and the image read through pointers that advance one plane per
-// step.  The two extra rows of Pb hold the y neighbours of the halo rows.
-// In the reference boundary mode, lane 0 of a block at x = 0 carries the
-// previous linear element of lane 1's voxel, (W - 1, y - 1): its phi and its
-// normalised gradient reach lane 1 through the ordinary shuffles.
-// INSIDE: every output of the block lies in the valid region (blk_inside).
-// EDGE: the step may meet a z rule or an end of the block's plane range
-// (steps of the first and last groups of three, and groups near the first or
-// last plane of the volume); otherwise every plane test is known to pass.
-// FACE: the block touches an x or y face (per-thread rules apply).
-// acc collects out * 0, which is NaN once any output is not finite.
-template <int C, Arith A, bool INSIDE, bool EDGE, bool FACE>
-__device__ __forceinline__ void stencil_step_f(const StencilCtx &k, const StepConst &c, StencilState &S, int sc,
-                                               const float *&pp, float *&op, const float *&dp,
-                                               const unsigned char *&ip, float (*Pb)[ST_WARPS + 2][32],
-                                               float2 (*Gb)[ST_WARPS][32], float &acc) {
-    constexpr int C1 = (C + 1) % 3, C2 = (C + 2) % 3;
-    float p3 = 0.0f, exn = 0.0f, eyn = 0.0f;  // plane sc + 3
-    if (!EDGE || sc + 3 < k.L) {
-        if (!FACE || k.in) p3 = __ldg(pp);
-        if (k.need_x) exn = __ldg(pp + k.xoff);
-        if (k.need_y) eyn = __ldg(pp + k.yoff);
-    }
-    float dn = 0.0f;  // data factor of plane sc + 1
-    const int pd = sc + 1;
-    if (k.outp && (!EDGE || (pd >= k.z0 && pd < k.z1))) {
-        if (INSIDE || (k.inside_xy && pd >= k.r && pd < k.L - k.r)) dn = __ldg(dp);
-        else dn = border_data(ip, c);
-    }
-    dp += k.dplane;
-    if (!INSIDE) ip += k.WH * (c.img_f32 ? 4 : 1);
-    pp += k.WH;
-    Pb[C2][k.w + 1][k.lane] = S.P[C2];
-    if (k.w == 0) Pb[C2][0][k.lane] = S.EY[C2];
-    if (k.w == ST_WARPS - 1) Pb[C2][ST_WARPS + 1][k.lane] = S.EY[C2];
-    const float p0 = S.P[C], p1 = S.P[C1], p2 = S.P[C2];
-    float L1 = __shfl_up_sync(0xffffffffu, p1, 1);
-    float R1 = __shfl_down_sync(0xffffffffu, p1, 1);
-    if (k.lane == 0) L1 = S.EX[C1];
-    if (k.lane == 31) R1 = S.EX[C1];
-    if (FACE) {
-        if (k.xl_self) L1 = p1;
-        if (k.xr_self) R1 = p1;
-    }
-    const float U1 = Pb[C1][k.urow][k.lane];
-    const float D1 = Pb[C1][k.drow][k.lane];
-    // gradient of plane pn = sc + 1 (z rules at the first and last plane; a
-    // plane outside the volume gets a value that no output reads)
-    const int pn = sc + 1;
-    const GN gn = gn_from<A>(L1, R1, U1, D1, (!EDGE || pn > 0) ? p0 : p1, (!EDGE || pn < k.L - 1) ? p2 : p1);
-    S.G[C1] = GN4{gn.nx, gn.gx, gn.nz, gn.gz};
-    Gb[C1][k.w][k.lane] = make_float2(gn.ny, gn.gy);
-    __syncthreads();
-    const GN4 &gc = S.G[C];
-    float nxL = __shfl_up_sync(0xffffffffu, gc.nx, 1), nxR = __shfl_down_sync(0xffffffffu, gc.nx, 1);
-    float gxL = __shfl_up_sync(0xffffffffu, gc.gx, 1), gxR = __shfl_down_sync(0xffffffffu, gc.gx, 1);
-    if ((!EDGE || sc >= k.z0) && k.outp) {
-        if (FACE) {
-            if (k.xl_self) {
-                nxL = gc.nx;
-                gxL = gc.gx;
-            }
-            if (k.xr_self) {
-                nxR = gc.nx;
-                gxR = gc.gx;
-            }
-        }
-        const float2 yl2 = Gb[C][k.gwl][k.lane], yr2 = Gb[C][k.gwr][k.lane];
-        const float nyl = yl2.x, nyr = yr2.x, gyl = yl2.y, gyr = yr2.y;
-        const GN4 &gp = S.G[C2];
-        const bool zlo = !EDGE || sc > 0, zhi = !EDGE || sc < k.L - 1;
-        const float nzl = zlo ? gp.nz : gc.nz, nzr = zhi ? gn.nz : gc.nz;
-        const float gzl = zlo ? gp.gz : gc.gz, gzr = zhi ? gn.gz : gc.gz;
-        const float kap = __fadd_rn(__fadd_rn(half_diff(nxR, nxL), half_diff(nyr, nyl)), half_diff(nzr, nzl));
-        const float lap = __fadd_rn(__fadd_rn(half_diff(gxR, gxL), half_diff(gyr, gyl)), half_diff(gzr, gzl));
-        const float dh = dirac<A>(p0, c.eps);
-        const float out = update_phi(p0, dh, S.DT[C], kap, lap, c.dt, c.nu, c.mu);
-        *op = out;
-        acc = __fmaf_rn(out, 0.0f, acc);
-    }
-    op += k.WH;
-    S.P[C] = p3;
-    S.EX[C] = exn;
-    S.EY[C] = eyn;
-    S.DT[C1] = dn;
-}
-
-// The steps of a block on the fast path in groups of three (one per ring
-// slot); groups that can meet no z rule and no end of the plane range run
-// without the plane tests.
-template <Arith A, bool INSIDE, bool FACE>
-__device__ __forceinline__ void stencil_planes_f(const StencilCtx &k, const StepConst &c, StencilState &S, int count,
-                                                 const float *&pp, float *&op, const float *&dp,
-                                                 const unsigned char *&ip, float (*Pb)[ST_WARPS + 2][32],
-                                                 float2 (*Gb)[ST_WARPS][32], float &acc) {
-    for (int i = 0; i < count; i += 3) {
-        const int sc = k.first + i;
-        const bool edge = i == 0 || i + 3 >= count || sc <= 0 || sc + 5 >= k.L;
-        if (edge) {
-            stencil_step_f<0, A, INSIDE, true, FACE>(k, c, S, sc, pp, op, dp, ip, Pb, Gb, acc);
-            if (i + 1 < count) stencil_step_f<1, A, INSIDE, true, FACE>(k, c, S, sc + 1, pp, op, dp, ip, Pb, Gb, acc);
-            if (i + 2 < count) stencil_step_f<2, A, INSIDE, true, FACE>(k, c, S, sc + 2, pp, op, dp, ip, Pb, Gb, acc);
-        } else {
-            stencil_step_f<0, A, INSIDE, false, FACE>(k, c, S, sc, pp, op, dp, ip, Pb, Gb, acc);
-            stencil_step_f<1, A, INSIDE, false, FACE>(k, c, S, sc + 1, pp, op, dp, ip, Pb, Gb, acc);
-            stencil_step_f<2, A, INSIDE, false, FACE>(k, c, S, sc + 2, pp, op, dp, ip, Pb, Gb, acc);
-        }
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1182,8 +1043,10 @@ __global__ void __launch_bounds__(ST_WARPS * 32) box_kernel(const SubVolDev *__r
     }
 }
 
-template <Arith A, bool DEBUG>
-__global__ void __launch_bounds__(ST_WARPS * 32, 2) stencil_kernel(const SubVolDev *__restrict__ svs,
+// The debug step's stencil: the same arithmetic, one voxel per thread, with
+// the intermediate fields written out.
+template <Arith A>
+__global__ void __launch_bounds__(ST_WARPS * 32, 2) stencil_debug_kernel(const SubVolDev *__restrict__ svs,
                                                                    const int *__restrict__ pre,
                                                                    const StepConst c, int parity,
                                                                    unsigned *__restrict__ flag, DebugOut dbg) {
@@ -1207,11 +1070,6 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 2) stencil_kernel(const SubVolD
     const int tz = t / nty;
     const int x0 = tx * ST_OX, y0 = ty * ST_OY;
     k.ref = c.boundary == 0;
-    // Every block takes the fast path but in the debug step and, in the
-    // reference mode, the blocks at x = 0 that hold row 0 (where the previous
-    // linear element of voxel (0, 0) lies in the previous plane).
-    const bool fast = !DEBUG && !(k.ref && x0 == 0 && y0 < 2);
-    const bool prev_lane = fast && k.ref && x0 == 0 && lane == 0;
     k.x = x0 - 1 + lane;
     k.y = y0 - 1 + w;
     k.w = w;
@@ -1219,43 +1077,35 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 2) stencil_kernel(const SubVolD
     k.z0 = tz * c.zc;
     k.z1 = min(k.z0 + c.zc, k.L);
     k.first = k.z0 - 2;
-    // the thread's voxel: lane 0 at x = 0 may carry (W - 1, y - 1)
-    const int ex = prev_lane ? k.W - 1 : k.x, ey = prev_lane ? k.y - 1 : k.y;
-    k.in = ex >= 0 && ex < k.W && ey >= 0 && ey < k.H;
-    k.outp = k.in && !prev_lane && lane >= 1 && lane <= ST_OX && w >= 1 && w <= ST_OY;
+    k.in = k.x >= 0 && k.x < k.W && k.y >= 0 && k.y < k.H;
+    k.outp = k.in && lane >= 1 && lane <= ST_OX && w >= 1 && w <= ST_OY;
     k.WH = (size_t)k.W * k.H;
-    k.col = k.in ? (size_t)ey * k.W + ex : 0;
+    k.col = k.in ? (size_t)k.y * k.W + k.x : 0;
     k.phi = (parity ? s.phi[1] : s.phi[0]) + k.col;
     k.phi_out = parity ? s.phi[0] : s.phi[1];
     const bool valid = s.Wv > 0;
     const int r = k.r;
-    k.inside_xy = valid && ex >= r && ex < k.W - r && ey >= r && ey < k.H - r;
+    k.inside_xy = valid && k.x >= r && k.x < k.W - r && k.y >= r && k.y < k.H - r;
     k.blk_inside = valid && x0 >= r && x0 + ST_OX - 1 < k.W - r && y0 >= r && y0 + ST_OY - 1 < k.H - r &&
                    k.z0 >= r && k.z1 - 1 < k.L - r;
     k.dplane = (size_t)s.Wp * s.Hv;
-    k.dcol = k.inside_xy ? s.db + (size_t)(ey - r) * s.Wp + (ex - r) : s.db;
+    k.dcol = k.inside_xy ? s.db + (size_t)(k.y - r) * s.Wp + (k.x - r) : s.db;
     if (c.full_data) {  // every voxel's data factor comes from the box or expanded data-term kernels
         k.blk_inside = true;
         k.dplane = k.WH;
         k.dcol = s.db + 2 * (size_t)s.Wp * s.Hv * s.Lv + k.col + (size_t)r * k.WH;
     }
     // The shuffles and shared rows supply every neighbour except: x-1 for
-    // lane 0 (and, on the debug path, the previous linear element for x == 0
-    // in the reference mode), both at linear offset -1; x+1 for lane 31;
-    // y-1 / y+1 for the halo rows.  Corner threads of the halo are never read.
+    // lane 0 and the previous linear element for x == 0 in the reference
+    // mode, both at linear offset -1; x+1 for lane 31; y-1 / y+1 for the halo
+    // rows.  Corner threads of the halo are never read.
     const bool halo_row = w == 0 || w == ST_WARPS - 1;
     const bool halo_col = lane == 0 || lane == 31;
     k.need_x = k.in && !(halo_row && halo_col) &&
-               ((lane == 0) || (!fast && k.x == 0 && k.ref) || (lane == 31 && ex + 1 < k.W));
+               ((lane == 0) || (k.x == 0 && k.ref) || (lane == 31 && k.x + 1 < k.W));
     k.xoff = lane == 31 ? 1 : -1;
-    k.need_y = k.in && halo_row && !halo_col && (w == 0 ? ey > 0 : ey + 1 < k.H);
+    k.need_y = k.in && halo_row && !halo_col && (w == 0 ? k.y > 0 : k.y + 1 < k.H);
     k.yoff = w == 0 ? -(ptrdiff_t)k.W : (ptrdiff_t)k.W;
-    k.xl_self = !k.ref && ex == 0;
-    k.xr_self = ex == k.W - 1;
-    k.urow = ey > 0 ? w : w + 1;
-    k.drow = ey < k.H - 1 ? w + 2 : w + 1;
-    k.gwl = ey > 0 ? w - 1 : w;
-    k.gwr = ey < k.H - 1 ? w + 1 : w;
 
     StencilState S;
     const int sp = k.first;
@@ -1270,37 +1120,12 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 2) stencil_kernel(const SubVolD
     S.DT[0] = S.DT[1] = S.DT[2] = 0.0f;
     for (int i = 0; i < 3; ++i) S.G[i] = GN4{0.f, 0.f, 0.f, 0.f};
     Pb[1][w + 1][lane] = S.P[1];
-    if (w == 0) Pb[1][0][lane] = S.EY[1];
-    if (w == ST_WARPS - 1) Pb[1][ST_WARPS + 1][lane] = S.EY[1];
     __syncthreads();
     const int count = k.z1 - k.first;
-    if (fast) {
-        const float *pp = k.phi + (ptrdiff_t)(k.first + 3) * (ptrdiff_t)k.WH;
-        float *op = k.phi_out + (ptrdiff_t)k.first * (ptrdiff_t)k.WH + (ptrdiff_t)k.col;
-        // plane first + 1 of the data column and of the image (read only
-        // from plane z0 on)
-        const float *dp = k.dcol + ((ptrdiff_t)k.first + 1 - k.r) * (ptrdiff_t)k.dplane;
-        const ptrdiff_t esz = c.img_f32 ? 4 : 1;
-        const unsigned char *ip = static_cast<const unsigned char *>(s.img) +
-                                  ((ptrdiff_t)k.col + ((ptrdiff_t)k.first + 1) * (ptrdiff_t)k.WH) * esz;
-        // x/y-interior blocks: every thread and neighbour load inside, no x
-        // or y face rule
-        const bool face = !(x0 >= 2 && x0 + 32 <= k.W && y0 >= 2 && y0 + ST_OY + 2 <= k.H);
-        float acc = 0.0f;
-        if (face) {
-            if (k.blk_inside) stencil_planes_f<A, true, true>(k, c, S, count, pp, op, dp, ip, Pb, Gb, acc);
-            else stencil_planes_f<A, false, true>(k, c, S, count, pp, op, dp, ip, Pb, Gb, acc);
-        } else {
-            if (k.blk_inside) stencil_planes_f<A, true, false>(k, c, S, count, pp, op, dp, ip, Pb, Gb, acc);
-            else stencil_planes_f<A, false, false>(k, c, S, count, pp, op, dp, ip, Pb, Gb, acc);
-        }
-        if (!isfinite(acc)) atomicOr(flag, kFlagNonFinite);
-        return;
-    }
     for (int i = 0; i < count; i += 3) {
-        stencil_step<0, A, DEBUG>(k, c, S, i, Pb, Gb, flag, dbg);
-        if (i + 1 < count) stencil_step<1, A, DEBUG>(k, c, S, i + 1, Pb, Gb, flag, dbg);
-        if (i + 2 < count) stencil_step<2, A, DEBUG>(k, c, S, i + 2, Pb, Gb, flag, dbg);
+        stencil_step<0, A>(k, c, S, i, Pb, Gb, flag, dbg);
+        if (i + 1 < count) stencil_step<1, A>(k, c, S, i + 1, Pb, Gb, flag, dbg);
+        if (i + 2 < count) stencil_step<2, A>(k, c, S, i + 2, Pb, Gb, flag, dbg);
     }
 }
 

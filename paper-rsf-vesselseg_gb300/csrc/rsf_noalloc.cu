@@ -165,6 +165,7 @@ extern "C" rsf_status rsf_evolve_noalloc(const rsf_params *p, const void *image,
     c.xrpw = sh.xrpw;
     c.pairs = sh.pairs;
     c.zc = sh.zc;
+    rsf::set_pair_const(c.pk, c.eps, c.dt, c.nu, c.mu);
     alignas(64) unsigned char map[rsf::TMAP_BYTES];
     if (sh.zt) {
         if (!rsf::encode_pair_map(map, d)) return fail(RSF_ERR_CUDA, "rsf_evolve_noalloc: TMA tensor map encoding failed");

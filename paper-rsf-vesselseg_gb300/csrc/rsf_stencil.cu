@@ -1,18 +1,18 @@
 // rsf_stencil.cu -- the stencil / update kernel instantiations.
-#include "rsf_kernels.cuh"
+#include "rsf_stencil_pair.cuh"
 
 namespace rsf {
 
 cudaError_t launch_stencil(const SubVolDev *svs, const int *pre, int blocks, const StepConst &c, int parity,
                            int arith, unsigned *flag, const DebugOut *dbg, cudaStream_t st) {
-    const DebugOut none = {nullptr, 0};
-    constexpr int T = ST_WARPS * 32;
     if (dbg) {
-        if (arith == 1) stencil_kernel<Arith::Reference, true><<<blocks, T, 0, st>>>(svs, pre, c, parity, flag, *dbg);
-        else stencil_kernel<Arith::Portable, true><<<blocks, T, 0, st>>>(svs, pre, c, parity, flag, *dbg);
+        constexpr int T = ST_WARPS * 32;
+        if (arith == 1) stencil_debug_kernel<Arith::Reference><<<blocks, T, 0, st>>>(svs, pre, c, parity, flag, *dbg);
+        else stencil_debug_kernel<Arith::Portable><<<blocks, T, 0, st>>>(svs, pre, c, parity, flag, *dbg);
     } else {
-        if (arith == 1) stencil_kernel<Arith::Reference, false><<<blocks, T, 0, st>>>(svs, pre, c, parity, flag, none);
-        else stencil_kernel<Arith::Portable, false><<<blocks, T, 0, st>>>(svs, pre, c, parity, flag, none);
+        constexpr int T = SP_WARPS * 32;
+        if (arith == 1) stencil_pair_kernel<Arith::Reference><<<blocks, T, 0, st>>>(svs, pre, c, parity, flag);
+        else stencil_pair_kernel<Arith::Portable><<<blocks, T, 0, st>>>(svs, pre, c, parity, flag);
     }
     return cudaGetLastError();
 }

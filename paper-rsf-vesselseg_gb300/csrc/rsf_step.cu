@@ -57,21 +57,42 @@ int choose_xb(const int *Wv, int n) {
     return best;
 }
 
-// Stencil planes per block: the most of ST_ZC_MAX, ST_ZC and ST_ZC / 2 that
-// still gives four waves of blocks (two resident per SM); each block
-// recomputes the gradient of two planes before its first output, so deeper
-// blocks waste less (8.06 against 8.26 ms per launch on the 48-sub-volume
-// batch for 128 against 64 planes).
+// Stencil planes per block.  A block recomputes the gradient of two planes
+// before its first output, so deep blocks waste less; but a block streams its
+// planes one after another, each behind a barrier, so a small volume wants many
+// shallow ones.  The candidate with the lowest modelled time is taken.  A block
+// takes its planes, the two before them and about three of set-up as steps; a
+// step costs 0.45 (us) of an SM's issue per block sharing it and at least the
+// 0.9 of its own latency chain, and the last wave is three quarters empty.
 int choose_zc(const int *whl, int n) {
-    int zc = ST_ZC_MAX;
-    for (; zc > ST_ZC / 2; zc /= 2) {
+    const double issue = 0.45, chain = 0.9;
+    const int sms = sm_count(), setup = 5;
+    int best = ST_ZC_MAX;
+    double best_t = -1.0;
+    for (int zc : {ST_ZC_MAX, 96, ST_ZC, 48, ST_ZC / 2, 24, 16, 12, 8, 6, 4}) {
         long long blocks = 0;
-        for (int i = 0; i < n; i++)
-            blocks += (long long)((whl[3 * i] + ST_OX - 1) / ST_OX) * ((whl[3 * i + 1] + ST_OY - 1) / ST_OY) *
-                      ((whl[3 * i + 2] + zc - 1) / zc);
-        if (blocks >= 4LL * 2 * sm_count()) break;
+        double steps = 0.0;
+        int deepest = 0;
+        for (int i = 0; i < n; i++) {
+            const int L = whl[3 * i + 2], chunks = (L + zc - 1) / zc;
+            const long long cols = (long long)((whl[3 * i] + ST_OX - 1) / ST_OX) * ((whl[3 * i + 1] + ST_OY - 1) / ST_OY);
+            blocks += cols * chunks;
+            steps += (double)cols * (L + setup * chunks);
+            if (L < zc ? L > deepest : zc > deepest) deepest = L < zc ? L : zc;
+        }
+        double t = 0.0;
+        if (blocks <= 3LL * sms) {
+            const double step = issue * (double)((blocks + sms - 1) / sms);
+            t = (deepest + setup) * (step > chain ? step : chain);
+        } else {
+            t = issue * (steps / sms + 0.75 * (deepest + setup));
+        }
+        if (best_t < 0.0 || t < best_t) {
+            best_t = t;
+            best = zc;
+        }
     }
-    return zc;
+    return best;
 }
 
 int choose_xrpw(const int *whl, int n, int k, int xb_w) {
@@ -178,7 +199,7 @@ void tile_counts(const SubVolDev &d, int kspec, const LaunchShape &sh, int tiles
     tiles[NKERN + 3] = g ? (int)(((long long)d.W * d.H * d.L + GB_T - 1) / GB_T) : 0;
 }
 
-// Raises the dynamic shared-memory limit of the x-pass instantiations on the
+// Raises the dynamic shared-memory limit of the kernels that need it on the
 // current device; called once per workspace, outside any stream capture.
 cudaError_t configure_device() {
     cudaError_t e = config_xpass_0();
