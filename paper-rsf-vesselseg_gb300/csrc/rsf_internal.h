@@ -222,6 +222,7 @@ cudaError_t launch_reassemble(const TileDev *d_tiles, const int n[3], const int 
                               const int *const hi[3], int mode, float *out, int W, int H, int L, cudaStream_t st);
 // SM copy between device-accessible addresses (rsf_copy.cu).
 cudaError_t launch_copy(void *dst, const void *src, size_t bytes, cudaStream_t st);
+cudaError_t config_signed_distance();
 // Signed distance of {seed > thr}; scratch holds 3 * W*H*L words.
 cudaError_t launch_signed_distance(const void *seed, int f32, float thr, float *phi, int W, int H, int L,
                                    unsigned *scratch, cudaStream_t st);

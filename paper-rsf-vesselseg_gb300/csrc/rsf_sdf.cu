@@ -21,6 +21,17 @@
 // Column threads are adjacent in x, so every access of a column step is
 // coalesced across the warp; the envelope stacks live in device scratch laid
 // out [k][column] for the same reason.
+//
+// Columns of up to kTileMax voxels take the tiled kernels instead: both
+// classes at once (a voxel needs its distance to the other class only, so one
+// signed value per voxel carries both transforms), a block holding 32 whole
+// columns in shared memory and every voxel searching outwards from itself.
+// The envelope is a serial chain of dependent loads per column, with one thread
+// per column; the search has a thread per four voxels and stops at the
+// distance found, and beyond kFine rows it skips blocks of 16 rows whose
+// smallest value cannot improve on it, so that sparse seeds stay cheap.
+// 256 x 448 x 512 voxels, a tenth of them inside:
+// 3.90 ms with the envelopes, 0.80 ms here.
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -167,7 +178,205 @@ __global__ void __launch_bounds__(kColThreads) sdf_cols(ColArgs a) {
     }
 }
 
+// ---------------------------------------------------------------------------
+// Tiled path.  Values are signed: positive inside, negative outside, the
+// magnitude the distance to the other class so far.
+// ---------------------------------------------------------------------------
+constexpr int kTileMax = 1408;          // column length: 32 columns of 32-bit values and their block minima in shared memory
+constexpr int kFine = 24;               // rows searched one by one to either side
+constexpr int kSkip = 16;               // rows per skipped block beyond
+constexpr short kNone16 = 32767;        // no voxel of the other class in the row
+constexpr int kNone = 1 << 28;          // nor in the plane; plus any squared offset it stays above every distance
+
+// Signed distance along x to the other class: one warp per row.  The row's
+// class words (32 voxels each) and, per word, the first voxel of each class
+// to its right are gathered from the end; a second sweep carries the last
+// ones to the left.
+__global__ void __launch_bounds__(32 * kRowWarps) sdf_rows_tile(const void *seed, int f32, float thr, short *d, int W,
+                                                                long long rows) {
+    constexpr int kWords = (kTileMax + 31) / 32;
+    __shared__ unsigned word_s[kRowWarps][kWords];
+    __shared__ int next_s[kRowWarps][kWords][2];
+    const long long row = (long long)blockIdx.x * kRowWarps + threadIdx.x / 32;
+    if (row >= rows) return;  // uniform per warp
+    const int lane = threadIdx.x & 31;
+    unsigned *word = word_s[threadIdx.x / 32];
+    int(*next)[2] = next_s[threadIdx.x / 32];
+    const size_t base = (size_t)row * W;
+    const int nw = (W + 31) / 32, far = 1 << 20;
+    int nx[2] = {far, far};  // nearest outside / inside voxel to the right
+    for (int i = nw - 1; i >= 0; --i) {
+        const int x = 32 * i + lane;
+        const unsigned in = __ballot_sync(0xffffffffu, x < W && is_inside(seed, f32, base + x, thr));
+        const unsigned have = i < nw - 1 || (W & 31) == 0 ? 0xffffffffu : (1u << (W & 31)) - 1u;
+        if (lane == 0) {
+            word[i] = in;
+            next[i][0] = nx[0];
+            next[i][1] = nx[1];
+        }
+        if (~in & have) nx[0] = 32 * i + __ffs(~in & have) - 1;
+        if (in) nx[1] = 32 * i + __ffs(in) - 1;
+    }
+    __syncwarp();
+    int px[2] = {-far, -far};  // to the left
+    for (int i = 0; i < nw; ++i) {
+        const int x = 32 * i + lane;
+        const unsigned in = word[i], have = i < nw - 1 || (W & 31) == 0 ? 0xffffffffu : (1u << (W & 31)) - 1u;
+        const unsigned out = ~in & have;
+        const int c = (in >> lane) & 1;
+        const unsigned other = c ? out : in;
+        const unsigned lo = other & ((1u << lane) - 1u), hi = other & ~((2u << lane) - 1u);
+        const int left = lo ? 32 * i + 31 - __clz(lo) : px[1 - c];
+        const int right = hi ? 32 * i + __ffs(hi) - 1 : next[i][1 - c];
+        const int dist = min(min(x - left, right - x), (int)kNone16);
+        if (x < W) d[base + x] = (short)(c ? dist : -dist);
+        if (out) px[0] = 32 * i + 31 - __clz(out);
+        if (in) px[1] = 32 * i + 31 - __clz(in);
+    }
+}
+
+struct TileArgs {
+    const void *in;     // signed row distances (int16), or squared plane distances (int32) for FINAL
+    int *out;           // squared plane distances, signed
+    float *phi;         // FINAL
+    int W, n, ntx;
+    long long plane;    // element offset of a column group's outer index
+    long long stride;   // element step along the column
+    float fill;
+};
+
+// Squared distance along a strided axis added to the values in `in`, for 32
+// columns per block.  A thread takes four consecutive rows, which share every
+// value they read: rows y0 - t and y0 + 3 + t lie t .. t + 3 rows from them.
+template <bool FINAL, int T>
+__global__ void __launch_bounds__(T) sdf_cols_tile(TileArgs a) {
+    extern __shared__ int sdf_sm[];
+    int *v = sdf_sm;                                // [n][32]
+    const int nb = (a.n + kSkip - 1) / kSkip;
+    int *mo = v + 32 * a.n, *mi = mo + 32 * nb;     // block minima of the distance to outside / inside
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    constexpr int NW = T / 32;
+    const int x = (blockIdx.x % a.ntx) * 32 + lane;
+    const bool have = x < a.W;
+    const size_t base = (size_t)(blockIdx.x / a.ntx) * (size_t)a.plane + x;
+    for (int r = w; r < a.n; r += NW) {
+        int q = 1;
+        if (have) {
+            const size_t i = base + (size_t)r * (size_t)a.stride;
+            if (FINAL) {
+                q = __ldg(static_cast<const int *>(a.in) + i);
+            } else {
+                const int d = __ldg(static_cast<const short *>(a.in) + i);
+                const int m = abs(d) == kNone16 ? kNone : d * d;
+                q = d > 0 ? m : -m;
+            }
+        }
+        v[32 * r + lane] = q;
+    }
+    __syncthreads();
+    for (int b = w; b < nb; b += NW) {
+        int so = kNone, si = kNone;
+        for (int r = kSkip * b; r < min(kSkip * (b + 1), a.n); ++r) {
+            const int q = v[32 * r + lane];
+            so = min(so, max(q, 0));
+            si = min(si, max(-q, 0));
+        }
+        mo[32 * b + lane] = so;
+        mi[32 * b + lane] = si;
+    }
+    __syncthreads();
+    for (int y0 = 4 * w; y0 < a.n; y0 += 4 * NW) {
+        int s[4], best[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int q = v[32 * min(y0 + j, a.n - 1) + lane];
+            s[j] = q > 0 ? 1 : -1;
+            best[j] = abs(q);
+        }
+        // a voxel of the other class counts 0, one of the same class its own distance
+        auto take = [&](int q, int j, int d2) { best[j] = min(best[j], max(s[j] * q + d2, d2)); };
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int q = v[32 * min(y0 + i, a.n - 1) + lane];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (i != j) take(q, j, (i - j) * (i - j));
+        }
+        auto worst = [&] { return max(max(best[0], best[1]), max(best[2], best[3])); };
+        // rows past an end repeat the last one at a larger offset, which never wins
+        int t = 1;
+        for (; t <= kFine && __any_sync(0xffffffffu, t * t < worst()); ++t) {
+            const int ql = v[32 * max(y0 - t, 0) + lane], qr = v[32 * min(y0 + 3 + t, a.n - 1) + lane];
+            const int t0 = t * t, t1 = t0 + 2 * t + 1, t2 = t0 + 4 * t + 4, t3 = t0 + 6 * t + 9;
+            take(ql, 0, t0);
+            take(ql, 1, t1);
+            take(ql, 2, t2);
+            take(ql, 3, t3);
+            take(qr, 3, t0);
+            take(qr, 2, t1);
+            take(qr, 1, t2);
+            take(qr, 0, t3);
+        }
+        if (t > kFine && __any_sync(0xffffffffu, t * t < worst())) {
+            // (a lane that gets here has four voxels of one class: mixed ones found each other)
+            const int *m = s[0] > 0 ? mo : mi;
+            for (int side = 0; side < 2; ++side) {
+                const int step = side ? 1 : -1;
+                for (int b = side ? min(y0 + 3 + t, a.n - 1) / kSkip : max(y0 - t, 0) / kSkip; b >= 0 && b < nb; b += step) {
+                    const int gap = max(side ? kSkip * b - (y0 + 3) : y0 - (kSkip * b + kSkip - 1), 0);
+                    const int wst = worst();
+                    if (!__any_sync(0xffffffffu, gap * gap < wst)) break;
+                    if (!__any_sync(0xffffffffu, gap * gap + m[32 * b + lane] < wst)) continue;
+                    for (int r = kSkip * b; r < min(kSkip * (b + 1), a.n); ++r) {
+                        const int q = v[32 * r + lane];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) take(q, j, (r - y0 - j) * (r - y0 - j));
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (!have || y0 + j >= a.n) continue;
+            const size_t i = base + (size_t)(y0 + j) * (size_t)a.stride;
+            if (FINAL) {
+                const float mag = best[j] >= kNone ? a.fill : __fsqrt_rn(__int2float_rn(best[j]));
+                a.phi[i] = s[j] > 0 ? mag : -mag;
+            } else {
+                a.out[i] = s[j] * best[j];
+            }
+        }
+    }
+}
+
+size_t tile_smem(int n) { return 128 * ((size_t)n + 2 * ((n + kSkip - 1) / kSkip)); }
+
+// 256 threads share an SM three or more times up to about 500 rows; longer
+// columns leave one or two blocks, which then bring 512.
+constexpr int kWideFrom = 560;
+
+template <bool FINAL>
+void launch_tile(const TileArgs &a, long long groups, cudaStream_t st) {
+    const unsigned blocks = (unsigned)(groups * a.ntx);
+    if (a.n >= kWideFrom) sdf_cols_tile<FINAL, 512><<<blocks, 512, tile_smem(a.n), st>>>(a);
+    else sdf_cols_tile<FINAL, 256><<<blocks, 256, tile_smem(a.n), st>>>(a);
+}
+
+template <bool FINAL, int T>
+cudaError_t allow_tile() {
+    return cudaFuncSetAttribute(sdf_cols_tile<FINAL, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)tile_smem(T == 512 ? kTileMax : kWideFrom));
+}
+
 }  // namespace
+
+cudaError_t config_signed_distance() {
+    cudaError_t e = allow_tile<false, 256>();
+    if (e == cudaSuccess) e = allow_tile<true, 256>();
+    if (e == cudaSuccess) e = allow_tile<false, 512>();
+    if (e == cudaSuccess) e = allow_tile<true, 512>();
+    return e;
+}
 
 cudaError_t launch_signed_distance(const void *seed, int f32, float thr, float *phi, int W, int H, int L,
                                    unsigned *scratch, cudaStream_t st) {
@@ -175,6 +384,16 @@ cudaError_t launch_signed_distance(const void *seed, int f32, float thr, float *
     unsigned *d = scratch, *sv = scratch + N, *sf = scratch + 2 * N;
     const long long rows = (long long)H * L;
     const float fill = (float)W + (float)H + (float)L;
+    if (W <= kTileMax && H <= kTileMax && L <= kTileMax) {
+        short *dx = reinterpret_cast<short *>(scratch + N);
+        int *dxy = reinterpret_cast<int *>(scratch);
+        sdf_rows_tile<<<(unsigned)((rows + kRowWarps - 1) / kRowWarps), 32 * kRowWarps, 0, st>>>(seed, f32, thr, dx, W,
+                                                                                                rows);
+        const int ntx = (W + 31) / 32;
+        launch_tile<false>(TileArgs{dx, dxy, nullptr, W, H, ntx, (long long)W * H, W, fill}, L, st);
+        launch_tile<true>(TileArgs{dxy, nullptr, phi, W, L, ntx, W, (long long)W * H, fill}, H, st);
+        return cudaGetLastError();
+    }
     for (int feat_inside = 0; feat_inside < 2; feat_inside++) {
         sdf_rows<<<(unsigned)((rows + kRowWarps - 1) / kRowWarps), 32 * kRowWarps, 0, st>>>(seed, f32, thr,
                                                                                            feat_inside, d, W, rows);

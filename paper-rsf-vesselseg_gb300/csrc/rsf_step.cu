@@ -208,6 +208,7 @@ cudaError_t configure_device() {
     if (e == cudaSuccess) e = config_xpass_35();
     if (e == cudaSuccess) e = config_ztpass_21();
     if (e == cudaSuccess) e = config_ztpass_35();
+    if (e == cudaSuccess) e = config_signed_distance();
     return e;
 }
 
