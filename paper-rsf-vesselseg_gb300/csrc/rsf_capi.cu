@@ -50,7 +50,7 @@ struct rsf_workspace {
     float *pool_g = nullptr;     // expanded data term's x-blurred fields, 4 * max_voxels (first use)
     SubVolDev *d_svs = nullptr;
     int *d_pre = nullptr;        // NPRE * (max_subvols + 1)
-    unsigned char *d_maps = nullptr;  // TMA maps of the pair planes, max_subvols * TMAP_BYTES
+    unsigned char *d_maps = nullptr;  // TMA maps of the y-pass fields, max_subvols * TMAP_BYTES
     unsigned *d_flag = nullptr;
     // Pinned staging of the table, kStages slots used in turn: a call waits
     // only for the upload of the call kStages before it, so consecutive
@@ -410,7 +410,7 @@ rsf_status prepare(rsf_workspace *ws, const rsf_subvol *svs, int32_t n, int k, i
         }
         h_svs[i] = d;
         if (shape->zt && d.Wv > 0 && !rsf::encode_pair_map(h_maps + (size_t)i * rsf::TMAP_BYTES, d))
-            return fail(RSF_ERR_CUDA, "TMA tensor map encoding of the pair planes failed");
+            return fail(RSF_ERR_CUDA, "TMA tensor map encoding of the y-pass fields failed");
     }
     for (int j = 0; j < rsf::NPRE; j++) totals[j] = pre[j * n1 + n];
     cudaError_t e = cudaMemcpyAsync(ws->d_svs, h_svs, (size_t)n * sizeof(SubVolDev), cudaMemcpyHostToDevice, st);
@@ -445,7 +445,7 @@ StepConst make_const(const rsf_params *p, int k, const float *taps, rsf_dtype dt
     c.nsv = n;
     c.xb_w = sh.xb_w;
     c.xrpw = sh.xrpw;
-    c.pairs = sh.pairs;
+    c.zout = sh.zout;
     c.zc = sh.zc;
     c.ymaps = sh.zt ? maps : nullptr;
     c.box = (int)p->sigma2;
@@ -731,7 +731,7 @@ rsf_status rsf_step_adjoint_batched(rsf_workspace *ws, const rsf_params *p, rsf_
     }
     cudaStream_t st = (cudaStream_t)stream;
     // Specialised tap counts recompute the blurs with the forward step's own
-    // streaming x- and y-passes (pair planes in pool_x, pool_y) and the
+    // streaming x- and y-passes (fields in pool_x, pool_y) and the
     // z-pass's adjoint variant, which leaves the data-term adjoint pair and
     // e_out, e_in in each volume's xs slice.
     const int kspec = rsf::kernel_k(k, RSF_ARITH_PORTABLE, false);

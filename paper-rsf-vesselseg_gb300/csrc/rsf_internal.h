@@ -13,10 +13,15 @@ constexpr int MAXK = 128;  // largest supported tap count (sigma up to ~18)
 // Kernel tilings (the launchers derive tile counts from them).
 constexpr int XP_ROWS = 4;     // x-pass: warps per block
 constexpr int XP_RPW = 8;      // x-pass: largest rows per warp (XP_ROWS apart; chosen per launch)
-constexpr int YP_COLS = 128;   // y-pass: columns per block (one column of one pair per thread)
+constexpr int YP_COLS = 128;   // y-pass: float2 columns per block (one field pair of one column per thread)
 constexpr int YB_TX = 128;     // generic y-pass: columns per block
 constexpr int YB_YB = 16;      // generic y-pass: outputs per thread along y
-constexpr int ZP_PAIRS = 32;   // z-pass: column pairs per block (four lanes each)
+constexpr int ZP_COLS = 128;   // z-pass: columns per block
+// z-pass: resident blocks per SM that its 4 K accumulator registers leave room
+// for (21 taps: 3.70 ms per launch on the 48-sub-volume batch with 4, 4.17 with
+// 3; 29 and 35 taps spill with 3: 771 against 1061 us on a 195 M voxel batch,
+// 1.02 against 1.45 ms on 512^3)
+constexpr int zpass_blocks(int K) { return K <= 21 ? 4 : 2; }
 constexpr int ZB_TX = 128;     // generic z-pass: columns per block
 constexpr int ZB_ZB = 16;      // generic z-pass: outputs per thread along z
 constexpr int ST_OX = 30;      // stencil: output columns per warp (lanes 1..30)
@@ -31,9 +36,9 @@ constexpr int XB_CHOICES[2] = {5, 9};
 // One sub-volume as the kernels see it.
 //   xb: x-pass fields, each Wp x H x L   (row stride Wp)
 //   yb: y-pass fields, each Wp x Hv x L
-//   The specialised tap counts keep the fields as two float2 pair planes,
-//   pair 0 (H, 1-H) and pair 1 (I H, I (1-H)); the run-time-k kernels as four
-//   separate float planes (H, 1-H, I H, I (1-H)).
+//   The specialised tap counts keep the fields interleaved, float4 (H, 1-H,
+//   I H, I (1-H)) per voxel; the run-time-k kernels as four separate float
+//   planes in that order.
 //   db: data factor lambda (e_out - e_in) of the valid region, Wp x Hv x Lv;
 //       it reuses the x-pass storage, which is dead once the y-pass has run.
 //       With the box e-term or the expanded data term it holds f_out and
@@ -55,6 +60,10 @@ struct SubVolDev {
 struct StepConst {
     float taps[MAXK];
     float2 taps2[MAXK];  // (g, g) pairs for the packed multiply-adds
+    // tap t as a packed operand
+    __device__ __forceinline__ unsigned long long tap2(int t) const {
+        return pack2(taps2[t]);
+    }
     int k, r;
     float eps, dt, mu, nu, l1, l2;
     int lam_equal;
@@ -63,7 +72,7 @@ struct StepConst {
     int nsv;        // number of sub-volumes in the table
     int xb_w;       // x-pass outputs per lane for this launch
     int xrpw;       // x-pass rows per warp for this launch
-    int pairs;      // 1: x/y fields in float2 pair planes (specialised tap counts)
+    int zout;       // z-pass output planes per block for this launch (specialised tap counts)
     int zc;         // stencil planes per block for this launch
     int box;        // e-term box radius (int)sigma2; 0: e = (I - f)^2
     int gauss;      // 1: expanded Gaussian data term (rsf_gauss.cu)
@@ -71,13 +80,13 @@ struct StepConst {
     float s3;       // gauss: the valid correlation of ones, K*1
     ptrdiff_t gdelta;  // gauss: offset (floats) of the scratch G from xb
     PairConst pk;   // the packed arithmetic's constants
-    const void *ymaps;  // per sub-volume TMA map of the y-pass pair planes (TMAP_BYTES each), or null
+    const void *ymaps;  // per sub-volume TMA map of the y-pass fields (TMAP_BYTES each), or null
 };
 
 // TMA tensor maps (CUtensorMap) as the kernels see them: 128 bytes each, in
 // device memory aligned to 128 bytes.
 constexpr int TMAP_BYTES = 128;
-// Encodes the z-pass map of d's pair planes into `out` (host memory); false
+// Encodes the z-pass map of d's y-pass fields into `out` (host memory); false
 // when the driver's encoder is unavailable or refuses the layout.
 bool encode_pair_map(void *out, const SubVolDev &d);
 bool tensor_maps_available();
@@ -118,7 +127,7 @@ constexpr int MAX_BOX = 8;  // largest e-term box radius
 struct LaunchShape {
     int xb_w;   // x-pass outputs per lane
     int xrpw;   // x-pass rows per warp (1, 2, 4 or XP_RPW)
-    int pairs;  // 1: x/y fields in float2 pair planes (specialised tap counts)
+    int zout;   // z-pass output planes per block (specialised tap counts)
     int zt;     // 1: the z-pass loads planes with TMA (needs a map per sub-volume)
     int zc;     // stencil planes per block
     int gauss;  // 1: the expanded data term's kernels run (tiles NKERN .. NPRE - 1)
@@ -175,18 +184,22 @@ void adjoint_tiles(const AdjVol &v, bool streamed, int tiles[NADJ]);
     cudaError_t config_xpass_##K();                                                                             \
     cudaError_t launch_ypass_##K(const SubVolDev *, const int *, int, const StepConst &, cudaStream_t);          \
     cudaError_t launch_zpass_##K(const SubVolDev *, const int *, int, const StepConst &, const DebugOut *,      \
-                                 cudaStream_t);
+                                 cudaStream_t);                                                                \
+    cudaError_t config_zpass_##K();
 RSF_DECLARE_K(0)
 RSF_DECLARE_K(21)
 RSF_DECLARE_K(29)
 RSF_DECLARE_K(35)
 #undef RSF_DECLARE_K
-// The streaming z-pass with the adjoint's emit (pair planes, specialised k):
+// The streaming z-pass with the adjoint's emit (specialised k):
 // sub-volume i of the table is volume i of `vols`.
+cudaError_t config_zpass_adjoint_21();
 cudaError_t launch_zpass_adjoint_21(const SubVolDev *, const int *, int, const StepConst &, const AdjVol *vols,
                                     cudaStream_t);
+cudaError_t config_zpass_adjoint_29();
 cudaError_t launch_zpass_adjoint_29(const SubVolDev *, const int *, int, const StepConst &, const AdjVol *vols,
                                     cudaStream_t);
+cudaError_t config_zpass_adjoint_35();
 cudaError_t launch_zpass_adjoint_35(const SubVolDev *, const int *, int, const StepConst &, const AdjVol *vols,
                                     cudaStream_t);
 cudaError_t config_ztpass_21();

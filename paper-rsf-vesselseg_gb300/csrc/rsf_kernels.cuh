@@ -49,8 +49,6 @@ __device__ __forceinline__ float load_img(const void *img, size_t i, int f32) {
                : (float)__ldg(static_cast<const unsigned char *>(img) + i);
 }
 
-__device__ __forceinline__ float2 ld2(const float *p) { return __ldg(reinterpret_cast<const float2 *>(p)); }
-
 // Valid correlation of XB consecutive outputs of one packed field pair:
 // src points at the lane's first input, consecutive inputs are two float2
 // apart (the shared slab holds float4 (H, 1-H, I H, I (1-H)) per element).
@@ -58,16 +56,18 @@ template <int K, int XB>
 __device__ __forceinline__ void xconv_pair(const float2 *src, const StepConst &c, const float2 *taps_s, int k,
                                            float2 (&acc)[XB]) {
     if constexpr (K > 0) {
+        unsigned long long u[XB];
 #pragma unroll
         for (int q = 0; q < XB + K - 1; ++q) {
-            const float2 v = src[2 * q];
+            const unsigned long long v = *reinterpret_cast<const unsigned long long *>(src + 2 * q);
 #pragma unroll
             for (int m = 0; m < XB; ++m) {
                 const int tt = q - m;
-                if (tt == 0) acc[m] = fma2(v, c.taps2[0], make_float2(0.f, 0.f));
-                else if (tt > 0 && tt < K) acc[m] = fma2(v, c.taps2[tt], acc[m]);
+                if (tt >= 0 && tt < K) u[m] = fma2(v, c.tap2(tt), tt == 0 ? 0ull : u[m]);
             }
         }
+#pragma unroll
+        for (int m = 0; m < XB; ++m) acc[m] = unpack2(u[m]);
     } else {
 #pragma unroll
         for (int m = 0; m < XB; ++m) acc[m] = make_float2(0.f, 0.f);
@@ -94,7 +94,7 @@ __device__ __forceinline__ void xconv_pair(const float2 *src, const StepConst &c
 template <int K, int XB, Arith A>
 __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__restrict__ svs,
                                                               const int *__restrict__ pre,
-                                                              const StepConst c, int parity) {
+                                                              const __grid_constant__ StepConst c, int parity) {
     extern __shared__ float4 sm4[];
     constexpr int XT = 32 * XB;
     const int k = K > 0 ? K : c.k;
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__
         const float *phi = (parity ? s.phi[1] : s.phi[0]) + row;
         if constexpr (K > 0) {
             // all of the lane's loads first, so that they are in flight together
-            constexpr int NE = (XT + K - 1 + 31) / 32;
+            constexpr int NE = ((XT + K - 1 + 31) / 32 + 1) & ~1;
             float ph[NE], im[NE];
 #pragma unroll
             for (int q = 0; q < NE; ++q) {
@@ -135,18 +135,15 @@ __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__
                 ph[q] = ok ? __ldg(phi + x) : 0.0f;
                 im[q] = ok ? load_img(s.img, row + x, c.img_f32) : 0.0f;
             }
+            // (elements past the row feed only outputs past Wv)
 #pragma unroll
-            for (int q = 0; q < NE; ++q) {
+            for (int q = 0; q < NE; q += 2) {
                 const int e = lane + 32 * q;
-                if (e < span) {
-                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (x0 + e < s.W) {
-                        const float h = heaviside<A>(ph[q], c.eps);
-                        const float hi = __fsub_rn(1.0f, h);
-                        v = make_float4(h, hi, __fmul_rn(im[q], h), __fmul_rn(im[q], hi));
-                    }
-                    in[e] = v;
-                }
+                const float2 h = heaviside2<A>(make_float2(ph[q], ph[q + 1]), c.eps, c.pk);
+                const float2 hi = sub2(dup2(1.0f), h);
+                if (e < span) in[e] = make_float4(h.x, hi.x, __fmul_rn(im[q], h.x), __fmul_rn(im[q], hi.x));
+                if (e + 32 < span)
+                    in[e + 32] = make_float4(h.y, hi.y, __fmul_rn(im[q + 1], h.y), __fmul_rn(im[q + 1], hi.y));
             }
         } else {
             for (int e = lane; e < span; e += 32) {
@@ -169,8 +166,7 @@ __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__
         const float2 *src = reinterpret_cast<const float2 *>(in + XB * lane);
         float2 acc[XB];
         if constexpr (K > 0) {
-            // two float2 pair planes: each pair's results are staged as float2
-            // and written as float4 (two columns)
+            // each pair's results are staged as float2 and written together
             float2 *s01 = reinterpret_cast<float2 *>(st01), *s23 = reinterpret_cast<float2 *>(st23);
             xconv_pair<K, XB>(src, c, taps_s, k, acc);
 #pragma unroll
@@ -180,14 +176,12 @@ __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__
 #pragma unroll
             for (int m = 0; m < XB; ++m) s23[XB * lane + m] = acc[m];
             __syncwarp();
-            const size_t pstride = (size_t)s.Wp * s.H * s.L;
-            const size_t orow = ((size_t)z * s.H + y) * s.Wp;
+            float4 *dst = reinterpret_cast<float4 *>(s.xb) + ((size_t)z * s.H + y) * s.Wp + x0;
 #pragma unroll
-            for (int pp = 0; pp < 2; ++pp) {
-                const float4 *sf = reinterpret_cast<const float4 *>(pp ? s23 : s01);
-                float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float2 *>(s.xb) + pp * pstride + orow + x0);
-                for (int e = lane; e < XT / 2; e += 32)
-                    if (x0 + 2 * e < s.Wv) dst[e] = sf[e];
+            for (int q = 0; q < XB; ++q) {
+                const int e = lane + 32 * q;
+                const float2 a = s01[e], b = s23[e];
+                if (x0 + e < s.Wv) dst[e] = make_float4(a.x, a.y, b.x, b.y);
             }
         } else {
             xconv_pair<K, XB>(src, c, taps_s, k, acc);
@@ -248,31 +242,15 @@ struct Ring {
     size_t stride;
     int n;
     bool act;         // inactive threads load nothing (their results are discarded)
-    // Optional side stream riding in the same commit groups: with element i
-    // comes the aligned 32-bit word holding byte side + (i - lag) * sstride,
-    // for i >= first.  The word around a valid byte stays inside that byte's
-    // 4-byte-aligned block, so it never touches another allocation.
-    unsigned *sbase = nullptr;
-    const unsigned char *side = nullptr;
-    size_t sstride = 0;
-    int lag = 0, first = 0;
-    bool sact = false;
     __device__ __forceinline__ float2 *slot(int i) const { return base + (i & (RING - 1)) * step; }
-    __device__ __forceinline__ unsigned *sslot(int i) const { return sbase + (i & (RING - 1)) * step; }
-    __device__ __forceinline__ const unsigned char *sbyte(int i) const { return side + (size_t)(i - lag) * sstride; }
     __device__ __forceinline__ void fill(int i) const {
-        if (act && i < n) {
-            cp_async8(slot(i), src + (size_t)i * stride);
-            if (sact && i >= first)
-                cp_async4(sslot(i),
-                          reinterpret_cast<const void *>(reinterpret_cast<uintptr_t>(sbyte(i)) & ~(uintptr_t)3));
-        }
+        if (act && i < n) cp_async8(slot(i), src + (size_t)i * stride);
     }
 };
 
 template <int K, bool GUARD, typename Emit>
-__device__ __forceinline__ void stream_block(const Ring &rg, int base, const StepConst &c, float2 (&acc)[K],
-                                             Emit &emit) {
+__device__ __forceinline__ void stream_block(const Ring &rg, int base, const StepConst &c,
+                                             unsigned long long (&acc)[K], Emit &emit) {
 #pragma unroll
     for (int j = 0; j < K; ++j) {
         const int i = base + j;
@@ -282,15 +260,14 @@ __device__ __forceinline__ void stream_block(const Ring &rg, int base, const Ste
             cp_commit();
         }
         cp_wait_ring();
-        const float2 v = *rg.slot(i);
+        const unsigned long long v = *reinterpret_cast<const unsigned long long *>(rg.slot(i));
 #pragma unroll
         for (int tt = 0; tt < K; ++tt) {
             const int slot = (j - tt + K) % K;
-            if (tt == 0) acc[slot] = fma2(v, c.taps2[0], make_float2(0.f, 0.f));
-            else acc[slot] = fma2(v, c.taps2[tt], acc[slot]);
+            acc[slot] = fma2(v, c.tap2(tt), tt == 0 ? 0ull : acc[slot]);
         }
         const int o = i - (K - 1);
-        if (o >= 0) emit(o, acc[(j + 1) % K], i);
+        if (o >= 0) emit(o, unpack2(acc[(j + 1) % K]), i);
     }
 }
 
@@ -301,103 +278,14 @@ __device__ __forceinline__ void stream_axis(const Ring &rg, const StepConst &c, 
         rg.fill(q);
         cp_commit();
     }
-    float2 acc[K];
+    unsigned long long acc[K];
 #pragma unroll
-    for (int j = 0; j < K; ++j) acc[j] = make_float2(0.f, 0.f);
+    for (int j = 0; j < K; ++j) acc[j] = 0ull;
     int base = 0;
     for (; base + K <= rg.n; base += K) stream_block<K, false>(rg, base, c, acc, emit);
     if (base < rg.n) stream_block<K, true>(rg, base, c, acc, emit);
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
-
-// Ring with compile-time slots, for tap counts that are a multiple of the
-// ring depth RD (21 and 35 with RD = 7, 29 with RD = 29).  Blocks of K
-// elements start at multiples of K, so element base + j sits in slot j % RD,
-// a constant of the unrolled block; the global addresses advance by one stride per element
-// instead of being recomputed.  Same commit-group protocol as Ring: element
-// i is group i; iteration i refills the slot of element i-1 with element
-// i-1+RD and then waits until at most RD-1 groups are pending.
-template <int RD>
-__device__ __forceinline__ void cp_wait_depth() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(RD - 1) : "memory");
-}
-
-template <int RD>
-struct RingC {
-    float2 *base;              // this thread's slot 0; slot q at base + q * step
-    int step;
-    const float *next;         // global address of element `nfill`
-    size_t stride;
-    int nfill, n;
-    bool act;
-    // side stream: the aligned word around byte snext for elements >= sfirst
-    unsigned *sbase = nullptr;
-    const unsigned char *snext = nullptr;
-    size_t sstride = 0;
-    int sfirst = 0;
-    bool sact = false;
-    // `slot` is a constant after the caller's loop is unrolled
-    __device__ __forceinline__ void fill(int slot) {
-        if (act && nfill < n) {
-            cp_async8(base + slot * step, next);
-            if (sact && nfill >= sfirst)
-                cp_async4(sbase + slot * step,
-                          reinterpret_cast<const void *>(reinterpret_cast<uintptr_t>(snext) & ~(uintptr_t)3));
-        }
-        next += stride;  // addresses past the end are formed but never read
-        if (nfill >= sfirst) snext += sstride;
-        ++nfill;
-    }
-};
-
-template <int K, int RD, bool FIRST, bool GUARD, typename Emit>
-__device__ __forceinline__ void stream_block_c(RingC<RD> &rg, int base, const StepConst &c, float2 (&acc)[K],
-                                               Emit &emit) {
-    static_assert(K % RD == 0, "the ring depth must divide the tap count");
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-        if (GUARD && base + j >= rg.n) break;
-        if (!(FIRST && j == 0)) {
-            rg.fill((j - 1 + RD) % RD);
-            cp_commit();
-        }
-        cp_wait_depth<RD>();
-        const float2 v = rg.base[(j % RD) * rg.step];
-#pragma unroll
-        for (int tt = 0; tt < K; ++tt) {
-            const int slot = (j - tt + K) % K;
-            if (tt == 0) acc[slot] = fma2(v, c.taps2[0], make_float2(0.f, 0.f));
-            else acc[slot] = fma2(v, c.taps2[tt], acc[slot]);
-        }
-        if (!FIRST || j >= K - 1) emit(base + j - (K - 1), acc[(j + 1) % K], j % RD);
-    }
-}
-
-template <int K, int RD, typename Emit>
-__device__ __forceinline__ void stream_axis_c(RingC<RD> &rg, const StepConst &c, Emit &emit) {
-#pragma unroll
-    for (int q = 0; q < RD; ++q) {
-        rg.fill(q);
-        cp_commit();
-    }
-    float2 acc[K];
-#pragma unroll
-    for (int j = 0; j < K; ++j) acc[j] = make_float2(0.f, 0.f);
-    if (rg.n < K) {
-        stream_block_c<K, RD, true, true>(rg, 0, c, acc, emit);
-    } else {
-        stream_block_c<K, RD, true, false>(rg, 0, c, acc, emit);
-        int base = K;
-        for (; base + K <= rg.n; base += K) stream_block_c<K, RD, false, false>(rg, base, c, acc, emit);
-        if (base < rg.n) stream_block_c<K, RD, false, true>(rg, base, c, acc, emit);
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
-// Depth of the compile-time ring of a specialised tap count: 7 for 21 and
-// 35; 29 (prime) takes a ring as deep as its taps (44.5 KB of shared memory
-// per block, within what its registers already allow per SM).
-__host__ __device__ constexpr int ring_depth(int K) { return K % 7 == 0 ? 7 : K == 29 ? 29 : RING; }
 
 // Register-blocked version for a tap count known only at run time: NB
 // consecutive outputs per call, same accumulation order.
@@ -418,31 +306,28 @@ __device__ __forceinline__ void conv_block_rt(const float *__restrict__ base, si
 }
 
 // ---------------------------------------------------------------------------
-// y-pass.  One thread streams one column of one pair plane of one z plane
-// (float2 elements: both fields of the pair, one packed multiply-add).
+// y-pass.  One thread streams one column of one pair (every other float2 of
+// the interleaved fields): the 2 Wp float2 columns of a z plane, over all
+// planes, are numbered consecutively.
 // ---------------------------------------------------------------------------
 template <int K>
 __global__ void __launch_bounds__(YP_COLS) ypass_kernel(const SubVolDev *__restrict__ svs,
-                                                        const int *__restrict__ pre, const StepConst c) {
+                                                        const int *__restrict__ pre,
+                                                        const __grid_constant__ StepConst c) {
     const int b = blockIdx.x;
     const int sv = find_sv(pre, c.nsv, b);
     const SubVolDev s = svs[sv];
-    int t = b - __ldg(pre + sv);
-    const int ntx = (s.Wv + YP_COLS - 1) / YP_COLS;
-    const int tx = t % ntx;
-    t /= ntx;
-    const int p = t & 1;
-    const int z = t >> 1;
+    const long long q = (long long)(b - __ldg(pre + sv)) * YP_COLS + threadIdx.x;
+    const int row = 2 * s.Wp;
+    const int z = (int)(q / row), x = (int)(q - (long long)z * row);
     __shared__ float2 ring[RING * YP_COLS];
-    const int x = tx * YP_COLS + threadIdx.x;
-    if (x >= s.Wv) return;
-    const float *src = s.xb + 2 * ((size_t)p * s.Wp * s.H * s.L + (size_t)z * s.H * s.Wp + x);
-    float2 *dst = reinterpret_cast<float2 *>(s.yb) + (size_t)p * s.Wp * s.Hv * s.L + (size_t)z * s.Hv * s.Wp + x;
-    const size_t wp = (size_t)s.Wp;
+    if (z >= s.L || x >= 2 * s.Wv) return;
+    const float *src = s.xb + 2 * ((size_t)z * s.H * row + x);
+    float2 *dst = reinterpret_cast<float2 *>(s.yb) + (size_t)z * s.Hv * row + x;
     // The y-pass is bound by HBM bandwidth: it keeps the deeper 8-slot ring
     // (more loads in flight) rather than the compile-time-slot ring.
-    auto emit = [&](int o, float2 v, int) { dst[(size_t)o * wp] = v; };
-    const Ring rg = {ring + threadIdx.x, YP_COLS, src, 2 * wp, s.H, true};
+    auto emit = [&](int o, float2 v, int) { dst[(size_t)o * row] = v; };
+    const Ring rg = {ring + threadIdx.x, YP_COLS, src, 2 * (size_t)row, s.H, true};
     stream_axis<K>(rg, c, emit);
 }
 
@@ -478,252 +363,206 @@ __global__ void __launch_bounds__(YB_TX) ypass_generic_kernel(const SubVolDev *_
 }
 
 // ---------------------------------------------------------------------------
-// z-pass.  Four lanes per column pair, one field each, streaming z.  When an
-// output plane completes, the lanes exchange their blurred values so that
-// each lane forms one local fit (f_out or f_in of one of the two columns) and
-// its e term; lanes 0 and 2 of the group write lambda (e_out - e_in).
+// z-pass.  One thread streams one column of all four fields (float4 elements),
+// so that it forms both local fits of its voxel by itself: 2 K rotating
+// accumulator pairs, inputs through a per-thread ring of float4 slots filled by
+// cp.async.  The kernel is bound by instruction issue, and everything but the
+// multiply-adds is paid once per voxel this way (with the two pairs on
+// different lanes it took 186 thread instructions per voxel, 21 taps, and
+// 6.78 ms per launch on the 48 sub-volumes of 946 M voxels; now 3.70 ms).
+// The ring's depth divides the taps (7 for 21 and 35; 29 needs 29), so every
+// slot index of a K-element block is a constant; element i is commit group i,
+// and iteration i refills the slot of element i-1 with element i-1+RD before it
+// waits for group i.  A block takes ZP_COLS columns, numbered consecutively
+// over the padded rows of a plane, and c.zout output planes.
 // ---------------------------------------------------------------------------
-// x column of lane f of a 4-lane group (column pair x, x+1): with the four
-// separate y fields lane f streams field f of both columns; with the pair
-// layout lane f streams pair f >> 1 of column x + (f & 1).
-template <bool PAIRS>
-__device__ __forceinline__ int zlane_col(int x, int f) {
-    return PAIRS ? x + (f & 1) : x + (f >> 1);
-}
+__host__ __device__ constexpr int ring_depth(int K) { return K % 7 == 0 ? 7 : K; }
+__host__ __device__ constexpr size_t zpass_smem(int K) { return (size_t)ring_depth(K) * ZP_COLS * sizeof(float4); }
 
-template <bool PAIRS>
-__device__ __forceinline__ void fits_and_data(const SubVolDev &s, const StepConst &c, int f, int x, int y, int o,
-                                              bool live, float I, float2 B, const DebugOut &dbg, bool debug) {
-    // Separate fields: B = (field f at x, field f at x+1); lane f forms
-    //   0 -> f_out(x), 1 -> f_in(x), 2 -> f_out(x+1), 3 -> f_in(x+1).
-    // Pair layout: B = (pair f>>1 at column x + (f&1)); lane f forms
-    //   0 -> f_out(x), 1 -> f_out(x+1), 2 -> f_in(x), 3 -> f_in(x+1).
-    // Both are num / den with num = lane f+2's B.x for f < 2, else B.y, and
-    // den = B.x for f < 2, else lane f-2's B.y.  I is the image at the
-    // lane's voxel (prefetched by the caller).
-    const float bx_hi = __shfl_down_sync(0xffffffffu, B.x, 2);
-    const float by_lo = __shfl_up_sync(0xffffffffu, B.y, 2);
-    const float num = f < 2 ? bx_hi : B.y;
-    const float den = f < 2 ? B.x : by_lo;
-    const float fv = __fdiv_rn(num, den);
-    const int xc = zlane_col<PAIRS>(x, f);
-    const float d = __fsub_rn(I, fv);
-    const float e = __fmul_rn(d, d);
-    // the lane holding f_out of a column gets that column's e_in
-    const float e_in = __shfl_down_sync(0xffffffffu, e, PAIRS ? 2 : 1);
-    const bool outer = PAIRS ? f < 2 : (f & 1) == 0;
-    if (live && outer)
-        s.db[((size_t)o * s.Hv + y) * s.Wp + xc] = data_factor(e, e_in, c.l1, c.l2, c.lam_equal != 0);
-    if (debug && live) {
-        const int r = c.r;
-        const int fin = outer ? 0 : 1;
-        const size_t vi = ((size_t)(o + r) * s.H + (y + r)) * s.W + (xc + r);
-        dbg.f[(size_t)fin * dbg.n + vi] = fv;
-        dbg.f[(size_t)(2 + fin) * dbg.n + vi] = e;
+// One block of K elements.  The steady form has no branch, so that the fits of
+// one element overlap the multiply-adds of the next (with the end tested inside
+// it, and one copy of the body for start, middle and end, the 21-tap kernel
+// took 6.4 ms per launch instead of 3.5).
+template <int K, bool FIRST, bool GUARD, class Fill, class Emit>
+__device__ __forceinline__ void zstream_block(const ulonglong2 *ring, int left, const StepConst &c,
+                                              unsigned long long (&a)[K], unsigned long long (&b)[K], Fill &fill,
+                                              Emit &emit) {
+    constexpr int RD = ring_depth(K);
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        if (GUARD && j >= left) break;
+        fill((j - 1 + RD) % RD);
+        asm volatile("cp.async.wait_group %0;" ::"n"(RD - 1) : "memory");
+        const ulonglong2 v = ring[(j % RD) * ZP_COLS];
+#pragma unroll
+        for (int tt = 0; tt < K; ++tt) {
+            const int s = (j - tt + K) % K;
+            if (FIRST && tt > j) continue;  // an output that starts before element 0
+            a[s] = fma2(v.x, c.tap2(tt), tt == 0 ? 0ull : a[s]);
+            b[s] = fma2(v.y, c.tap2(tt), tt == 0 ? 0ull : b[s]);
+        }
+        if (!FIRST || j == K - 1) emit(unpack2(a[(j + 1) % K]), unpack2(b[(j + 1) % K]));
     }
 }
 
-// The streaming z-pass of one block (tile t of sub-volume s): every lane
-// gets its column's blurred pair at each output plane o and the image there,
-// and hands them to fits(f, x, y, o, live, I, B), which all lanes of the warp
-// call together (it may shuffle), for o = 0, 1, ..., Lv - 1 in order.
-// begin(xc, y, live) runs first, with the lane's output column xc.
-template <int K, bool PAIRS, class Begin, class Fits>
-__device__ __forceinline__ void zpass_body(const SubVolDev &s, const StepConst &c, int t, Begin begin, Fits fits) {
-    const int ntx = (s.Wv + 2 * ZP_PAIRS - 1) / (2 * ZP_PAIRS);
-    const int tx = t % ntx;
-    const int y = t / ntx;
-    const int f = threadIdx.x & 3;
-    const int x = 2 * (tx * ZP_PAIRS + (threadIdx.x >> 2));
-    const bool act = x < s.Wv;
-    // separate fields: field f, column pair x; pair layout: pair f >> 1,
-    // column x + (f & 1), float2 elements (plane stride in floats doubles)
-    const float *src = PAIRS ? s.yb + (size_t)(f >> 1) * 2 * ((size_t)s.Wp * s.Hv * s.L) +
-                                   2 * ((size_t)y * s.Wp + (act ? x + (f & 1) : 0))
-                             : s.yb + f * ((size_t)s.Wp * s.Hv * s.L) + (size_t)y * s.Wp + (act ? x : 0);
-    const size_t pstride = (PAIRS ? 2 : 1) * (size_t)s.Wp * s.Hv;
-    constexpr int RS = ring_depth(K) > RING ? ring_depth(K) : RING;
-    __shared__ float2 ring[RS * ZP_PAIRS * 4];
-    __shared__ unsigned iring[RS * ZP_PAIRS * 4];
-    // The image at this lane's voxel of output plane o (input plane o + r)
-    // rides in the ring with element i = o + 2r.
-    const int xc = zlane_col<PAIRS>(x, f);
-    const bool live = act && xc < s.Wv;
-    const size_t esz = c.img_f32 ? 4 : 1;
-    const unsigned char *img0 = static_cast<const unsigned char *>(s.img) +
-                                (((size_t)(y + c.r)) * s.W + (size_t)(xc + c.r)) * esz;
-    const size_t sstride = (size_t)s.W * s.H * esz;
-    begin(xc, y, live);
-    if constexpr (K % ring_depth(K) == 0 && ring_depth(K) != RING) {
-        constexpr int RD = ring_depth(K);
-        RingC<RD> rg = {ring + threadIdx.x, ZP_PAIRS * 4, src, pstride, 0, s.L, act};
-        rg.sbase = iring + threadIdx.x;
-        rg.snext = img0 + (size_t)c.r * sstride;  // element 2r carries plane r, the first output's
-        rg.sstride = sstride;
-        rg.sfirst = 2 * c.r;
-        rg.sact = live;
-        // low two bits of the byte address of output o's image voxel:
-        // (shift0 + o * sstride) mod 4
-        const unsigned shift0 = (unsigned)(reinterpret_cast<uintptr_t>(img0 + (size_t)c.r * sstride) & 3);
-        const unsigned shift_step = (unsigned)(sstride & 3);
-        auto emit = [&](int o, float2 v, int slot) {
-            float I = 0.0f;
-            if (live) {
-                const unsigned wd = rg.sbase[slot * rg.step];
-                if (c.img_f32) I = __uint_as_float(wd);
-                else I = (float)((wd >> (8 * ((shift0 + (unsigned)o * shift_step) & 3u))) & 0xffu);
-            }
-            fits(f, x, y, o, live, I, v);
-        };
-        stream_axis_c<K, RD>(rg, c, emit);
-    } else {
-        Ring rg = {ring + threadIdx.x, ZP_PAIRS * 4, src, pstride, s.L, act};
-        rg.sbase = iring + threadIdx.x;
-        rg.side = img0;
-        rg.sstride = sstride;
-        rg.lag = c.r;
-        rg.first = 2 * c.r;
-        rg.sact = live;
-        auto emit = [&](int o, float2 v, int i) {
-            float I = 0.0f;
-            if (live) {
-                const unsigned wd = *rg.sslot(i);
-                if (c.img_f32) I = __uint_as_float(wd);
-                else I = (float)((wd >> (8 * (unsigned)(reinterpret_cast<uintptr_t>(rg.sbyte(i)) & 3))) & 0xffu);
-            }
-            fits(f, x, y, o, live, I, v);
-        };
-        stream_axis<K>(rg, c, emit);
-    }
+// Rotating accumulation of n inputs (n >= K) src[i * stride]: hands
+// emit(pair 0, pair 1) the outputs 0 .. n - K in order.
+template <int K, class Emit>
+__device__ __forceinline__ void zstream(const float4 *src, size_t stride, int n, const StepConst &c, Emit emit) {
+    constexpr int RD = ring_depth(K);
+    extern __shared__ ulonglong2 zring_s[];
+    ulonglong2 *ring = zring_s + threadIdx.x;
+    const float4 *next = src;
+    int unread = n;
+    auto fill = [&](int slot) {
+        if (unread > 0) {
+            const unsigned d = (unsigned)__cvta_generic_to_shared(ring + slot * ZP_COLS);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(next) : "memory");
+        }
+        next += stride;  // addresses past the end are formed but never read
+        --unread;
+        cp_commit();
+    };
+#pragma unroll
+    for (int q = 0; q + 1 < RD; ++q) fill(q);
+    unsigned long long a[K], b[K];
+    zstream_block<K, true, false>(ring, K, c, a, b, fill, emit);
+    int left = n - K;
+    for (; left >= K; left -= K) zstream_block<K, false, false>(ring, left, c, a, b, fill, emit);
+    if (left > 0) zstream_block<K, false, true>(ring, left, c, a, b, fill, emit);
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-template <int K, bool DEBUG, bool PAIRS = false>
-__global__ void __launch_bounds__(ZP_PAIRS * 4) zpass_kernel(const SubVolDev *__restrict__ svs,
-                                                             const int *__restrict__ pre, const StepConst c,
-                                                             DebugOut dbg) {
-    const int b = blockIdx.x;
-    const int sv = find_sv(pre, c.nsv, b);
+// The column of this thread: offset p within a plane of the padded fields, valid
+// x and y, outputs [o0, o0 + n).
+struct ZCol {
+    size_t p, plane;   // plane: Wp * Hv
+    int x, y, o0, n;
+    bool live;
+};
+__device__ __forceinline__ ZCol zcol_of(const SubVolDev &s, const StepConst &c, int t) {
+    ZCol z;
+    z.plane = (size_t)s.Wp * s.Hv;
+    const int ntp = (int)((z.plane + ZP_COLS - 1) / ZP_COLS);
+    z.p = (size_t)(t % ntp) * ZP_COLS + threadIdx.x;
+    z.y = (int)(z.p / s.Wp);
+    z.x = (int)(z.p - (size_t)z.y * s.Wp);
+    z.o0 = (t / ntp) * c.zout;
+    z.n = min(c.zout, s.Lv - z.o0);
+    z.live = z.p < z.plane && z.x < s.Wv;
+    return z;
+}
+
+// The image at an address, as the bits that image_value turns into a float
+// once it is needed (loads run three outputs ahead).
+__device__ __forceinline__ unsigned image_bits(const unsigned char *ip, int f32) {
+    return f32 ? __ldg(reinterpret_cast<const unsigned *>(ip)) : (unsigned)__ldg(ip);
+}
+__device__ __forceinline__ float image_value(unsigned w, int f32) { return f32 ? __uint_as_float(w) : (float)w; }
+
+template <int K>
+__global__ void __launch_bounds__(ZP_COLS, zpass_blocks(K)) zpass_kernel(const SubVolDev *__restrict__ svs,
+                                                                         const int *__restrict__ pre,
+                                                                         const __grid_constant__ StepConst c) {
+    const int blk = blockIdx.x;
+    const int sv = find_sv(pre, c.nsv, blk);
     const SubVolDev s = svs[sv];
-    zpass_body<K, PAIRS>(
-        s, c, b - __ldg(pre + sv), [](int, int, bool) {},
-        [&](int f, int x, int y, int o, bool live, float I, float2 v) {
-            fits_and_data<PAIRS>(s, c, f, x, y, o, live, I, v, dbg, DEBUG);
-        });
+    const ZCol z = zcol_of(s, c, blk - __ldg(pre + sv));
+    if (!z.live) return;  // no barrier or shuffle below
+    const size_t esz = c.img_f32 ? 4 : 1, istep = (size_t)s.W * s.H * esz;
+    const unsigned char *ip = static_cast<const unsigned char *>(s.img) +
+                              (((size_t)(z.o0 + c.r) * s.H + (z.y + c.r)) * s.W + (z.x + c.r)) * esz;
+    float *db = s.db + (size_t)z.o0 * z.plane + z.p;
+    int unread = z.n;  // image words not yet loaded
+    auto image = [&] {
+        const unsigned w = unread > 0 ? image_bits(ip, c.img_f32) : 0u;
+        ip += istep;
+        --unread;
+        return w;
+    };
+    unsigned i0 = image(), i1 = image(), i2 = image();
+    zstream<K>(reinterpret_cast<const float4 *>(s.yb) + (size_t)z.o0 * z.plane + z.p, z.plane, z.n + K - 1, c,
+               [&](float2 h, float2 ih) {
+                   const float I = image_value(i0, c.img_f32);
+                   i0 = i1;
+                   i1 = i2;
+                   i2 = image();
+                   const float2 f = div2(ih, h);  // f_out, f_in
+                   const float d0 = __fsub_rn(I, f.x), d1 = __fsub_rn(I, f.y);
+                   *db = data_factor(__fmul_rn(d0, d0), __fmul_rn(d1, d1), c.l1, c.l2, c.lam_equal != 0);
+                   db += z.plane;
+               });
 }
 
-// The same z-pass bounded only to two resident blocks per SM.  For 35 taps
-// the default bounds hold it to 128 registers with a 56-byte spill of the 35
-// accumulator pairs; this one takes 164 registers without a spill (3 blocks
-// per SM instead of 4) and measured 1.43 against 1.89 ms per launch on a
-// 512^3 volume.
-template <int K, bool PAIRS>
-__global__ void __launch_bounds__(ZP_PAIRS * 4, 2) zpass_wide_kernel(const SubVolDev *__restrict__ svs,
-                                                                     const int *__restrict__ pre,
-                                                                     const StepConst c) {
-    const int b = blockIdx.x;
-    const int sv = find_sv(pre, c.nsv, b);
-    const SubVolDev s = svs[sv];
-    const DebugOut none = {nullptr, 0};
-    zpass_body<K, PAIRS>(
-        s, c, b - __ldg(pre + sv), [](int, int, bool) {},
-        [&](int f, int x, int y, int o, bool live, float I, float2 v) {
-            fits_and_data<PAIRS>(s, c, f, x, y, o, live, I, v, none, false);
-        });
-}
-
-// The adjoint's recompute of the fits (rsf_adjoint.cu): the forward z-pass
-// over pair planes, emitting at each valid voxel, instead of the data factor,
+// The adjoint's recompute of the fits (rsf_adjoint.cu): the forward z-pass,
+// emitting at each valid voxel, instead of the data factor,
 //   e_out = (I - f_out)^2 and e_in at the full-volume index, and the pair
 //   (B1_bar - B3_bar, B2_bar - B4_bar) in the valid layout (row stride Wv),
 // with B1..B4 the blurs of I H, H, I (1-H), 1-H, f_out = B1 / B2,
 // f_in = B3 / B4, and for data_bar = -u dt delta(phi)
 //   f_out_bar = -2 (I - f_out) lambda1 data_bar, f_in_bar = 2 (I - f_in) lambda2 data_bar,
 //   B1_bar = f_out_bar / B2, B2_bar = -f_out_bar f_out / B2 (B3, B4 alike).
-// ph, uo: phi and u at the lane's voxel of output plane o.  The pair goes to
-// a.xs (2 Wv Hv Lv floats), e_out and e_in to a.xs + 2 N and a.xs + 3 N.
-__device__ __forceinline__ void adjoint_fits(const SubVolDev &s, const StepConst &c, const AdjVol &a, int f, int x,
-                                             int y, int o, bool live, float I, float2 B, float ph, float uo) {
-    // lanes as in fits_and_data's pair layout: 0, 1 -> f_out at x, x + 1;
-    // 2, 3 -> f_in at x, x + 1
-    const float bx_hi = __shfl_down_sync(0xffffffffu, B.x, 2);
-    const float by_lo = __shfl_up_sync(0xffffffffu, B.y, 2);
-    const bool outer = f < 2;
-    const float num = outer ? bx_hi : B.y;
-    const float den = outer ? B.x : by_lo;
-    const int xc = x + (f & 1);
-    const size_t vi = ((size_t)(o + c.r) * s.H + (y + c.r)) * s.W + (xc + c.r);
-    float bn = 0.0f, bd = 0.0f, e = 0.0f;
-    if (live) {
-        const float rb = __frcp_rn(den);
-        const float fv = num * rb;
-        const float d = I - fv;
-        e = d * d;
-        const float delta = __fdividef(0.318309886183790672f * c.eps, fmaf(ph, ph, c.eps * c.eps));
-        const float data_bar = -uo * c.dt * delta;
-        const float fbar = -2.0f * d * (outer ? c.l1 * data_bar : -c.l2 * data_bar);
-        bn = fbar * rb;
-        bd = -fbar * fv * rb;
-    }
-    const float bn_in = __shfl_down_sync(0xffffffffu, bn, 2);
-    const float bd_in = __shfl_down_sync(0xffffffffu, bd, 2);
-    if (live) {
-        const size_t n = (size_t)s.W * s.H * s.L;
-        if (outer) {
-            const size_t nv = (size_t)s.Wv * s.Hv * s.Lv;
-            const size_t vo = ((size_t)o * s.Hv + y) * s.Wv + xc;
-            a.xs[vo] = bn - bn_in;
-            a.xs[nv + vo] = bd - bd_in;
-            a.xs[2 * n + vi] = e;
-        } else {
-            a.xs[3 * n + vi] = e;
-        }
-    }
-}
-
+// The pair goes to a.xs (2 Wv Hv Lv floats), e_out and e_in to a.xs + 2 N and
+// a.xs + 3 N.  phi and u of the next three output planes ride in registers
+// with the image.
 template <int K>
-__global__ void __launch_bounds__(ZP_PAIRS * 4) zpass_adjoint_kernel(const SubVolDev *__restrict__ svs,
-                                                                     const int *__restrict__ pre, const StepConst c,
-                                                                     const AdjVol *__restrict__ vols) {
-    const int b = blockIdx.x;
-    const int sv = find_sv(pre, c.nsv, b);
+__global__ void __launch_bounds__(ZP_COLS, zpass_blocks(K)) zpass_adjoint_kernel(const SubVolDev *__restrict__ svs,
+                                                                                 const int *__restrict__ pre,
+                                                                                 const __grid_constant__ StepConst c,
+                                                                                 const AdjVol *__restrict__ vols) {
+    const int blk = blockIdx.x;
+    const int sv = find_sv(pre, c.nsv, blk);
     const SubVolDev s = svs[sv];
     const AdjVol a = vols[sv];
-    // phi and u of output planes o, o + 1, o + 2 ride in registers: each
-    // output's loads are issued three planes ahead (the streaming loop is
-    // latency-bound when the volume gives few blocks per SM).
-    const size_t plane = (size_t)s.W * s.H;
-    float p0 = 0.f, p1 = 0.f, p2 = 0.f, u0 = 0.f, u1 = 0.f, u2 = 0.f;
-    size_t vnext = 0;  // offset of the lane's voxel in plane o + 3 + r
-    auto begin = [&](int xc, int y, bool live) {
-        const size_t v0 = ((size_t)c.r * s.H + (y + c.r)) * s.W + (xc + c.r);
-        if (live) {
-            p0 = __ldg(a.phi + v0);
-            u0 = __ldg(a.u + v0);
-            if (s.Lv > 1) {
-                p1 = __ldg(a.phi + v0 + plane);
-                u1 = __ldg(a.u + v0 + plane);
-            }
-            if (s.Lv > 2) {
-                p2 = __ldg(a.phi + v0 + 2 * plane);
-                u2 = __ldg(a.u + v0 + 2 * plane);
-            }
-        }
-        vnext = v0 + 3 * plane;
+    const ZCol z = zcol_of(s, c, blk - __ldg(pre + sv));
+    if (!z.live) return;
+    const size_t esz = c.img_f32 ? 4 : 1, plane = (size_t)s.W * s.H;
+    size_t v = ((size_t)(z.o0 + c.r) * s.H + (z.y + c.r)) * s.W + (z.x + c.r);  // the next load's voxel
+    float *eo = a.xs + 2 * plane * s.L + v, *ei = eo + plane * s.L;
+    const size_t nv = (size_t)s.Wv * s.Hv * s.Lv, vplane = (size_t)s.Wv * s.Hv;
+    float *pq = a.xs + (size_t)z.o0 * vplane + (size_t)z.y * s.Wv + z.x;
+    struct In {
+        unsigned i;
+        float phi, u;
     };
-    zpass_body<K, true>(s, c, b - __ldg(pre + sv), begin,
-                        [&](int f, int x, int y, int o, bool live, float I, float2 v) {
-                            const float ph = p0, uo = u0;
-                            p0 = p1;
-                            u0 = u1;
-                            p1 = p2;
-                            u1 = u2;
-                            if (live && o + 3 < s.Lv) {
-                                p2 = __ldg(a.phi + vnext);
-                                u2 = __ldg(a.u + vnext);
-                            }
-                            vnext += plane;
-                            adjoint_fits(s, c, a, f, x, y, o, live, I, v, ph, uo);
-                        });
+    int unread = z.n;
+    auto load = [&] {
+        In n = {0u, 0.0f, 0.0f};
+        if (unread > 0)
+            n = In{image_bits(static_cast<const unsigned char *>(s.img) + v * esz, c.img_f32), __ldg(a.phi + v),
+                   __ldg(a.u + v)};
+        v += plane;
+        --unread;
+        return n;
+    };
+    In n0 = load(), n1 = load(), n2 = load();
+    zstream<K>(reinterpret_cast<const float4 *>(s.yb) + (size_t)z.o0 * z.plane + z.p, z.plane, z.n + K - 1, c,
+               [&](float2 h, float2 ih) {
+                   const float I = image_value(n0.i, c.img_f32), ph = n0.phi, uo = n0.u;
+                   n0 = n1;
+                   n1 = n2;
+                   n2 = load();
+                   const float delta = __fdividef(0.318309886183790672f * c.eps, fmaf(ph, ph, c.eps * c.eps));
+                   const float data_bar = -uo * c.dt * delta;
+                   auto side = [&](float num, float den, float weight, float &bn, float &bd) {
+                       const float rb = __frcp_rn(den);
+                       const float fv = num * rb;
+                       const float d = I - fv;
+                       const float fbar = -2.0f * d * (weight * data_bar);
+                       bn = fbar * rb;
+                       bd = -fbar * fv * rb;
+                       return d * d;
+                   };
+                   float bn0, bd0, bn1, bd1;
+                   const float e0 = side(ih.x, h.x, c.l1, bn0, bd0), e1 = side(ih.y, h.y, -c.l2, bn1, bd1);
+                   *eo = e0;
+                   *ei = e1;
+                   pq[0] = bn0 - bn1;
+                   pq[nv] = bd0 - bd1;
+                   eo += plane;
+                   ei += plane;
+                   pq += vplane;
+               });
 }
 
 template <bool DEBUG>

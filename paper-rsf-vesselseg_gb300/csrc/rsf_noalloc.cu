@@ -114,7 +114,7 @@ extern "C" rsf_status rsf_evolve_noalloc(const rsf_params *p, const void *image,
 
     rsf::SubVolDev *d_table = reinterpret_cast<rsf::SubVolDev *>(base);
     int *d_pre = reinterpret_cast<int *>(base + 1024);
-    unsigned char *d_map = base + 2048;  // TMA map of the y-pass pair planes
+    unsigned char *d_map = base + 2048;  // TMA map of the y-pass fields
     unsigned *d_flag = reinterpret_cast<unsigned *>(base + kTableBytes);
     float *phi2 = reinterpret_cast<float *>(base + kTableBytes + kFlagBytes);
     float *xfields = reinterpret_cast<float *>(base + kTableBytes + kFlagBytes + kPhiBytes);
@@ -163,7 +163,7 @@ extern "C" rsf_status rsf_evolve_noalloc(const rsf_params *p, const void *image,
     c.nsv = 1;
     c.xb_w = sh.xb_w;
     c.xrpw = sh.xrpw;
-    c.pairs = sh.pairs;
+    c.zout = sh.zout;
     c.zc = sh.zc;
     rsf::set_pair_const(c.pk, c.eps, c.dt, c.nu, c.mu);
     alignas(64) unsigned char map[rsf::TMAP_BYTES];

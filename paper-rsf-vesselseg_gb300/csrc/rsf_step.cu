@@ -113,6 +113,27 @@ int choose_xrpw(const int *whl, int n, int k, int xb_w) {
     return rpw;
 }
 
+// Output planes per z-pass block.  A block streams its outputs and the K - 1
+// planes before them, so cutting a column costs K - 1 steps per cut and pays
+// only where the batch leaves the SMs short of warps: the fewest cuts that give
+// every SM its resident blocks, as long as a cut is no shorter than the taps.
+int choose_zout(const int *whl, int n, int k) {
+    const long long want = (long long)zpass_blocks(k) * sm_count();
+    int deepest = 1;
+    for (int i = 0; i < n; i++) deepest = whl[3 * i + 2] > deepest ? whl[3 * i + 2] : deepest;
+    for (int cuts = 1;; cuts++) {
+        const int zout = (deepest - k + cuts) / cuts;
+        long long blocks = 0;
+        for (int i = 0; i < n; i++) {
+            int Wv, Hv, Lv, Wp;
+            valid_extents(whl[3 * i], whl[3 * i + 1], whl[3 * i + 2], k, Wv, Hv, Lv, Wp);
+            if (Wv > 0) blocks += (((long long)Wp * Hv + ZP_COLS - 1) / ZP_COLS) * ((Lv + zout - 1) / (zout > 0 ? zout : 1));
+        }
+        if (zout < 1) return 1;
+        if (blocks >= want || (deepest - k + cuts + 1) / (cuts + 1) < k) return zout;
+    }
+}
+
 LaunchShape choose_shape(const int *whl, int n, int k, int kspec, int gauss) {
     LaunchShape sh;
     std::vector<int> wv((size_t)n);
@@ -123,9 +144,9 @@ LaunchShape choose_shape(const int *whl, int n, int k, int kspec, int gauss) {
     }
     sh.xb_w = choose_xb(wv.data(), n);
     sh.xrpw = choose_xrpw(whl, n, k, sh.xb_w);
-    sh.pairs = kspec > 0 ? 1 : 0;
     sh.zt = tma_z(kspec) && tma_z_requested() && tensor_maps_available() ? 1 : 0;
     sh.zc = choose_zc(whl, n);
+    sh.zout = choose_zout(whl, n, k);
     sh.gauss = gauss;
     return sh;
 }
@@ -150,10 +171,10 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 }  // namespace
 
-// The y-pass pair planes as a 4-D float tensor (2 Wp floats, Hv rows, L planes, 2
-// pairs); the z-pass box is one plane of a ZT_X x ZT_Y column tile of both
-// pairs.  Rows are 8 Wp bytes, a multiple of 32, and the pool offsets keep
-// every base 64-byte aligned, as TMA requires.
+// The y-pass fields as a 4-D float tensor (4 Wp floats, Hv rows, L planes, 1);
+// the z-pass box is one plane of a ZT_X x ZT_Y column tile.  Rows are 16 Wp
+// bytes, a multiple of 64, and the pool offsets keep every base 64-byte
+// aligned, as TMA requires.
 bool tensor_maps_available() { return tensor_map_encoder() != nullptr; }
 
 // The TMA-fed z-pass runs when the environment variable RSF_ZPASS is "tma"
@@ -168,10 +189,10 @@ bool encode_pair_map(void *out, const SubVolDev &d) {
     static_assert(sizeof(CUtensorMap) == TMAP_BYTES, "tensor map size");
     PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
     if (!enc || d.Wv <= 0) return false;
-    const cuuint64_t dims[4] = {2 * (cuuint64_t)d.Wp, (cuuint64_t)d.Hv, (cuuint64_t)d.L, 2};
-    const cuuint64_t row = 8 * (cuuint64_t)d.Wp;
+    const cuuint64_t dims[4] = {4 * (cuuint64_t)d.Wp, (cuuint64_t)d.Hv, (cuuint64_t)d.L, 1};
+    const cuuint64_t row = 16 * (cuuint64_t)d.Wp;
     const cuuint64_t strides[3] = {row, row * d.Hv, row * d.Hv * d.L};
-    const cuuint32_t box[4] = {2 * ZT_X, ZT_Y, 1, 2};
+    const cuuint32_t box[4] = {4 * ZT_X, ZT_Y, 1, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     return enc(static_cast<CUtensorMap *>(out), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, d.yb, dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -185,11 +206,11 @@ void tile_counts(const SubVolDev &d, int kspec, const LaunchShape &sh, int tiles
     tiles[0] = valid ? ((d.Wv + xt - 1) / xt) * ((d.H + xr - 1) / xr) * d.L : 0;
     if (!valid) tiles[1] = 0;
     else if (kspec == 0) tiles[1] = ((d.Wv + YB_TX - 1) / YB_TX) * ((d.Hv + YB_YB - 1) / YB_YB) * 4 * d.L;
-    else tiles[1] = ((d.Wv + YP_COLS - 1) / YP_COLS) * 2 * d.L;  // one column of one pair per thread
+    else tiles[1] = (int)((2LL * d.Wp * d.L + YP_COLS - 1) / YP_COLS);  // one column of one pair per thread
     if (!valid) tiles[2] = 0;
     else if (sh.zt) tiles[2] = ((d.Wv + ZT_X - 1) / ZT_X) * ((d.Hv + ZT_Y - 1) / ZT_Y);
     else if (kspec == 0) tiles[2] = ((d.Wv + ZB_TX - 1) / ZB_TX) * ((d.Lv + ZB_ZB - 1) / ZB_ZB) * d.Hv;
-    else tiles[2] = ((d.Wv + 2 * ZP_PAIRS - 1) / (2 * ZP_PAIRS)) * d.Hv;
+    else tiles[2] = (int)(((long long)d.Wp * d.Hv + ZP_COLS - 1) / ZP_COLS) * ((d.Lv + sh.zout - 1) / sh.zout);
     tiles[3] = ((d.W + ST_OX - 1) / ST_OX) * ((d.H + ST_OY - 1) / ST_OY) * ((d.L + zc - 1) / zc);
     // expanded data term: gauss_x, second y-pass, gauss_z, gauss_border
     const bool g = sh.gauss != 0;
@@ -206,6 +227,9 @@ cudaError_t configure_device() {
     if (e == cudaSuccess) e = config_xpass_21();
     if (e == cudaSuccess) e = config_xpass_29();
     if (e == cudaSuccess) e = config_xpass_35();
+    if (e == cudaSuccess) e = config_zpass_21();
+    if (e == cudaSuccess) e = config_zpass_29();
+    if (e == cudaSuccess) e = config_zpass_35();
     if (e == cudaSuccess) e = config_ztpass_21();
     if (e == cudaSuccess) e = config_ztpass_35();
     if (e == cudaSuccess) e = config_signed_distance();

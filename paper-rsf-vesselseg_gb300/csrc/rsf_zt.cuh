@@ -3,11 +3,10 @@
 // e = (I - f)^2 (kernel.cu:25-55 with sigma2 = 0) and the data factor
 // lambda (e_out - e_in) of the valid region, for 21 and 35 taps.
 //
-// Input: the y-pass output as two float2 pair planes, pair 0 (H, 1-H) and
-// pair 1 (I H, I (1-H)), each Wp x Hv x L.  A block owns a tile of ZT_X x ZT_Y
-// columns and streams z.  One producer thread moves z plane i of the tile's
-// two pair planes into ring slot i mod k with one TMA tile load
-// (cp.async.bulk.tensor, 4-D box {2 ZT_X floats, ZT_Y rows, 1 plane, 2 pairs}).
+// Input: the y-pass output, float4 (H, 1-H, I H, I (1-H)) per voxel of Wp x Hv x
+// L.  A block owns a tile of ZT_X x ZT_Y columns and streams z.  One producer
+// thread moves z plane i of the tile into ring slot i mod k with one TMA tile
+// load (cp.async.bulk.tensor, 4-D box {4 ZT_X floats, ZT_Y rows, 1 plane, 1}).
 // The ring is handed over in groups of ZT_G consecutive planes: each group
 // completes on one "full" mbarrier (the bytes of its ZT_G loads) and is
 // released on one "empty" mbarrier, so a consumer waits and arrives once per
@@ -17,7 +16,7 @@
 // accumulator pairs; in the k-unrolled loop the ring slot, its barrier phase
 // and the accumulator of z-output o (slot o mod k) are constants.  When
 // output o completes, the thread forms one fit with the partner thread of the
-// other pair (lane xor 16) and pair 0 writes lambda (e_out - e_in).  The
+// other pair (lane xor 1) and pair 0 writes lambda (e_out - e_in).  The
 // image word of output o is loaded 3 (21 taps) or 5 (35 taps) outputs ahead
 // into a register ring and converted only when used.
 #pragma once
@@ -51,7 +50,7 @@ __global__ void __launch_bounds__(ZT_THREADS, K <= 21 ? 3 : 1) ztpass_kernel(con
     static_assert(K % AHEAD == 0, "the image ring depth must divide the tap count");
     static_assert(K % ZT_G == 0, "the barrier group must divide the tap count");
     extern __shared__ __align__(128) unsigned char zsm[];
-    float(*slot)[2][ZT_Y][2 * ZT_X] = reinterpret_cast<float(*)[2][ZT_Y][2 * ZT_X]>(zsm);
+    float(*slot)[ZT_Y][4 * ZT_X] = reinterpret_cast<float(*)[ZT_Y][4 * ZT_X]>(zsm);
     uint64_t *full = reinterpret_cast<uint64_t *>(zsm + (size_t)K * ZT_SLOT_BYTES);
     uint64_t *empty = full + NG;
     const int b = blockIdx.x;
@@ -87,13 +86,13 @@ __global__ void __launch_bounds__(ZT_THREADS, K <= 21 ? 3 : 1) ztpass_kernel(con
                 const int first = g * ZT_G, n = min(ZT_G, L - first);
                 mbar_arrive_expect_tx(&full[q], (unsigned)n * ZT_SLOT_BYTES);
                 for (int j = 0; j < n; ++j)
-                    tma_load_4d(&slot[q * ZT_G + j][0][0][0], map, 2 * x0, y0, first + j, 0, &full[q]);
+                    tma_load_4d(&slot[q * ZT_G + j][0][0], map, 4 * x0, y0, first + j, 0, &full[q]);
             }
         }
         return;
     }
-    // consumer: column x, pair p (lanes 0-15 pair 0, 16-31 pair 1)
-    const int yy = warp >> 1, xx = (warp & 1) * 16 + (lane & 15), p = lane >> 4;
+    // consumer: column x, pair p (even lanes pair 0, odd lanes pair 1)
+    const int yy = warp >> 1, xx = (warp & 1) * 16 + (lane >> 1), p = lane & 1;
     const int x = x0 + xx, y = y0 + yy;
     const bool act = x < Wv && y < Hv;
     const int r = c.r;
@@ -114,7 +113,7 @@ __global__ void __launch_bounds__(ZT_THREADS, K <= 21 ? 3 : 1) ztpass_kernel(con
     };
     float *dbp = s.db + (size_t)y * s.Wp + x;
     const size_t db_plane = (size_t)s.Wp * Hv;
-    const float2 *vsrc = reinterpret_cast<const float2 *>(&slot[0][p][yy][2 * xx]);
+    const float2 *vsrc = reinterpret_cast<const float2 *>(&slot[0][yy][4 * xx + 2 * p]);
     constexpr int kSlot = (int)(ZT_SLOT_BYTES / sizeof(float2));
     unsigned img[AHEAD];
 #pragma unroll
@@ -159,12 +158,12 @@ __global__ void __launch_bounds__(ZT_THREADS, K <= 21 ? 3 : 1) ztpass_kernel(con
                 img[m] = image_word(o + AHEAD);
                 // pair 0 holds (H, 1-H), pair 1 (I H, I (1-H)) of the same column
                 const float2 B = acc[(j + 1) % K];
-                const float other = __shfl_xor_sync(0xffffffffu, p ? B.x : B.y, 16);
+                const float other = __shfl_xor_sync(0xffffffffu, p ? B.x : B.y, 1);
                 const float num = p ? B.y : other, den = p ? other : B.x;
                 const float fv = __fdiv_rn(num, den);  // pair 0: f_out, pair 1: f_in
                 const float d = __fsub_rn(I, fv);
                 const float e = __fmul_rn(d, d);
-                const float e_in = __shfl_xor_sync(0xffffffffu, e, 16);
+                const float e_in = __shfl_xor_sync(0xffffffffu, e, 1);
                 if (p == 0 && act) dbp[(size_t)o * db_plane] = data_factor(e, e_in, c.l1, c.l2, c.lam_equal != 0);
             }
         }

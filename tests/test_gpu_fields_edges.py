@@ -1,0 +1,50 @@
+"""The blurred fields and local fits of the specialised tap counts (21, 29, 35)
+at the edges of their tiles: valid regions of one voxel and of ragged rows,
+columns cut along z, and images at the ends of the packed quotient's range.
+Bit for bit against the oracle (a NaN's payload is the platform's own)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def _run(orc, shape, p, phi, img, iters):
+    from rsf_gb300 import Workspace
+
+    want = orc.evolve(phi, img.astype(np.float32),
+                      orc.params(sigma=p.sigma, dt=p.dt, mu=p.mu, lambda1=p.lambda1, lambda2=p.lambda2, nu=p.nu,
+                                 eps=p.eps), iters)
+    with Workspace(phi.size) as ws:
+        t = torch.from_numpy(phi.copy()).cuda()
+        ws.evolve(torch.from_numpy(img).cuda(), t, p, iters)
+        got = t.cpu().numpy()
+    same = (got.view(np.uint32) == want.view(np.uint32)) | (np.isnan(got) & np.isnan(want))
+    assert same.all(), f"{int((~same).sum())} voxels differ"
+
+
+@pytest.mark.parametrize("sigma,k", [(3.0, 21), (4.0, 29), (5.0, 35)])
+@pytest.mark.parametrize("extra", [(0, 0, 0), (1, 2, 3), (2, 0, 40), (75, 3, 9), (130, 1, 1)])
+def test_valid_region_edges(sigma, k, extra, orc, cuda, rsflib):
+    from rsf_gb300 import Params
+
+    shape = tuple(k + e for e in extra)
+    rng = np.random.default_rng(sum(shape))
+    phi = np.clip(4.0 * rng.standard_normal(shape), -3.0, 3.0).astype(np.float32)
+    img = rng.integers(0, 256, shape).astype(np.uint8 if extra[0] % 2 else np.float32)
+    img[:, : k // 2] = 0  # a black background: blurs of exactly 0
+    _run(orc, shape, Params(sigma=sigma, dt=0.1, mu=1.0, lambda1=1.0, lambda2=1.0, nu=65.025, eps=1.0), phi, img, 2)
+
+
+@pytest.mark.parametrize("scale", [0.0, 1e-42, 1e-33, 1e-25, -1.0, 1e18, 3e38])
+@pytest.mark.parametrize("eps,spread", [(1.0, 3.0), (0.2, 1e9), (1e-7, 3.0), (3e6, 1e20)])
+def test_value_ranges(scale, eps, spread, orc, cuda, rsflib):
+    from rsf_gb300 import Params
+
+    shape = (23, 24, 25)
+    rng = np.random.default_rng(5)
+    phi = (spread * rng.standard_normal(shape)).astype(np.float32)
+    with np.errstate(over="ignore"):
+        img = (scale * rng.random(shape)).astype(np.float32)
+    _run(orc, shape, Params(sigma=3.0, dt=0.1, mu=0.1, lambda1=1e-3, lambda2=2e-3, nu=0.1, eps=eps), phi, img, 1)
