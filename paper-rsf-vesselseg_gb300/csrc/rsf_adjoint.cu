@@ -25,25 +25,23 @@
 // among its three axis neighbours whose right index is j, and -0.5 v(m) for
 // every m whose left index is j, so boundary rules transpose exactly.
 //
-// Kernels: H; blur recompute x, y, z (the z kernel also forms the data-term
-// adjoint); transposed blur z, y, x (the x kernel forms H_bar); gradients and
-// unit normals; the pointwise terms with the parameter sums; the stencil
-// adjoint w; the final D^T gather.  The blurs along y and z compute several
+// Kernels: the forward step's x- and y-passes and the z-pass's adjoint variant
+// (zpass_adjoint_kernel, zchunk_adjoint_kernel), which the caller launches and
+// which leave the data-term adjoint; then here transposed blur z, y, x (the x
+// kernel forms H_bar); gradients and unit normals; the pointwise terms with the
+// parameter sums; the stencil adjoint w; the final D^T gather.  The blurs along y and z compute several
 // consecutive outputs per thread; the last three kernels run on blocks of
 // 32 x 8 voxels, the others on one item per thread.  Every kernel covers the
 // whole batch in one launch: a block finds its volume in a block prefix
-// array (one per kernel) and its tile within the volume.  For 21, 29 and 35
-// taps the caller replaces the first four kernels by the forward step's
-// streaming x- and y-passes and the z-pass's adjoint variant
-// (zpass_adjoint_kernel), which leave the same fields in xs.
+// array (one per kernel) and its tile within the volume.
 //
 // Scratch per volume (N = W H L; slices of the workspace pools of 1, 4 and
 // 4 floats per voxel):
-//   phi2 : H (blur input), later H_bar
-//   xs   : blur-x fields (4 Wv H L), then [0, 2N) the valid-layout adjoint pair
+//   phi2 : H_bar
+//   xs   : x fields (4 Wp H L), then [0, 2N) the valid-layout adjoint pair
 //          and [2N, 4N) e_out, e_in (kappa_bar over e_out); then g_x, g_y in
 //          [0, 2N), later w_x, w_y
-//   ys   : blur-y fields (4 Wv Hv L), then the z-transposed pair [0, 2N), the
+//   ys   : y fields (4 Wp Hv L), then the z-transposed pair [0, 2N), the
 //          y-transposed pair at 2N; later g_z (then w_z), n_x, n_y, n_z
 #include <cuda_runtime.h>
 
@@ -184,45 +182,6 @@ __device__ __forceinline__ float dirac_fast(float phi, float eps) {
 __device__ __forceinline__ long long nvox(const AdjVol &a) { return (long long)a.W * a.H * a.L; }
 __device__ __forceinline__ long long item(const BlockVol &bv) { return bv.t * kThreads + threadIdx.x; }
 
-__global__ void __launch_bounds__(kThreads) adj_heaviside(AdjConst c, const AdjVol *__restrict__ vols,
-                                                          const int *__restrict__ pre) {
-    const BlockVol bv = block_vol(pre, c.nvol);
-    const AdjVol a = vols[bv.v];
-    const long long i = item(bv);
-    if (i < nvox(a)) a.phi2[i] = heaviside<Arith::Portable>(a.phi[i], c.eps);
-}
-
-// Valid correlation along x of (I H, H, I (1-H), 1-H): (Wv, H, L) per field,
-// from H in phi2 to xs.
-__global__ void __launch_bounds__(kThreads) adj_blur_x(AdjConst c, const AdjVol *__restrict__ vols,
-                                                       const int *__restrict__ pre) {
-    const BlockVol bv = block_vol(pre, c.nvol);
-    const AdjVol a = vols[bv.v];
-    const long long n = (long long)a.Wv * a.H * a.L;
-    const long long o = item(bv);
-    if (o >= n) return;
-    const int xv = (int)(o % a.Wv);
-    const long long row = o / a.Wv;  // z * H + y
-    const long long base = row * a.W + xv;
-    const float *h = a.phi2;
-    float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-    for (int t = 0; t < c.k; t++) {
-        const float hv = h[base + t];
-        const float I = img_at(a.img, base + t, c.img_f32);
-        const float hi = 1.0f - hv;
-        const float g = c.taps[t];
-        a0 = fmaf(I * hv, g, a0);
-        a1 = fmaf(hv, g, a1);
-        a2 = fmaf(I * hi, g, a2);
-        a3 = fmaf(hi, g, a3);
-    }
-    float *out = a.xs;
-    out[o] = a0;
-    out[n + o] = a1;
-    out[2 * n + o] = a2;
-    out[3 * n + o] = a3;
-}
-
 // Correlation of NB consecutive outputs start .. start+NB-1 along a strided
 // axis of nin inputs, register-blocked so that each input load feeds up to
 // NB outputs.  Valid: out[o] = sum_t g[t] in[o + t].  Transposed (the
@@ -246,70 +205,6 @@ __device__ __forceinline__ void corr_block(const AdjConst &c, const float *__res
 
 constexpr int kNB = 8;   // outputs per thread along z
 constexpr int kNBy = 4;  // outputs per thread along y (shorter columns keep more threads in flight)
-
-// Valid correlation along y: xs (Wv, H, L) -> ys (Wv, Hv, L), four fields.
-__global__ void __launch_bounds__(kThreads) adj_blur_y(AdjConst c, const AdjVol *__restrict__ vols,
-                                                       const int *__restrict__ pre) {
-    const BlockVol bv = block_vol(pre, c.nvol);
-    const AdjVol a = vols[bv.v];
-    const long long nin = (long long)a.Wv * a.H * a.L, n = (long long)a.Wv * a.Hv * a.L;
-    const int nyb = (a.Hv + kNBy - 1) / kNBy;
-    const long long q = item(bv);
-    if (q >= (long long)a.Wv * nyb * a.L) return;
-    const int xv = (int)(q % a.Wv);
-    const long long t1 = q / a.Wv;
-    const int y0 = (int)(t1 % nyb) * kNBy;
-    const int z = (int)(t1 / nyb);
-    for (int f = 0; f < 4; f++) {
-        float acc[kNBy];
-        corr_block<kNBy, false>(c, a.xs + f * nin + (long long)z * a.H * a.Wv + xv, a.Wv, y0, a.H, acc);
-#pragma unroll
-        for (int m = 0; m < kNBy; ++m)
-            if (y0 + m < a.Hv) a.ys[f * n + ((long long)z * a.Hv + y0 + m) * a.Wv + xv] = acc[m];
-    }
-}
-
-// Valid correlation along z, then the data-term adjoint at each valid voxel:
-// writes (B1_bar - B3_bar, B2_bar - B4_bar) in the valid layout to xs and
-// e_out, e_in at the full-volume index to xs + 2N, xs + 3N.
-__global__ void __launch_bounds__(kThreads) adj_blur_z_data(AdjConst c, const AdjVol *__restrict__ vols,
-                                                            const int *__restrict__ pre) {
-    const BlockVol bv = block_vol(pre, c.nvol);
-    const AdjVol a = vols[bv.v];
-    const long long N = nvox(a);
-    const long long nin = (long long)a.Wv * a.Hv * a.L, n = (long long)a.Wv * a.Hv * a.Lv;
-    const long long plane = (long long)a.Wv * a.Hv;
-    const int nzb = (a.Lv + kNB - 1) / kNB;
-    const long long q = item(bv);
-    if (q >= plane * nzb) return;
-    const long long pxy = q % plane;
-    const int z0 = (int)(q / plane) * kNB;
-    const int xv = (int)(pxy % a.Wv), yv = (int)(pxy / a.Wv);
-    float B[4][kNB];
-    for (int f = 0; f < 4; f++) corr_block<kNB, false>(c, a.ys + f * nin + pxy, plane, z0, a.L, B[f]);
-    float *pq = a.xs, *eo_out = a.xs + 2 * N, *ei_out = a.xs + 3 * N;
-#pragma unroll
-    for (int m = 0; m < kNB; ++m) {
-        const int zv = z0 + m;
-        if (zv >= a.Lv) break;
-        const long long o = (long long)zv * plane + pxy;
-        const long long i = ((long long)(zv + c.r) * a.H + (yv + c.r)) * a.W + xv + c.r;
-        const float I = img_at(a.img, i, c.img_f32);
-        const float rb1 = __frcp_rn(B[1][m]), rb3 = __frcp_rn(B[3][m]);
-        const float fo = B[0][m] * rb1, fi = B[2][m] * rb3;
-        const float dfo = I - fo, dfi = I - fi;
-        eo_out[i] = dfo * dfo;
-        ei_out[i] = dfi * dfi;
-        const float delta = dirac_fast(a.phi[i], c.eps);
-        const float data_bar = -a.u[i] * c.dt * delta;
-        const float fo_bar = -2.0f * dfo * (c.l1 * data_bar);
-        const float fi_bar = -2.0f * dfi * (-c.l2 * data_bar);
-        const float b1 = fo_bar * rb1, b2 = -fo_bar * fo * rb1;
-        const float b3 = fi_bar * rb3, b4 = -fi_bar * fi * rb3;
-        pq[o] = b1 - b3;
-        pq[n + o] = b2 - b4;
-    }
-}
 
 // Transposed (full) correlation along z: xs (Wv, Hv, Lv) -> ys (Wv, Hv, L), two fields.
 __global__ void __launch_bounds__(kThreads) adj_blurT_z(AdjConst c, const AdjVol *__restrict__ vols,
@@ -584,18 +479,12 @@ long long cdiv(long long a, long long b) { return (a + b - 1) / b; }
 
 }  // namespace
 
-void adjoint_tiles(const AdjVol &v, bool streamed, int tiles[NADJ]) {
+void adjoint_tiles(const AdjVol &v, int tiles[NADJ]) {
     const long long N = (long long)v.W * v.H * v.L;
     const bool valid = v.Wv > 0;
     const long long bxy = cdiv(v.W, kBX) * cdiv(v.H, kBY);
     long long t[NADJ] = {};
     if (valid) {
-        if (!streamed) {
-            t[ADJ_H] = cdiv(N, kThreads);
-            t[ADJ_BX] = cdiv((long long)v.Wv * v.H * v.L, kThreads);
-            t[ADJ_BY] = cdiv((long long)v.Wv * cdiv(v.Hv, kNBy) * v.L, kThreads);
-            t[ADJ_BZ] = cdiv((long long)v.Wv * v.Hv * cdiv(v.Lv, kNB), kThreads);
-        }
         t[ADJ_TZ] = cdiv((long long)v.Wv * v.Hv * cdiv(v.L, kNB), kThreads);
         t[ADJ_TY] = cdiv((long long)v.Wv * cdiv(v.H, kNBy) * v.L, kThreads);
     }
@@ -625,10 +514,6 @@ cudaError_t launch_step_adjoint(const float *taps, int k, const AdjScalars &s, c
     const int n1 = n + 1;
     auto P = [&](int j) { return pre + (size_t)j * n1; };
     const dim3 b2(kBX, kBY, 1);
-    if (tot[ADJ_H] > 0) adj_heaviside<<<tot[ADJ_H], kThreads, 0, st>>>(c, vols, P(ADJ_H));
-    if (tot[ADJ_BX] > 0) adj_blur_x<<<tot[ADJ_BX], kThreads, 0, st>>>(c, vols, P(ADJ_BX));
-    if (tot[ADJ_BY] > 0) adj_blur_y<<<tot[ADJ_BY], kThreads, 0, st>>>(c, vols, P(ADJ_BY));
-    if (tot[ADJ_BZ] > 0) adj_blur_z_data<<<tot[ADJ_BZ], kThreads, 0, st>>>(c, vols, P(ADJ_BZ));
     if (tot[ADJ_TZ] > 0) adj_blurT_z<<<tot[ADJ_TZ], kThreads, 0, st>>>(c, vols, P(ADJ_TZ));
     if (tot[ADJ_TY] > 0) adj_blurT_y<<<tot[ADJ_TY], kThreads, 0, st>>>(c, vols, P(ADJ_TY));
     if (tot[ADJ_TX] > 0) adj_blurT_x_hbar<<<tot[ADJ_TX], kThreads, 0, st>>>(c, vols, P(ADJ_TX));

@@ -730,10 +730,9 @@ rsf_status rsf_step_adjoint_batched(rsf_workspace *ws, const rsf_params *p, rsf_
         }
     }
     cudaStream_t st = (cudaStream_t)stream;
-    // Specialised tap counts recompute the blurs with the forward step's own
-    // streaming x- and y-passes (fields in pool_x, pool_y) and the
-    // z-pass's adjoint variant, which leaves the data-term adjoint pair and
-    // e_out, e_in in each volume's xs slice.
+    // The blurs are recomputed with the forward step's own x- and y-passes
+    // (fields in pool_x, pool_y) and the z-pass's adjoint variant, which leaves
+    // the data-term adjoint pair and e_out, e_in in each volume's xs slice.
     const int kspec = rsf::kernel_k(k, RSF_ARITH_PORTABLE, false);
     // The adjoint's table: volume i's scratch slices at the running voxel
     // offset (1, 4 and 4 floats per voxel).
@@ -767,7 +766,7 @@ rsf_status rsf_step_adjoint_batched(rsf_workspace *ws, const rsf_params *p, rsf_
         rsf::valid_extents(a.W, a.H, a.L, k, a.Wv, a.Hv, a.Lv, wp);
         off += (size_t)(v.W * v.H * v.L);
         int tiles[rsf::NADJ];
-        rsf::adjoint_tiles(a, kspec > 0, tiles);
+        rsf::adjoint_tiles(a, tiles);
         for (int j = 0; j < rsf::NADJ; j++) {
             const int64_t next = (int64_t)h_pre[j * n1 + i] + tiles[j];
             if (tiles[j] < 0 || next > 0x7fffffffLL) return fail(RSF_ERR_SHAPE, "batch needs more than 2^31 blocks");
@@ -782,7 +781,7 @@ rsf_status rsf_step_adjoint_batched(rsf_workspace *ws, const rsf_params *p, rsf_
         e = cudaMemcpyAsync(ws->d_adj_pre, h_pre, rsf::NADJ * (size_t)n1 * sizeof(int), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = ws->mark_stage(st);
     if (e != cudaSuccess) return cuda_fail(e, "adjoint table upload");
-    if (kspec > 0) {
+    {
         std::vector<rsf_subvol> fw((size_t)n);
         for (int i = 0; i < n; i++)
             fw[i] = rsf_subvol{const_cast<float *>(subvols[i].phi), subvols[i].image, subvols[i].W, subvols[i].H,
@@ -801,17 +800,20 @@ rsf_status rsf_step_adjoint_batched(rsf_workspace *ws, const rsf_params *p, rsf_
         if (ftot[0] > 0) switch (kspec) {
                 case 21: e = rsf::launch_xpass_21(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, st); break;
                 case 29: e = rsf::launch_xpass_29(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, st); break;
-                default: e = rsf::launch_xpass_35(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, st); break;
+                case 35: e = rsf::launch_xpass_35(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, st); break;
+                default: e = rsf::launch_xpass_0(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, st); break;
             }
         if (e == cudaSuccess && ftot[1] > 0) switch (kspec) {
                 case 21: e = rsf::launch_ypass_21(svs, pre + f1, ftot[1], c, st); break;
                 case 29: e = rsf::launch_ypass_29(svs, pre + f1, ftot[1], c, st); break;
-                default: e = rsf::launch_ypass_35(svs, pre + f1, ftot[1], c, st); break;
+                case 35: e = rsf::launch_ypass_35(svs, pre + f1, ftot[1], c, st); break;
+                default: e = rsf::launch_ypass_0(svs, pre + f1, ftot[1], c, st); break;
             }
         if (e == cudaSuccess && ftot[2] > 0) switch (kspec) {
                 case 21: e = rsf::launch_zpass_adjoint_21(svs, pre + 2 * f1, ftot[2], c, ws->d_adj, st); break;
                 case 29: e = rsf::launch_zpass_adjoint_29(svs, pre + 2 * f1, ftot[2], c, ws->d_adj, st); break;
-                default: e = rsf::launch_zpass_adjoint_35(svs, pre + 2 * f1, ftot[2], c, ws->d_adj, st); break;
+                case 35: e = rsf::launch_zpass_adjoint_35(svs, pre + 2 * f1, ftot[2], c, ws->d_adj, st); break;
+                default: e = rsf::launch_zpass_adjoint_0(svs, pre + 2 * f1, ftot[2], c, ws->d_adj, st); break;
             }
         if (e != cudaSuccess) return cuda_fail(e, "adjoint blur recompute launch");
     }

@@ -11,7 +11,7 @@
 // The border band keeps e = (I - 1)^2.  Kernels, after a z-pass that stored
 // f_out, f_in of the valid region (the run-time-k path):
 //   gauss_x      f_out, f_out^2, f_in, f_in^2 correlated along x (scratch G)
-//   (y)          ypass_generic_kernel<1> correlates G along y into yb
+//   gauss_y      correlates G along y into yb
 //   gauss_z      along z, then e_out, e_in and lambda (e_out - e_in)
 //   gauss_border lambda (e_out - e_in) of the border band
 // All four write the data factor of every voxel after the fits, as the box
@@ -77,6 +77,36 @@ __global__ void __launch_bounds__(GX_T) gauss_x_kernel(const SubVolDev *__restri
 #pragma unroll
         for (int m = 0; m < GX_NB; ++m)
             if (x0 + m < s.Wv) g[f * fs + m] = acc[f][m];
+}
+
+// The expanded data term's y-pass: the scratch G at xb + gdelta, four float
+// planes, into yb.
+__global__ void __launch_bounds__(YB_TX) gauss_y_kernel(const SubVolDev *__restrict__ svs,
+                                                              const int *__restrict__ pre, const StepConst c) {
+    __shared__ float taps_s[MAXK];
+    const int b = blockIdx.x;
+    const int sv = find_sv(pre, c.nsv, b);
+    const SubVolDev s = svs[sv];
+    int t = b - __ldg(pre + sv);
+    const int ntx = (s.Wv + YB_TX - 1) / YB_TX, nty = (s.Hv + YB_YB - 1) / YB_YB;
+    const int tx = t % ntx;
+    t /= ntx;
+    const int ty = t % nty;
+    t /= nty;
+    const int f = t & 3;
+    const int z = t >> 2;
+    for (int i = threadIdx.x; i < c.k; i += blockDim.x) taps_s[i] = c.taps[i];
+    __syncthreads();
+    const int x = tx * YB_TX + threadIdx.x;
+    if (x >= s.Wv) return;
+    const int y0 = ty * YB_YB;
+    const float *src = s.xb + c.gdelta + f * ((size_t)s.Wp * s.H * s.L) + (size_t)z * s.H * s.Wp + x;
+    float *dst = s.yb + f * ((size_t)s.Wp * s.Hv * s.L) + (size_t)z * s.Hv * s.Wp + x;
+    float acc[YB_YB];
+    conv_block_rt<YB_YB>(src, (size_t)s.Wp, y0, s.H, taps_s, c.k, acc);
+#pragma unroll
+    for (int m = 0; m < YB_YB; ++m)
+        if (y0 + m < s.Hv) dst[(size_t)(y0 + m) * s.Wp] = acc[m];
 }
 
 template <bool DEBUG>
@@ -154,7 +184,7 @@ cudaError_t launch_gauss(const SubVolDev *svs, const int *pre, int n1, const int
                          const DebugOut *dbg, cudaStream_t st) {
     const DebugOut none = {nullptr, 0};
     if (tot[NKERN] > 0) gauss_x_kernel<<<tot[NKERN], GX_T, 0, st>>>(svs, pre + NKERN * n1, c);
-    if (tot[NKERN + 1] > 0) ypass_generic_kernel<1><<<tot[NKERN + 1], YB_TX, 0, st>>>(svs, pre + (NKERN + 1) * n1, c);
+    if (tot[NKERN + 1] > 0) gauss_y_kernel<<<tot[NKERN + 1], YB_TX, 0, st>>>(svs, pre + (NKERN + 1) * n1, c);
     if (tot[NKERN + 2] > 0) {
         if (dbg) gauss_z_kernel<true><<<tot[NKERN + 2], ZB_TX, 0, st>>>(svs, pre + (NKERN + 2) * n1, c, *dbg);
         else gauss_z_kernel<false><<<tot[NKERN + 2], ZB_TX, 0, st>>>(svs, pre + (NKERN + 2) * n1, c, none);

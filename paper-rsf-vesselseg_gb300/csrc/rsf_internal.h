@@ -14,16 +14,18 @@ constexpr int MAXK = 128;  // largest supported tap count (sigma up to ~18)
 constexpr int XP_ROWS = 4;     // x-pass: warps per block
 constexpr int XP_RPW = 8;      // x-pass: largest rows per warp (XP_ROWS apart; chosen per launch)
 constexpr int YP_COLS = 128;   // y-pass: float2 columns per block (one field pair of one column per thread)
-constexpr int YB_TX = 128;     // generic y-pass: columns per block
-constexpr int YB_YB = 16;      // generic y-pass: outputs per thread along y
+constexpr int YB_TX = 128;     // expanded data term's y kernel: columns per block
+constexpr int YB_YB = 16;      // and outputs per thread
 constexpr int ZP_COLS = 128;   // z-pass: columns per block
 // z-pass: resident blocks per SM that its 4 K accumulator registers leave room
 // for (21 taps: 3.70 ms per launch on the 48-sub-volume batch with 4, 4.17 with
 // 3; 29 and 35 taps spill with 3: 771 against 1061 us on a 195 M voxel batch,
 // 1.02 against 1.45 ms on 512^3)
 constexpr int zpass_blocks(int K) { return K <= 21 ? 4 : 2; }
-constexpr int ZB_TX = 128;     // generic z-pass: columns per block
-constexpr int ZB_ZB = 16;      // generic z-pass: outputs per thread along z
+constexpr int YG_NB = 16;      // run-time-k y-pass: outputs per thread
+constexpr int ZG_NB = 8;       // run-time-k z-pass: outputs per thread
+constexpr int ZB_TX = 128;     // expanded data term's z kernel: columns per block
+constexpr int ZB_ZB = 16;      // and outputs per thread
 constexpr int ST_OX = 30;      // stencil: output columns per warp (lanes 1..30)
 constexpr int ST_OY = 14;      // stencil: output rows per block (warps 1..14)
 constexpr int ST_WARPS = ST_OY + 2;
@@ -36,9 +38,7 @@ constexpr int XB_CHOICES[2] = {5, 9};
 // One sub-volume as the kernels see it.
 //   xb: x-pass fields, each Wp x H x L   (row stride Wp)
 //   yb: y-pass fields, each Wp x Hv x L
-//   The specialised tap counts keep the fields interleaved, float4 (H, 1-H,
-//   I H, I (1-H)) per voxel; the run-time-k kernels as four separate float
-//   planes in that order.
+//   The fields are interleaved, float4 (H, 1-H, I H, I (1-H)) per voxel.
 //   db: data factor lambda (e_out - e_in) of the valid region, Wp x Hv x Lv;
 //       it reuses the x-pass storage, which is dead once the y-pass has run.
 //       With the box e-term or the expanded data term it holds f_out and
@@ -72,7 +72,7 @@ struct StepConst {
     int nsv;        // number of sub-volumes in the table
     int xb_w;       // x-pass outputs per lane for this launch
     int xrpw;       // x-pass rows per warp for this launch
-    int zout;       // z-pass output planes per block for this launch (specialised tap counts)
+    int zout;       // z-pass output planes per block for this launch
     int zc;         // stencil planes per block for this launch
     int box;        // e-term box radius (int)sigma2; 0: e = (I - f)^2
     int gauss;      // 1: expanded Gaussian data term (rsf_gauss.cu)
@@ -127,7 +127,7 @@ constexpr int MAX_BOX = 8;  // largest e-term box radius
 struct LaunchShape {
     int xb_w;   // x-pass outputs per lane
     int xrpw;   // x-pass rows per warp (1, 2, 4 or XP_RPW)
-    int zout;   // z-pass output planes per block (specialised tap counts)
+    int zout;   // z-pass output planes per block
     int zt;     // 1: the z-pass loads planes with TMA (needs a map per sub-volume)
     int zc;     // stencil planes per block
     int gauss;  // 1: the expanded data term's kernels run (tiles NKERN .. NPRE - 1)
@@ -170,14 +170,13 @@ struct AdjVol {
     int W, H, L;
     int Wv, Hv, Lv;    // valid blur extents; all > 0 or all 0
 };
-// Adjoint kernels with a block prefix array each (rsf_adjoint.cu): H, the
-// recompute blurs x, y, z, the transposed blurs z, y, x, normals, pointwise
-// terms, w, gather.
-constexpr int NADJ = 11;
-enum AdjKernel { ADJ_H, ADJ_BX, ADJ_BY, ADJ_BZ, ADJ_TZ, ADJ_TY, ADJ_TX, ADJ_NRM, ADJ_PT, ADJ_W, ADJ_G };
-// Blocks of each adjoint kernel for one volume; with `streamed` the
-// recompute (ADJ_H .. ADJ_BZ) runs in the forward step's kernels instead.
-void adjoint_tiles(const AdjVol &v, bool streamed, int tiles[NADJ]);
+// Adjoint kernels with a block prefix array each (rsf_adjoint.cu): the
+// transposed blurs z, y, x, normals, pointwise terms, w, gather.  (The recompute
+// before them runs in the forward step's kernels.)
+constexpr int NADJ = 7;
+enum AdjKernel { ADJ_TZ, ADJ_TY, ADJ_TX, ADJ_NRM, ADJ_PT, ADJ_W, ADJ_G };
+// Blocks of each adjoint kernel for one volume.
+void adjoint_tiles(const AdjVol &v, int tiles[NADJ]);
 
 #define RSF_DECLARE_K(K)                                                                                      \
     cudaError_t launch_xpass_##K(const SubVolDev *, const int *, int, const StepConst &, int, int, cudaStream_t); \
@@ -191,8 +190,10 @@ RSF_DECLARE_K(21)
 RSF_DECLARE_K(29)
 RSF_DECLARE_K(35)
 #undef RSF_DECLARE_K
-// The streaming z-pass with the adjoint's emit (specialised k):
+// The z-pass with the adjoint's emit:
 // sub-volume i of the table is volume i of `vols`.
+cudaError_t launch_zpass_adjoint_0(const SubVolDev *, const int *, int, const StepConst &, const AdjVol *vols,
+                                   cudaStream_t);
 cudaError_t config_zpass_adjoint_21();
 cudaError_t launch_zpass_adjoint_21(const SubVolDev *, const int *, int, const StepConst &, const AdjVol *vols,
                                     cudaStream_t);

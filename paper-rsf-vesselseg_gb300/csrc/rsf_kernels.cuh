@@ -52,34 +52,46 @@ __device__ __forceinline__ float load_img(const void *img, size_t i, int f32) {
 // Valid correlation of XB consecutive outputs of one packed field pair:
 // src points at the lane's first input, consecutive inputs are two float2
 // apart (the shared slab holds float4 (H, 1-H, I H, I (1-H)) per element).
+// With a run-time tap count the taps go in chunks of XB over a window of 2 XB
+// inputs (which may read up to 2 XB elements past the slab; the slabs are
+// followed by more shared memory, and no tap uses those).
 template <int K, int XB>
-__device__ __forceinline__ void xconv_pair(const float2 *src, const StepConst &c, const float2 *taps_s, int k,
-                                           float2 (&acc)[XB]) {
+__device__ __forceinline__ void xconv_pair(const float2 *src, const StepConst &c, int k, float2 (&acc)[XB]) {
+    const unsigned long long *in = reinterpret_cast<const unsigned long long *>(src);
+    unsigned long long u[XB];
     if constexpr (K > 0) {
-        unsigned long long u[XB];
 #pragma unroll
         for (int q = 0; q < XB + K - 1; ++q) {
-            const unsigned long long v = *reinterpret_cast<const unsigned long long *>(src + 2 * q);
+            const unsigned long long v = in[2 * q];
 #pragma unroll
             for (int m = 0; m < XB; ++m) {
                 const int tt = q - m;
                 if (tt >= 0 && tt < K) u[m] = fma2(v, c.tap2(tt), tt == 0 ? 0ull : u[m]);
             }
         }
-#pragma unroll
-        for (int m = 0; m < XB; ++m) acc[m] = unpack2(u[m]);
     } else {
+        unsigned long long w[2 * XB];
 #pragma unroll
-        for (int m = 0; m < XB; ++m) acc[m] = make_float2(0.f, 0.f);
-        for (int q = 0; q < XB + k - 1; ++q) {
-            const float2 v = src[2 * q];
+        for (int m = 0; m < XB; ++m) {
+            u[m] = 0ull;
+            w[m] = in[2 * m];
+        }
+        for (int t0 = 0; t0 < k; t0 += XB) {
 #pragma unroll
-            for (int m = 0; m < XB; ++m) {
-                const int tt = q - m;
-                if (tt >= 0 && tt < k) acc[m] = fma2(v, taps_s[tt], acc[m]);
+            for (int m = 0; m < XB; ++m) w[XB + m] = in[2 * (t0 + XB + m)];
+#pragma unroll
+            for (int j = 0; j < XB; ++j) {
+                if (t0 + j >= k) break;
+                const unsigned long long g = c.tap2(t0 + j);
+#pragma unroll
+                for (int m = 0; m < XB; ++m) u[m] = fma2(w[m + j], g, u[m]);
             }
+#pragma unroll
+            for (int m = 0; m < XB; ++m) w[m] = w[XB + m];
         }
     }
+#pragma unroll
+    for (int m = 0; m < XB; ++m) acc[m] = unpack2(u[m]);
 }
 
 // ---------------------------------------------------------------------------
@@ -88,8 +100,8 @@ __device__ __forceinline__ void xconv_pair(const float2 *src, const StepConst &c
 // a lane produces XB consecutive outputs of one packed field pair at a time
 // (XB odd, so the lanes' 64-bit loads fall in distinct banks), the results
 // are staged in shared memory and written as float4 rows.
-// Shared memory: XP_ROWS * span float4 inputs, MAXK float2 taps (generic k),
-// XP_ROWS * 2 * XT floats of pair-0 staging.
+// Shared memory: XP_ROWS * span float4 inputs, XP_ROWS * XT float2 of pair-0
+// staging.
 // ---------------------------------------------------------------------------
 template <int K, int XB, Arith A>
 __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__restrict__ svs,
@@ -109,11 +121,6 @@ __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__
     const int ty = t % nty;
     const int z = t / nty;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float2 *taps_s = reinterpret_cast<float2 *>(sm4 + XP_ROWS * span);  // MAXK pairs, then the pair-0 stages
-    if (K == 0) {
-        for (int i = threadIdx.x; i < k; i += blockDim.x) taps_s[i] = c.taps2[i];
-        __syncthreads();
-    }
     float4 *in = sm4 + warp * span;
     const int x0 = tx * XT;
     // c.xrpw rows per warp, XP_ROWS apart: the block setup above is paid
@@ -146,67 +153,39 @@ __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__
                     in[e + 32] = make_float4(h.y, hi.y, __fmul_rn(im[q + 1], h.y), __fmul_rn(im[q + 1], hi.y));
             }
         } else {
-            for (int e = lane; e < span; e += 32) {
+            for (int e = lane; e < span; e += 64) {
                 const int x = x0 + e;
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (x < s.W) {
-                    const float h = heaviside<A>(__ldg(phi + x), c.eps);
-                    const float I = load_img(s.img, row + x, c.img_f32);
-                    const float hi = __fsub_rn(1.0f, h);
-                    v = make_float4(h, hi, __fmul_rn(I, h), __fmul_rn(I, hi));
-                }
-                in[e] = v;
+                const bool ok0 = x < s.W, ok1 = e + 32 < span && x + 32 < s.W;
+                const float p0 = ok0 ? __ldg(phi + x) : 0.0f, p1 = ok1 ? __ldg(phi + x + 32) : 0.0f;
+                const float i0 = ok0 ? load_img(s.img, row + x, c.img_f32) : 0.0f;
+                const float i1 = ok1 ? load_img(s.img, row + x + 32, c.img_f32) : 0.0f;
+                const float2 h = heaviside2<A>(make_float2(p0, p1), c.eps, c.pk);
+                const float2 hi = sub2(dup2(1.0f), h);
+                in[e] = make_float4(h.x, hi.x, __fmul_rn(i0, h.x), __fmul_rn(i0, hi.x));
+                if (e + 32 < span) in[e + 32] = make_float4(h.y, hi.y, __fmul_rn(i1, h.y), __fmul_rn(i1, hi.y));
             }
         }
         __syncwarp();
         // Pair 0 (H, 1-H) is staged in its own slab, pair 1 (I H, I (1-H)) in
         // the input slab once every lane has finished reading it.
-        float *st01 = reinterpret_cast<float *>(sm4 + XP_ROWS * span) + 2 * MAXK + warp * 2 * XT;
-        float *st23 = reinterpret_cast<float *>(in);
+        float2 *s01 = reinterpret_cast<float2 *>(sm4 + XP_ROWS * span) + warp * XT;
+        float2 *s23 = reinterpret_cast<float2 *>(in);
         const float2 *src = reinterpret_cast<const float2 *>(in + XB * lane);
         float2 acc[XB];
-        if constexpr (K > 0) {
-            // each pair's results are staged as float2 and written together
-            float2 *s01 = reinterpret_cast<float2 *>(st01), *s23 = reinterpret_cast<float2 *>(st23);
-            xconv_pair<K, XB>(src, c, taps_s, k, acc);
+        xconv_pair<K, XB>(src, c, k, acc);
 #pragma unroll
-            for (int m = 0; m < XB; ++m) s01[XB * lane + m] = acc[m];
-            xconv_pair<K, XB>(src + 1, c, taps_s, k, acc);
-            __syncwarp();
+        for (int m = 0; m < XB; ++m) s01[XB * lane + m] = acc[m];
+        xconv_pair<K, XB>(src + 1, c, k, acc);
+        __syncwarp();
 #pragma unroll
-            for (int m = 0; m < XB; ++m) s23[XB * lane + m] = acc[m];
-            __syncwarp();
-            float4 *dst = reinterpret_cast<float4 *>(s.xb) + ((size_t)z * s.H + y) * s.Wp + x0;
+        for (int m = 0; m < XB; ++m) s23[XB * lane + m] = acc[m];
+        __syncwarp();
+        float4 *dst = reinterpret_cast<float4 *>(s.xb) + ((size_t)z * s.H + y) * s.Wp + x0;
 #pragma unroll
-            for (int q = 0; q < XB; ++q) {
-                const int e = lane + 32 * q;
-                const float2 a = s01[e], b = s23[e];
-                if (x0 + e < s.Wv) dst[e] = make_float4(a.x, a.y, b.x, b.y);
-            }
-        } else {
-            xconv_pair<K, XB>(src, c, taps_s, k, acc);
-#pragma unroll
-            for (int m = 0; m < XB; ++m) {
-                st01[XB * lane + m] = acc[m].x;
-                st01[XT + XB * lane + m] = acc[m].y;
-            }
-            xconv_pair<K, XB>(src + 1, c, taps_s, k, acc);
-            __syncwarp();
-#pragma unroll
-            for (int m = 0; m < XB; ++m) {
-                st23[XB * lane + m] = acc[m].x;
-                st23[XT + XB * lane + m] = acc[m].y;
-            }
-            __syncwarp();
-            const size_t fstride = (size_t)s.Wp * s.H * s.L;
-            const size_t orow = ((size_t)z * s.H + y) * s.Wp;
-#pragma unroll
-            for (int f = 0; f < 4; ++f) {
-                const float4 *sf = reinterpret_cast<const float4 *>((f < 2 ? st01 : st23) + (f & 1) * XT);
-                float4 *dst = reinterpret_cast<float4 *>(s.xb + f * fstride + orow + x0);
-                for (int e = lane; e < XT / 4; e += 32)
-                    if (x0 + 4 * e < s.Wv) dst[e] = sf[e];
-            }
+        for (int q = 0; q < XB; ++q) {
+            const int e = lane + 32 * q;
+            const float2 a = s01[e], b = s23[e];
+            if (x0 + e < s.Wv) dst[e] = make_float4(a.x, a.y, b.x, b.y);
         }
     }
 }
@@ -331,35 +310,56 @@ __global__ void __launch_bounds__(YP_COLS) ypass_kernel(const SubVolDev *__restr
     stream_axis<K>(rg, c, emit);
 }
 
-// U = 1: the second (expanded data term) pass, reading the scratch G at
-// xb + gdelta instead of the x-pass fields.
-template <int U = 0>
-__global__ void __launch_bounds__(YB_TX) ypass_generic_kernel(const SubVolDev *__restrict__ svs,
-                                                              const int *__restrict__ pre, const StepConst c) {
-    __shared__ float taps_s[MAXK];
+// Run-time tap count: a thread forms YG_NB consecutive outputs of its column.
+// The taps go in chunks of YG_NB over a window of 2 YG_NB inputs in registers,
+// whose upper half is loaded a chunk ahead, so a tap costs YG_NB multiply-adds,
+// one load and no index test.
+template <int NB, class Load>
+__device__ __forceinline__ void conv_chunks(const StepConst &c, Load load, unsigned long long (&u)[NB]) {
+    unsigned long long w[2 * NB];
+#pragma unroll
+    for (int m = 0; m < NB; ++m) {
+        u[m] = 0ull;
+        w[m] = load(m);
+    }
+    for (int t0 = 0; t0 < c.k; t0 += NB) {
+#pragma unroll
+        for (int m = 0; m < NB; ++m) w[NB + m] = load(t0 + NB + m);
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+            if (t0 + j >= c.k) break;
+            const unsigned long long g = c.tap2(t0 + j);
+#pragma unroll
+            for (int m = 0; m < NB; ++m) u[m] = fma2(w[m + j], g, u[m]);
+        }
+#pragma unroll
+        for (int m = 0; m < NB; ++m) w[m] = w[NB + m];
+    }
+}
+
+template <int NB>
+__global__ void __launch_bounds__(YP_COLS) ypass_chunk_kernel(const SubVolDev *__restrict__ svs,
+                                                              const int *__restrict__ pre,
+                                                              const __grid_constant__ StepConst c) {
     const int b = blockIdx.x;
     const int sv = find_sv(pre, c.nsv, b);
     const SubVolDev s = svs[sv];
-    int t = b - __ldg(pre + sv);
-    const int ntx = (s.Wv + YB_TX - 1) / YB_TX, nty = (s.Hv + YB_YB - 1) / YB_YB;
-    const int tx = t % ntx;
-    t /= ntx;
-    const int ty = t % nty;
-    t /= nty;
-    const int f = t & 3;
-    const int z = t >> 2;
-    for (int i = threadIdx.x; i < c.k; i += blockDim.x) taps_s[i] = c.taps[i];
-    __syncthreads();
-    const int x = tx * YB_TX + threadIdx.x;
-    if (x >= s.Wv) return;
-    const int y0 = ty * YB_YB;
-    const float *src = (U ? s.xb + c.gdelta : s.xb) + f * ((size_t)s.Wp * s.H * s.L) + (size_t)z * s.H * s.Wp + x;
-    float *dst = s.yb + f * ((size_t)s.Wp * s.Hv * s.L) + (size_t)z * s.Hv * s.Wp + x;
-    float acc[YB_YB];
-    conv_block_rt<YB_YB>(src, (size_t)s.Wp, y0, s.H, taps_s, c.k, acc);
+    const int row = 2 * s.Wp;
+    const int t = b - __ldg(pre + sv);
+    const int ntq = (int)(((long long)row * s.L + YP_COLS - 1) / YP_COLS);
+    const long long q = (long long)(t % ntq) * YP_COLS + threadIdx.x;
+    const int y0 = (t / ntq) * NB;
+    const int z = (int)(q / row), x = (int)(q - (long long)z * row);
+    if (z >= s.L || x >= 2 * s.Wv) return;
+    const unsigned long long *src = reinterpret_cast<const unsigned long long *>(s.xb) +
+                                    ((size_t)z * s.H + y0) * row + x;
+    unsigned long long *dst = reinterpret_cast<unsigned long long *>(s.yb) + ((size_t)z * s.Hv + y0) * row + x;
+    const int have = min(s.H - y0, NB + c.k - 1);
+    unsigned long long u[NB];
+    conv_chunks<NB>(c, [&](int i) { return i < have ? __ldg(src + (size_t)i * row) : 0ull; }, u);
 #pragma unroll
-    for (int m = 0; m < YB_YB; ++m)
-        if (y0 + m < s.Hv) dst[(size_t)(y0 + m) * s.Wp] = acc[m];
+    for (int m = 0; m < NB; ++m)
+        if (y0 + m < s.Hv) dst[(size_t)m * row] = u[m];
 }
 
 // ---------------------------------------------------------------------------
@@ -494,6 +494,74 @@ __global__ void __launch_bounds__(ZP_COLS, zpass_blocks(K)) zpass_kernel(const S
                });
 }
 
+// Run-time tap count: ZG_NB outputs of one column of all four fields per thread,
+// in chunks as the y-pass.  emit(m, h, ih) gets output m's pairs.
+template <int NB, class Emit>
+__device__ __forceinline__ void zchunk(const SubVolDev &s, const StepConst &c, const ZCol &z, Emit emit) {
+    const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(s.yb) + (size_t)z.o0 * z.plane + z.p;
+    const int have = min(s.L - z.o0, NB + c.k - 1);
+    ulonglong2 w[2 * NB];
+    unsigned long long a[NB], b[NB];
+    auto load = [&](int i) { return i < have ? __ldg(src + (size_t)i * z.plane) : make_ulonglong2(0ull, 0ull); };
+#pragma unroll
+    for (int m = 0; m < NB; ++m) {
+        a[m] = b[m] = 0ull;
+        w[m] = load(m);
+    }
+    for (int t0 = 0; t0 < c.k; t0 += NB) {
+#pragma unroll
+        for (int m = 0; m < NB; ++m) w[NB + m] = load(t0 + NB + m);
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+            if (t0 + j >= c.k) break;
+            const unsigned long long g = c.tap2(t0 + j);
+#pragma unroll
+            for (int m = 0; m < NB; ++m) {
+                a[m] = fma2(w[m + j].x, g, a[m]);
+                b[m] = fma2(w[m + j].y, g, b[m]);
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < NB; ++m) w[m] = w[NB + m];
+    }
+#pragma unroll
+    for (int m = 0; m < NB; ++m)
+        if (m < z.n) emit(m, unpack2(a[m]), unpack2(b[m]));
+}
+
+template <bool DEBUG>
+__global__ void __launch_bounds__(ZP_COLS) zpass_chunk_kernel(const SubVolDev *__restrict__ svs,
+                                                              const int *__restrict__ pre,
+                                                              const __grid_constant__ StepConst c, DebugOut dbg) {
+    const int blk = blockIdx.x;
+    const int sv = find_sv(pre, c.nsv, blk);
+    const SubVolDev s = svs[sv];
+    const ZCol z = zcol_of(s, c, blk - __ldg(pre + sv));
+    if (!z.live) return;
+    const size_t v0 = ((size_t)(z.o0 + c.r) * s.H + (z.y + c.r)) * s.W + (z.x + c.r), plane = (size_t)s.W * s.H;
+    zchunk<ZG_NB>(s, c, z, [&](int m, float2 h, float2 ih) {
+        const size_t vi = v0 + (size_t)m * plane, di = (size_t)(z.o0 + m) * z.plane + z.p;
+        const float2 f = div2(ih, h);  // f_out, f_in
+        if (DEBUG) {
+            dbg.f[0 * dbg.n + vi] = f.x;
+            dbg.f[1 * dbg.n + vi] = f.y;
+        }
+        if (c.full_data) {  // the box or expanded data-term kernels form e from the fits
+            s.db[di] = f.x;
+            s.db[z.plane * s.Lv + di] = f.y;
+            return;
+        }
+        const float I = load_img(s.img, vi, c.img_f32);
+        const float d_o = __fsub_rn(I, f.x), d_i = __fsub_rn(I, f.y);
+        const float eo = __fmul_rn(d_o, d_o), ei = __fmul_rn(d_i, d_i);
+        s.db[di] = data_factor(eo, ei, c.l1, c.l2, c.lam_equal != 0);
+        if (DEBUG) {
+            dbg.f[2 * dbg.n + vi] = eo;
+            dbg.f[3 * dbg.n + vi] = ei;
+        }
+    });
+}
+
 // The adjoint's recompute of the fits (rsf_adjoint.cu): the forward z-pass,
 // emitting at each valid voxel, instead of the data factor,
 //   e_out = (I - f_out)^2 and e_in at the full-volume index, and the pair
@@ -503,8 +571,28 @@ __global__ void __launch_bounds__(ZP_COLS, zpass_blocks(K)) zpass_kernel(const S
 //   f_out_bar = -2 (I - f_out) lambda1 data_bar, f_in_bar = 2 (I - f_in) lambda2 data_bar,
 //   B1_bar = f_out_bar / B2, B2_bar = -f_out_bar f_out / B2 (B3, B4 alike).
 // The pair goes to a.xs (2 Wv Hv Lv floats), e_out and e_in to a.xs + 2 N and
-// a.xs + 3 N.  phi and u of the next three output planes ride in registers
-// with the image.
+// a.xs + 3 N.
+struct AdjFits {
+    float eo, ei, p, q;
+};
+__device__ __forceinline__ AdjFits adjoint_fits(const StepConst &c, float I, float ph, float uo, float2 h, float2 ih) {
+    const float delta = __fdividef(0.318309886183790672f * c.eps, fmaf(ph, ph, c.eps * c.eps));
+    const float data_bar = -uo * c.dt * delta;
+    auto side = [&](float num, float den, float weight, float &bn, float &bd) {
+        const float rb = __frcp_rn(den);
+        const float fv = num * rb;
+        const float d = I - fv;
+        const float fbar = -2.0f * d * (weight * data_bar);
+        bn = fbar * rb;
+        bd = -fbar * fv * rb;
+        return d * d;
+    };
+    float bn0, bd0, bn1, bd1;
+    const float eo = side(ih.x, h.x, c.l1, bn0, bd0), ei = side(ih.y, h.y, -c.l2, bn1, bd1);
+    return {eo, ei, bn0 - bn1, bd0 - bd1};
+}
+
+// phi and u of the next three output planes ride in registers with the image.
 template <int K>
 __global__ void __launch_bounds__(ZP_COLS, zpass_blocks(K)) zpass_adjoint_kernel(const SubVolDev *__restrict__ svs,
                                                                                  const int *__restrict__ pre,
@@ -542,86 +630,40 @@ __global__ void __launch_bounds__(ZP_COLS, zpass_blocks(K)) zpass_adjoint_kernel
                    n0 = n1;
                    n1 = n2;
                    n2 = load();
-                   const float delta = __fdividef(0.318309886183790672f * c.eps, fmaf(ph, ph, c.eps * c.eps));
-                   const float data_bar = -uo * c.dt * delta;
-                   auto side = [&](float num, float den, float weight, float &bn, float &bd) {
-                       const float rb = __frcp_rn(den);
-                       const float fv = num * rb;
-                       const float d = I - fv;
-                       const float fbar = -2.0f * d * (weight * data_bar);
-                       bn = fbar * rb;
-                       bd = -fbar * fv * rb;
-                       return d * d;
-                   };
-                   float bn0, bd0, bn1, bd1;
-                   const float e0 = side(ih.x, h.x, c.l1, bn0, bd0), e1 = side(ih.y, h.y, -c.l2, bn1, bd1);
-                   *eo = e0;
-                   *ei = e1;
-                   pq[0] = bn0 - bn1;
-                   pq[nv] = bd0 - bd1;
+                   const AdjFits f = adjoint_fits(c, I, ph, uo, h, ih);
+                   *eo = f.eo;
+                   *ei = f.ei;
+                   pq[0] = f.p;
+                   pq[nv] = f.q;
                    eo += plane;
                    ei += plane;
                    pq += vplane;
                });
 }
 
-template <bool DEBUG>
-__global__ void __launch_bounds__(ZB_TX) zpass_generic_kernel(const SubVolDev *__restrict__ svs,
-                                                              const int *__restrict__ pre, const StepConst c,
-                                                              DebugOut dbg) {
-    __shared__ float taps_s[MAXK];
-    const int b = blockIdx.x;
-    const int sv = find_sv(pre, c.nsv, b);
+template <int NB>
+__global__ void __launch_bounds__(ZP_COLS) zchunk_adjoint_kernel(const SubVolDev *__restrict__ svs,
+                                                                 const int *__restrict__ pre,
+                                                                 const __grid_constant__ StepConst c,
+                                                                 const AdjVol *__restrict__ vols) {
+    const int blk = blockIdx.x;
+    const int sv = find_sv(pre, c.nsv, blk);
     const SubVolDev s = svs[sv];
-    int t = b - __ldg(pre + sv);
-    const int ntx = (s.Wv + ZB_TX - 1) / ZB_TX, ntz = (s.Lv + ZB_ZB - 1) / ZB_ZB;
-    const int tx = t % ntx;
-    t /= ntx;
-    const int tz = t % ntz;
-    const int y = t / ntz;
-    for (int i = threadIdx.x; i < c.k; i += blockDim.x) taps_s[i] = c.taps[i];
-    __syncthreads();
-    const int x = tx * ZB_TX + threadIdx.x;
-    if (x >= s.Wv) return;
-    const int z0 = tz * ZB_ZB;
-    const size_t fs = (size_t)s.Wp * s.Hv * s.L, ps = (size_t)s.Wp * s.Hv;
-    const float *col = s.yb + (size_t)y * s.Wp + x;
-    float num[ZB_ZB], den[ZB_ZB], fo[ZB_ZB], fi[ZB_ZB];
-    conv_block_rt<ZB_ZB>(col + F_IH * fs, ps, z0, s.L, taps_s, c.k, num);
-    conv_block_rt<ZB_ZB>(col + F_H * fs, ps, z0, s.L, taps_s, c.k, den);
-#pragma unroll
-    for (int m = 0; m < ZB_ZB; ++m) fo[m] = __fdiv_rn(num[m], den[m]);
-    conv_block_rt<ZB_ZB>(col + F_IHI * fs, ps, z0, s.L, taps_s, c.k, num);
-    conv_block_rt<ZB_ZB>(col + F_HI * fs, ps, z0, s.L, taps_s, c.k, den);
-#pragma unroll
-    for (int m = 0; m < ZB_ZB; ++m) fi[m] = __fdiv_rn(num[m], den[m]);
-    const int r = c.r;
-#pragma unroll
-    for (int m = 0; m < ZB_ZB; ++m) {
-        const int o = z0 + m;
-        if (o >= s.Lv) break;
-        const size_t vi = ((size_t)(o + r) * s.H + (y + r)) * s.W + (x + r);
-        if (c.full_data) {  // the box or expanded data-term kernels form e from the fits
-            const size_t di = ((size_t)o * s.Hv + y) * s.Wp + x;
-            s.db[di] = fo[m];
-            s.db[(size_t)s.Wp * s.Hv * s.Lv + di] = fi[m];
-            if (DEBUG) {
-                dbg.f[0 * dbg.n + vi] = fo[m];
-                dbg.f[1 * dbg.n + vi] = fi[m];
-            }
-            continue;
-        }
-        const float I = load_img(s.img, vi, c.img_f32);
-        const float d_o = __fsub_rn(I, fo[m]), d_i = __fsub_rn(I, fi[m]);
-        const float eo = __fmul_rn(d_o, d_o), ei = __fmul_rn(d_i, d_i);
-        s.db[((size_t)o * s.Hv + y) * s.Wp + x] = data_factor(eo, ei, c.l1, c.l2, c.lam_equal != 0);
-        if (DEBUG) {
-            dbg.f[0 * dbg.n + vi] = fo[m];
-            dbg.f[1 * dbg.n + vi] = fi[m];
-            dbg.f[2 * dbg.n + vi] = eo;
-            dbg.f[3 * dbg.n + vi] = ei;
-        }
-    }
+    const AdjVol a = vols[sv];
+    const ZCol z = zcol_of(s, c, blk - __ldg(pre + sv));
+    if (!z.live) return;
+    const size_t plane = (size_t)s.W * s.H, n = plane * s.L;
+    const size_t v0 = ((size_t)(z.o0 + c.r) * s.H + (z.y + c.r)) * s.W + (z.x + c.r);
+    const size_t nv = (size_t)s.Wv * s.Hv * s.Lv, vplane = (size_t)s.Wv * s.Hv;
+    float *pq = a.xs + (size_t)z.o0 * vplane + (size_t)z.y * s.Wv + z.x;
+    zchunk<NB>(s, c, z, [&](int m, float2 h, float2 ih) {
+        const size_t v = v0 + (size_t)m * plane;
+        const AdjFits f = adjoint_fits(c, load_img(s.img, v, c.img_f32), __ldg(a.phi + v), __ldg(a.u + v), h, ih);
+        a.xs[2 * n + v] = f.eo;
+        a.xs[3 * n + v] = f.ei;
+        pq[(size_t)m * vplane] = f.p;
+        pq[nv + (size_t)m * vplane] = f.q;
+    });
 }
 
 // ---------------------------------------------------------------------------

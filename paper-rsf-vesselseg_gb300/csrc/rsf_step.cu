@@ -146,7 +146,7 @@ LaunchShape choose_shape(const int *whl, int n, int k, int kspec, int gauss) {
     sh.xrpw = choose_xrpw(whl, n, k, sh.xb_w);
     sh.zt = tma_z(kspec) && tma_z_requested() && tensor_maps_available() ? 1 : 0;
     sh.zc = choose_zc(whl, n);
-    sh.zout = choose_zout(whl, n, k);
+    sh.zout = kspec > 0 ? choose_zout(whl, n, k) : ZG_NB;
     sh.gauss = gauss;
     return sh;
 }
@@ -205,11 +205,10 @@ void tile_counts(const SubVolDev &d, int kspec, const LaunchShape &sh, int tiles
     const int xr = XP_ROWS * sh.xrpw;
     tiles[0] = valid ? ((d.Wv + xt - 1) / xt) * ((d.H + xr - 1) / xr) * d.L : 0;
     if (!valid) tiles[1] = 0;
-    else if (kspec == 0) tiles[1] = ((d.Wv + YB_TX - 1) / YB_TX) * ((d.Hv + YB_YB - 1) / YB_YB) * 4 * d.L;
     else tiles[1] = (int)((2LL * d.Wp * d.L + YP_COLS - 1) / YP_COLS);  // one column of one pair per thread
+    if (kspec == 0) tiles[1] *= (d.Hv + YG_NB - 1) / YG_NB;
     if (!valid) tiles[2] = 0;
     else if (sh.zt) tiles[2] = ((d.Wv + ZT_X - 1) / ZT_X) * ((d.Hv + ZT_Y - 1) / ZT_Y);
-    else if (kspec == 0) tiles[2] = ((d.Wv + ZB_TX - 1) / ZB_TX) * ((d.Lv + ZB_ZB - 1) / ZB_ZB) * d.Hv;
     else tiles[2] = (int)(((long long)d.Wp * d.Hv + ZP_COLS - 1) / ZP_COLS) * ((d.Lv + sh.zout - 1) / sh.zout);
     tiles[3] = ((d.W + ST_OX - 1) / ST_OX) * ((d.H + ST_OY - 1) / ST_OY) * ((d.L + zc - 1) / zc);
     // expanded data term: gauss_x, second y-pass, gauss_z, gauss_border

@@ -15,7 +15,7 @@ cudaError_t RSF_CAT(launch_ypass_, RSF_K)(const SubVolDev *svs, const int *pre, 
 #if RSF_K > 0
     ypass_kernel<RSF_K><<<blocks, YP_COLS, 0, st>>>(svs, pre, c);
 #else
-    ypass_generic_kernel<0><<<blocks, YB_TX, 0, st>>>(svs, pre, c);
+    ypass_chunk_kernel<YG_NB><<<blocks, YP_COLS, 0, st>>>(svs, pre, c);
 #endif
     return cudaGetLastError();
 }

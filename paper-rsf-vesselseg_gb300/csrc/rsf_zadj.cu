@@ -1,6 +1,7 @@
 // rsf_zadj.cu -- the z-pass with the adjoint's emit (the data-term adjoint instead
 // of the data factor) for one specialised tap count (compiled once per
-// -DRSF_K value; a unit of its own so that it compiles beside the z-pass).
+// -DRSF_K value, 0 for the run-time tap count; a unit of its own so that it
+// compiles beside the z-pass).
 #include "rsf_kernels.cuh"
 
 #ifndef RSF_K
@@ -11,14 +12,20 @@
 
 namespace rsf {
 
+#if RSF_K > 0
 cudaError_t RSF_CAT(config_zpass_adjoint_, RSF_K)() {
     return cudaFuncSetAttribute(zpass_adjoint_kernel<RSF_K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)zpass_smem(RSF_K));
 }
+#endif
 
 cudaError_t RSF_CAT(launch_zpass_adjoint_, RSF_K)(const SubVolDev *svs, const int *pre, int blocks,
                                                   const StepConst &c, const AdjVol *vols, cudaStream_t st) {
+#if RSF_K > 0
     zpass_adjoint_kernel<RSF_K><<<blocks, ZP_COLS, zpass_smem(RSF_K), st>>>(svs, pre, c, vols);
+#else
+    zchunk_adjoint_kernel<ZG_NB><<<blocks, ZP_COLS, 0, st>>>(svs, pre, c, vols);
+#endif
     return cudaGetLastError();
 }
 

@@ -17,8 +17,8 @@ cudaError_t RSF_CAT(launch_zpass_, RSF_K)(const SubVolDev *svs, const int *pre, 
     (void)dbg;
     zpass_kernel<RSF_K><<<blocks, ZP_COLS, zpass_smem(RSF_K), st>>>(svs, pre, c);
 #else
-    if (dbg) zpass_generic_kernel<true><<<blocks, ZB_TX, 0, st>>>(svs, pre, c, *dbg);
-    else zpass_generic_kernel<false><<<blocks, ZB_TX, 0, st>>>(svs, pre, c, DebugOut{nullptr, 0});
+    if (dbg) zpass_chunk_kernel<true><<<blocks, ZP_COLS, 0, st>>>(svs, pre, c, *dbg);
+    else zpass_chunk_kernel<false><<<blocks, ZP_COLS, 0, st>>>(svs, pre, c, DebugOut{nullptr, 0});
 #endif
     return cudaGetLastError();
 }

@@ -48,3 +48,17 @@ def test_value_ranges(scale, eps, spread, orc, cuda, rsflib):
     with np.errstate(over="ignore"):
         img = (scale * rng.random(shape)).astype(np.float32)
     _run(orc, shape, Params(sigma=3.0, dt=0.1, mu=0.1, lambda1=1e-3, lambda2=2e-3, nu=0.1, eps=eps), phi, img, 1)
+
+
+@pytest.mark.parametrize("sigma", [0.75, 1.0, 1.5, 2.0, 2.5, 6.0, 10.0])
+@pytest.mark.parametrize("extra", [(0, 0, 0), (1, 2, 3), (8, 16, 5), (9, 33, 41)])
+def test_run_time_tap_counts(sigma, extra, orc, cuda, rsflib):
+    """Tap counts without kernels of their own: chunks of 5 or 9 (x), 16 (y) and 8 (z) taps and outputs."""
+    from rsf_gb300 import Params
+
+    k = len(orc.taps(sigma))
+    shape = tuple(k + e for e in extra)
+    rng = np.random.default_rng(k)
+    phi = np.clip(4.0 * rng.standard_normal(shape), -3.0, 3.0).astype(np.float32)
+    img = rng.integers(0, 256, shape).astype(np.uint8 if extra[0] % 2 else np.float32)
+    _run(orc, shape, Params(sigma=sigma, dt=0.1, mu=1.0, lambda1=1.0, lambda2=0.5, nu=65.025, eps=0.2), phi, img, 2)
