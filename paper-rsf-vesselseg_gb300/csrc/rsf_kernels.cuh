@@ -867,10 +867,33 @@ __device__ __forceinline__ float border_data(const unsigned char *ip, const Step
 // reference's order (y outer, then x, then z) with each term fused in double
 // and rounded to float.  f(c) comes from the z-pass in the valid region and
 // is 30/30 = 1 in the border band.  Writes the data factor of every voxel;
-// runs on the stencil's tiling (lanes 1..30 x warps 1..14 x 32 planes).
+// runs on the stencil's tiling (lanes 1..30 x warps 1..14 x c.zc planes), a
+// grid row per BOX_Z of the planes.
+//
+// Double precision is what bounds the sum in its own terms (four operations
+// and six conversions per neighbour on a pipe with 1/64 of the FP32 rate), so
+// the terms are formed in pairs of floats (d^2 and w d^2 by their exact residuals,
+// the sum by Knuth's two-sum), e_out and e_in in the two lanes of packed
+// instructions.  That gives the sum to within 2^-45 of its size, while the
+// double sequence is within 2^-52; where the two ends of a 2^-43 margin round
+// to the same float, that float is the reference's.  Elsewhere (one term in
+// 2^18) the z column is redone in double.  72x100x131 voxels, s = 1: 809 us per
+// launch in double, BOX_MEASURED so.
 // ---------------------------------------------------------------------------
+// One z column of the box in double, from the sums before it.
+static __device__ __noinline__ float2 box_column_double(const void *img, size_t i, size_t step, int n, int f32,
+                                                        double wt, float fo, float fi, float2 s) {
+    for (int q = 0; q < n; ++q) {
+        const float In = load_img(img, i + (size_t)q * step, f32);
+        const float d1 = __fsub_rn(In, fo), d2 = __fsub_rn(In, fi);
+        s.x = __double2float_rn(__fma_rn(__dmul_rn(wt, (double)d1), (double)d1, (double)s.x));
+        s.y = __double2float_rn(__fma_rn(__dmul_rn(wt, (double)d2), (double)d2, (double)s.y));
+    }
+    return s;
+}
+
 template <bool DEBUG>
-__global__ void __launch_bounds__(ST_WARPS * 32) box_kernel(const SubVolDev *__restrict__ svs,
+__global__ void __launch_bounds__(ST_WARPS * 32, 2) box_kernel(const SubVolDev *__restrict__ svs,
                                                             const int *__restrict__ pre, const StepConst c,
                                                             DebugOut dbg) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -885,37 +908,59 @@ __global__ void __launch_bounds__(ST_WARPS * 32) box_kernel(const SubVolDev *__r
     const int tz = t / nty;
     const int x = tx * ST_OX - 1 + lane, y = ty * ST_OY - 1 + w;
     if (lane < 1 || lane > ST_OX || w < 1 || w > ST_OY || x >= s.W || y >= s.H) return;
-    const int z0 = tz * c.zc, z1 = min(z0 + c.zc, s.L);
+    const int z0 = tz * c.zc + (int)blockIdx.y * BOX_Z, z1 = min(min(z0 + BOX_Z, tz * c.zc + c.zc), s.L);
     const int bs = c.box, r = c.r;
     const double wt = 1.0 / (double)((2 * bs + 1) * (2 * bs + 1));
+    const float2 wh = dup2((float)wt), wl = dup2((float)(wt - (double)(float)wt));
     const size_t WH = (size_t)s.W * s.H, nvalid = (size_t)s.Wp * s.Hv * s.Lv;
     float *dfull = s.db + 2 * nvalid;
     const bool valid_xy = s.Wv > 0 && x >= r && x < r + s.Wv && y >= r && y < r + s.Hv;
     for (int z = z0; z < z1; ++z) {
+        const size_t vi = (size_t)z * WH + (size_t)y * s.W + x;
         float fo = 1.0f, fi = 1.0f;
         if (valid_xy && z >= r && z < r + s.Lv) {
             const size_t di = ((size_t)(z - r) * s.Hv + (y - r)) * s.Wp + (x - r);
             fo = s.db[di];
             fi = s.db[nvalid + di];
+        } else if (!DEBUG && c.lam_equal && !c.img_f32) {
+            dfull[vi] = data_factor(0.0f, 0.0f, c.l1, c.l2, true);
+            continue;
         }
-        float s1 = 0.0f, s2 = 0.0f;
-        for (int u = -bs; u <= bs; ++u) {
-            const int yy = y + u;
-            if (yy < 0 || yy >= s.H) continue;
-            for (int v = -bs; v <= bs; ++v) {
-                const int xx = x + v;
-                if (xx < 0 || xx >= s.W) continue;
-                for (int q = -bs; q <= bs; ++q) {
-                    const int zz = z + q;
-                    if (zz < 0 || zz >= s.L) continue;
-                    const float In = load_img(s.img, (size_t)zz * WH + (size_t)yy * s.W + xx, c.img_f32);
-                    const float d1 = __fsub_rn(In, fo), d2 = __fsub_rn(In, fi);
-                    s1 = __double2float_rn(__fma_rn(__dmul_rn(wt, (double)d1), (double)d1, (double)s1));
-                    s2 = __double2float_rn(__fma_rn(__dmul_rn(wt, (double)d2), (double)d2, (double)s2));
+        // fits of at least 2^-20 keep every nonzero difference above 2^-45 and
+        // its square's residuals in the normal range
+        const bool exact = fabsf(fo) >= 0x1p-20f && fabsf(fi) >= 0x1p-20f;
+        const int q0 = max(z - bs, 0), nq = min(z + bs, s.L - 1) - q0 + 1;
+        float2 e = make_float2(0.0f, 0.0f);
+        for (int yy = max(y - bs, 0); yy <= min(y + bs, s.H - 1); ++yy) {
+            for (int xx = max(x - bs, 0); xx <= min(x + bs, s.W - 1); ++xx) {
+                const size_t i0 = (size_t)q0 * WH + (size_t)yy * s.W + xx;
+                float2 sum = e;
+                bool sure = exact;
+                for (int qc = 0; qc < nq; qc += 3) {
+                    float In[3];  // loads of three terms in flight together
+#pragma unroll
+                    for (int m = 0; m < 3; ++m)
+                        In[m] = qc + m < nq ? load_img(s.img, i0 + (size_t)(qc + m) * WH, c.img_f32) : 0.0f;
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) {
+                        if (qc + m >= nq) break;
+                        const float2 d = make_float2(__fsub_rn(In[m], fo), __fsub_rn(In[m], fi));
+                        const float2 ph = mul2(d, d), pl = fma2(d, d, neg2(ph));
+                        const float2 qh = mul2(wh, ph);
+                        const float2 ql = fma2(wh, pl, fma2(wl, ph, fma2(wh, ph, neg2(qh))));
+                        const float2 t = add2(sum, qh);
+                        const float2 bb = sub2(t, sum);
+                        const float2 tail = add2(add2(sub2(sum, sub2(t, bb)), sub2(qh, bb)), ql);
+                        const float2 margin = mul2(t, dup2(0x1p-43f));
+                        const float2 hi = add2(t, add2(tail, margin)), lo = add2(t, sub2(tail, margin));
+                        sure = sure && hi.x == lo.x && hi.y == lo.y;
+                        sum = hi;
+                    }
                 }
+                e = sure ? sum : box_column_double(s.img, i0, WH, nq, c.img_f32, wt, fo, fi, e);
             }
         }
-        const size_t vi = (size_t)z * WH + (size_t)y * s.W + x;
+        const float s1 = e.x, s2 = e.y;
         dfull[vi] = data_factor(s1, s2, c.l1, c.l2, c.lam_equal != 0);
         if (DEBUG) {
             dbg.f[2 * dbg.n + vi] = s1;

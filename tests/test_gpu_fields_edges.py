@@ -62,3 +62,29 @@ def test_run_time_tap_counts(sigma, extra, orc, cuda, rsflib):
     phi = np.clip(4.0 * rng.standard_normal(shape), -3.0, 3.0).astype(np.float32)
     img = rng.integers(0, 256, shape).astype(np.uint8 if extra[0] % 2 else np.float32)
     _run(orc, shape, Params(sigma=sigma, dt=0.1, mu=1.0, lambda1=1.0, lambda2=0.5, nu=65.025, eps=0.2), phi, img, 2)
+
+
+@pytest.mark.parametrize("sigma2", [1.0, 2.0, 3.0])
+@pytest.mark.parametrize("kind", ["u8", "black", "f32", "tiny", "huge", "mixed"])
+def test_box_term_in_float_pairs(sigma2, kind, orc, cuda, rsflib):
+    """The box sum's float pairs against the double sequence: integers, zeros (fits of exactly 0), fractions,
+    and values that leave the pairs' range."""
+    from rsf_gb300 import Params, Workspace
+
+    shape = (19, 23, 31)
+    rng = np.random.default_rng(7)
+    phi = np.clip(4.0 * rng.standard_normal(shape), -3.0, 3.0).astype(np.float32)
+    img = {"u8": rng.integers(0, 256, shape).astype(np.uint8), "black": np.zeros(shape, np.uint8),
+           "f32": (200.0 * rng.random(shape)).astype(np.float32), "tiny": (1e-25 * rng.random(shape)).astype(np.float32),
+           "huge": (1e15 * rng.random(shape)).astype(np.float32),
+           "mixed": (10.0 ** rng.uniform(-12, 4, shape)).astype(np.float32)}[kind]
+    p = Params(sigma=1.0, dt=0.1, mu=0.5, lambda1=1e-3, lambda2=2e-3, nu=1.0, eps=1.0, sigma2=sigma2)
+    want = orc.evolve(phi, img.astype(np.float32),
+                      orc.params(sigma=1.0, dt=p.dt, mu=p.mu, lambda1=p.lambda1, lambda2=p.lambda2, nu=p.nu, eps=p.eps,
+                                 sigma2=sigma2), 2)
+    with Workspace(phi.size) as ws:
+        t = torch.from_numpy(phi.copy()).cuda()
+        ws.evolve(torch.from_numpy(img).cuda(), t, p, 2)
+        got = t.cpu().numpy()
+    same = (got.view(np.uint32) == want.view(np.uint32)) | (np.isnan(got) & np.isnan(want))
+    assert same.all(), f"{int((~same).sum())} voxels differ"
