@@ -36,6 +36,11 @@ rsf_status fail(rsf_status s, const char *msg) {
 }
 
 constexpr int64_t kMaxExtent = 1 << 20;
+// Batched iterations from which the loop is captured into a graph.  Capturing and
+// instantiating costs more than the few launches it replaces below that: a
+// training step of 4 iterations forward (two per call) and 4 back took 4.40 ms
+// with graphs always, 4.21 so; from 4 iterations on the two are level.
+constexpr int kGraphFrom = 4;
 }  // namespace
 
 void rsf::set_last_error(const char *msg) { std::snprintf(g_last_error, sizeof g_last_error, "%s", msg); }
@@ -413,7 +418,12 @@ rsf_status prepare(rsf_workspace *ws, const rsf_subvol *svs, int32_t n, int k, i
             return fail(RSF_ERR_CUDA, "TMA tensor map encoding of the y-pass fields failed");
     }
     for (int j = 0; j < rsf::NPRE; j++) totals[j] = pre[j * n1 + n];
-    cudaError_t e = cudaMemcpyAsync(ws->d_svs, h_svs, (size_t)n * sizeof(SubVolDev), cudaMemcpyHostToDevice, st);
+    const size_t bs = (size_t)n * sizeof(SubVolDev), bp = rsf::NPRE * (size_t)n1 * sizeof(int);
+    if (!shape->zt && bs + bp <= rsf::UPLOAD_BYTES) {
+        cudaError_t e = rsf::launch_upload(ws->d_svs, h_svs, bs, ws->d_pre, h_pre, bp, st);
+        return e == cudaSuccess ? RSF_OK : cuda_fail(e, "table upload");
+    }
+    cudaError_t e = cudaMemcpyAsync(ws->d_svs, h_svs, bs, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(ws->d_pre, h_pre, rsf::NPRE * (size_t)n1 * sizeof(int), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && shape->zt)
@@ -551,7 +561,7 @@ rsf_status run(rsf_workspace *ws, const rsf_params *p, rsf_dtype dtype, const rs
     }
     auto step = [&](int it, cudaStream_t on) {
         cudaEvent_t *ev = ws->timing ? &ws->events[(size_t)rsf::NKERN * it] : nullptr;
-        return rsf::launch_step(ws->d_svs, ws->d_pre, tot, c, it & 1, p->arith, ws->d_flag, nullptr, on, ev);
+        return rsf::launch_step(ws->d_svs, ws->d_pre, tot, c, it & 1, p->arith, it == 0, ws->d_flag, nullptr, on, ev);
     };
     cudaError_t e = cudaSuccess;
     if (!use_graph) {
@@ -605,7 +615,7 @@ rsf_status rsf_evolve(rsf_workspace *ws, const rsf_params *p, const void *image,
 rsf_status rsf_evolve_batched(rsf_workspace *ws, const rsf_params *p, rsf_dtype dtype, const rsf_subvol *subvols,
                               int32_t n, int32_t iters, void *stream) {
     if (!subvols) return fail(RSF_ERR_INVALID_ARGUMENT, "subvols is null");
-    return run(ws, p, dtype, subvols, n, iters, (cudaStream_t)stream, true);
+    return run(ws, p, dtype, subvols, n, iters, (cudaStream_t)stream, iters >= kGraphFrom);
 }
 
 rsf_status rsf_evolve_host(rsf_workspace *ws, const rsf_params *p, const void *image_host, rsf_dtype dtype,
@@ -663,7 +673,7 @@ rsf_status rsf_step_debug(rsf_workspace *ws, const rsf_params *p, const void *im
     StepConst c = make_const(p, k, taps, dtype, 1, sh, ws->d_maps);
     if (gauss && (s = gauss_pool(ws, &c.gdelta)) != RSF_OK) return s;
     const rsf::DebugOut dbg = {fields, (int64_t)W * H * L};
-    cudaError_t e = rsf::launch_step(ws->d_svs, ws->d_pre, tot, c, 0, p->arith, ws->d_flag, &dbg, st);
+    cudaError_t e = rsf::launch_step(ws->d_svs, ws->d_pre, tot, c, 0, p->arith, true, ws->d_flag, &dbg, st);
     return e == cudaSuccess ? RSF_OK : cuda_fail(e, "debug step");
 }
 
@@ -776,10 +786,15 @@ rsf_status rsf_step_adjoint_batched(rsf_workspace *ws, const rsf_params *p, rsf_
     }
     int tot[rsf::NADJ];
     for (int j = 0; j < rsf::NADJ; j++) tot[j] = h_pre[j * n1 + n];
-    cudaError_t e = cudaMemcpyAsync(ws->d_adj, h_adj, (size_t)n * sizeof(rsf::AdjVol), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(ws->d_adj_pre, h_pre, rsf::NADJ * (size_t)n1 * sizeof(int), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = ws->mark_stage(st);
+    const size_t ba = (size_t)n * sizeof(rsf::AdjVol), bp = rsf::NADJ * (size_t)n1 * sizeof(int);
+    cudaError_t e;
+    if (ba + bp <= rsf::UPLOAD_BYTES) {
+        e = rsf::launch_upload(ws->d_adj, h_adj, ba, ws->d_adj_pre, h_pre, bp, st);
+    } else {
+        e = cudaMemcpyAsync(ws->d_adj, h_adj, ba, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(ws->d_adj_pre, h_pre, bp, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = ws->mark_stage(st);
+    }
     if (e != cudaSuccess) return cuda_fail(e, "adjoint table upload");
     {
         std::vector<rsf_subvol> fw((size_t)n);
@@ -798,10 +813,10 @@ rsf_status rsf_step_adjoint_batched(rsf_workspace *ws, const rsf_params *p, rsf_
         const int *pre = ws->d_pre;
         const int f1 = n + 1;
         if (ftot[0] > 0) switch (kspec) {
-                case 21: e = rsf::launch_xpass_21(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, st); break;
-                case 29: e = rsf::launch_xpass_29(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, st); break;
-                case 35: e = rsf::launch_xpass_35(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, st); break;
-                default: e = rsf::launch_xpass_0(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, st); break;
+                case 21: e = rsf::launch_xpass_21(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, false, st); break;
+                case 29: e = rsf::launch_xpass_29(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, false, st); break;
+                case 35: e = rsf::launch_xpass_35(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, false, st); break;
+                default: e = rsf::launch_xpass_0(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, false, st); break;
             }
         if (e == cudaSuccess && ftot[1] > 0) switch (kspec) {
                 case 21: e = rsf::launch_ypass_21(svs, pre + f1, ftot[1], c, st); break;

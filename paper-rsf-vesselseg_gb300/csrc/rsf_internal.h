@@ -144,10 +144,17 @@ int choose_xrpw(const int *whl, int n, int k, int xb_w);
 int choose_zc(const int *whl, int n);  // whl: W, H, L of each sub-volume
 void valid_extents(int W, int H, int L, int k, int &Wv, int &Hv, int &Lv, int &Wp);
 
-// One iteration.  With `ev` (NKERN + 1 events) the events are recorded before
+// Copies two small host arrays (sizes in bytes, multiples of 4, at most
+// UPLOAD_BYTES together) to the device as one launch's parameters: the tables of
+// a small batch, without staging memory, events or the copy engine.
+constexpr size_t UPLOAD_BYTES = 2048;
+cudaError_t launch_upload(void *dst0, const void *src0, size_t bytes0, void *dst1, const void *src1, size_t bytes1,
+                          cudaStream_t st);
+
+// One iteration; `first`: the tables may have been uploaded just before.  With `ev` (NKERN + 1 events) the events are recorded before
 // the first and after every kernel, for per-kernel device times.
 cudaError_t launch_step(const SubVolDev *d_svs, const int *d_pre, const int *h_tot, const StepConst &c,
-                        int parity, int arith, unsigned *d_flag, const DebugOut *dbg, cudaStream_t st,
+                        int parity, int arith, bool first, unsigned *d_flag, const DebugOut *dbg, cudaStream_t st,
                         cudaEvent_t *ev = nullptr);
 
 cudaError_t configure_device();
@@ -180,7 +187,8 @@ enum AdjKernel { ADJ_TZ, ADJ_TY, ADJ_TX, ADJ_NRM, ADJ_PT, ADJ_W, ADJ_G };
 void adjoint_tiles(const AdjVol &v, int tiles[NADJ]);
 
 #define RSF_DECLARE_K(K)                                                                                      \
-    cudaError_t launch_xpass_##K(const SubVolDev *, const int *, int, const StepConst &, int, int, cudaStream_t); \
+    cudaError_t launch_xpass_##K(const SubVolDev *, const int *, int, const StepConst &, int, int, bool,          \
+                                 cudaStream_t);                                                                \
     cudaError_t config_xpass_##K();                                                                             \
     cudaError_t launch_ypass_##K(const SubVolDev *, const int *, int, const StepConst &, cudaStream_t);          \
     cudaError_t launch_zpass_##K(const SubVolDev *, const int *, int, const StepConst &, const DebugOut *,      \

@@ -179,7 +179,7 @@ extern "C" rsf_status rsf_evolve_noalloc(const rsf_params *p, const void *image,
     if (e == cudaSuccess && sh.zt) e = cudaMemcpyAsync(d_map, map, sizeof map, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_flag, 0, sizeof(unsigned), st);
     for (int it = 0; it < iters && e == cudaSuccess; it++)
-        e = rsf::launch_step(d_table, d_pre, tiles, c, it & 1, p->arith, d_flag, nullptr, st);
+        e = rsf::launch_step(d_table, d_pre, tiles, c, it & 1, p->arith, it == 0, d_flag, nullptr, st);
     if (e == cudaSuccess && (iters & 1))
         e = cudaMemcpyAsync(phi, phi2, (size_t)W * H * L * sizeof(float), cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess) {

@@ -11,8 +11,8 @@ cudaError_t launch_stencil(const SubVolDev *svs, const int *pre, int blocks, con
         else stencil_debug_kernel<Arith::Portable><<<blocks, T, 0, st>>>(svs, pre, c, parity, flag, *dbg);
     } else {
         constexpr int T = SP_WARPS * 32;
-        if (arith == 1) stencil_pair_kernel<Arith::Reference><<<blocks, T, 0, st>>>(svs, pre, c, parity, flag);
-        else stencil_pair_kernel<Arith::Portable><<<blocks, T, 0, st>>>(svs, pre, c, parity, flag);
+        return launch_dependent(true, arith == 1 ? stencil_pair_kernel<Arith::Reference> : stencil_pair_kernel<Arith::Portable>,
+                                (unsigned)blocks, T, 0, st, svs, pre, c, parity, flag);
     }
     return cudaGetLastError();
 }

@@ -352,6 +352,7 @@ __global__ void __launch_bounds__(SP_WARPS * 32, 3) stencil_pair_kernel(const Su
     }
 
     // The first SP_RING planes from z0 - 2 on.
+    pdl_wait();
     PairState S;
     const int first = k.z0 - 2;
     q.a += (ptrdiff_t)first * WH;
@@ -375,6 +376,7 @@ __global__ void __launch_bounds__(SP_WARPS * 32, 3) stencil_pair_kernel(const Su
     float2 acc = make_float2(0.0f, 0.0f);  // NaN once an output is not finite
     if (face) pair_planes<A, true>(k, c, S, q, sm, acc, xyin);
     else pair_planes<A, false>(k, c, S, q, sm, acc, xyin);
+    pdl_launch();
     if (!isfinite(acc.x + acc.y)) atomicOr(flag, kFlagNonFinite);
 }
 

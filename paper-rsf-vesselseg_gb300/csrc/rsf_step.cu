@@ -235,8 +235,31 @@ cudaError_t configure_device() {
     return e;
 }
 
+namespace {
+struct UploadWords {
+    unsigned w[UPLOAD_BYTES / 4];
+};
+__global__ void __launch_bounds__(256) upload_kernel(unsigned *d0, int n0, unsigned *d1, int n1,
+                                                     const __grid_constant__ UploadWords u) {
+    for (int i = threadIdx.x; i < n0 + n1; i += 256) {
+        if (i < n0) d0[i] = u.w[i];
+        else d1[i - n0] = u.w[i];
+    }
+}
+}  // namespace
+
+cudaError_t launch_upload(void *dst0, const void *src0, size_t bytes0, void *dst1, const void *src1, size_t bytes1,
+                          cudaStream_t st) {
+    UploadWords u;
+    std::memcpy(u.w, src0, bytes0);
+    std::memcpy(reinterpret_cast<unsigned char *>(u.w) + bytes0, src1, bytes1);
+    upload_kernel<<<1, 256, 0, st>>>(static_cast<unsigned *>(dst0), (int)(bytes0 / 4), static_cast<unsigned *>(dst1),
+                                     (int)(bytes1 / 4), u);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_step(const SubVolDev *svs, const int *pre, const int *tot, const StepConst &c, int parity,
-                        int arith, unsigned *flag, const DebugOut *dbg, cudaStream_t st, cudaEvent_t *ev) {
+                        int arith, bool first, unsigned *flag, const DebugOut *dbg, cudaStream_t st, cudaEvent_t *ev) {
     const int n1 = c.nsv + 1;
     const int kspec = kernel_k(c.k, arith, dbg != nullptr, c.box, c.gauss);
     cudaError_t e = cudaSuccess;
@@ -250,10 +273,10 @@ cudaError_t launch_step(const SubVolDev *svs, const int *pre, const int *tot, co
     if ((e = mark(0)) != cudaSuccess) return e;
     if (tot[0] > 0) {
         switch (kspec) {
-            case 21: e = launch_xpass_21(svs, pre, tot[0], c, parity, arith, st); break;
-            case 29: e = launch_xpass_29(svs, pre, tot[0], c, parity, arith, st); break;
-            case 35: e = launch_xpass_35(svs, pre, tot[0], c, parity, arith, st); break;
-            default: e = launch_xpass_0(svs, pre, tot[0], c, parity, arith, st); break;
+            case 21: e = launch_xpass_21(svs, pre, tot[0], c, parity, arith, !first, st); break;
+            case 29: e = launch_xpass_29(svs, pre, tot[0], c, parity, arith, !first, st); break;
+            case 35: e = launch_xpass_35(svs, pre, tot[0], c, parity, arith, !first, st); break;
+            default: e = launch_xpass_0(svs, pre, tot[0], c, parity, arith, !first, st); break;
         }
         if (e != cudaSuccess) return e;
     }

@@ -34,21 +34,16 @@ cudaError_t RSF_CAT(config_xpass_, RSF_K)() {
 }
 
 cudaError_t RSF_CAT(launch_xpass_, RSF_K)(const SubVolDev *svs, const int *pre, int blocks, const StepConst &c,
-                                          int parity, int arith, cudaStream_t st) {
+                                          int parity, int arith, bool dependent, cudaStream_t st) {
     const size_t smem = xpass_smem(RSF_K > 0 ? RSF_K : c.k, c.xb_w);
-    constexpr int T = XP_ROWS * 32;
+    auto kernel = c.xb_w == 5 ? xpass_kernel<RSF_K, 5, Arith::Portable> : xpass_kernel<RSF_K, 9, Arith::Portable>;
 #if RSF_K == 0
-    if (arith == 1) {
-        if (c.xb_w == 5) xpass_kernel<0, 5, Arith::Reference><<<blocks, T, smem, st>>>(svs, pre, c, parity);
-        else xpass_kernel<0, 9, Arith::Reference><<<blocks, T, smem, st>>>(svs, pre, c, parity);
-        return cudaGetLastError();
-    }
+    if (arith == 1)
+        kernel = c.xb_w == 5 ? xpass_kernel<0, 5, Arith::Reference> : xpass_kernel<0, 9, Arith::Reference>;
 #else
     (void)arith;
 #endif
-    if (c.xb_w == 5) xpass_kernel<RSF_K, 5, Arith::Portable><<<blocks, T, smem, st>>>(svs, pre, c, parity);
-    else xpass_kernel<RSF_K, 9, Arith::Portable><<<blocks, T, smem, st>>>(svs, pre, c, parity);
-    return cudaGetLastError();
+    return launch_dependent(dependent, kernel, (unsigned)blocks, XP_ROWS * 32, smem, st, svs, pre, c, parity);
 }
 
 }  // namespace rsf

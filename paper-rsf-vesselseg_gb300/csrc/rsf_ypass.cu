@@ -13,11 +13,10 @@ namespace rsf {
 cudaError_t RSF_CAT(launch_ypass_, RSF_K)(const SubVolDev *svs, const int *pre, int blocks, const StepConst &c,
                                           cudaStream_t st) {
 #if RSF_K > 0
-    ypass_kernel<RSF_K><<<blocks, YP_COLS, 0, st>>>(svs, pre, c);
+    return launch_dependent(true, ypass_kernel<RSF_K>, (unsigned)blocks, YP_COLS, 0, st, svs, pre, c);
 #else
-    ypass_chunk_kernel<YG_NB><<<blocks, YP_COLS, 0, st>>>(svs, pre, c);
+    return launch_dependent(true, ypass_chunk_kernel<YG_NB>, (unsigned)blocks, YP_COLS, 0, st, svs, pre, c);
 #endif
-    return cudaGetLastError();
 }
 
 }  // namespace rsf

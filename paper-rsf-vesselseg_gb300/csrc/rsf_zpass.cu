@@ -15,12 +15,12 @@ cudaError_t RSF_CAT(launch_zpass_, RSF_K)(const SubVolDev *svs, const int *pre, 
                                           const DebugOut *dbg, cudaStream_t st) {
 #if RSF_K > 0
     (void)dbg;
-    zpass_kernel<RSF_K><<<blocks, ZP_COLS, zpass_smem(RSF_K), st>>>(svs, pre, c);
+    return launch_dependent(true, zpass_kernel<RSF_K>, (unsigned)blocks, ZP_COLS, zpass_smem(RSF_K), st, svs, pre, c);
 #else
-    if (dbg) zpass_chunk_kernel<true><<<blocks, ZP_COLS, 0, st>>>(svs, pre, c, *dbg);
-    else zpass_chunk_kernel<false><<<blocks, ZP_COLS, 0, st>>>(svs, pre, c, DebugOut{nullptr, 0});
+    const DebugOut d = dbg ? *dbg : DebugOut{nullptr, 0};
+    return launch_dependent(true, dbg ? zpass_chunk_kernel<true> : zpass_chunk_kernel<false>, (unsigned)blocks, ZP_COLS, 0, st,
+                            svs, pre, c, d);
 #endif
-    return cudaGetLastError();
 }
 
 cudaError_t RSF_CAT(config_zpass_, RSF_K)() {
