@@ -28,8 +28,8 @@
 // Kernels: the forward step's x- and y-passes and the z-pass's adjoint variant
 // (zpass_adjoint_kernel, zchunk_adjoint_kernel), which the caller launches and
 // which leave the data-term adjoint; then here transposed blur z, y, x (the x
-// kernel forms H_bar); gradients and unit normals; the pointwise terms with the
-// parameter sums; the stencil adjoint w; the final D^T gather.  The blurs along y and z compute several
+// kernel forms H_bar); gradients; the pointwise terms with the parameter sums and
+// the stencil adjoint w; the final D^T gather.  The blurs along y and z compute several
 // consecutive outputs per thread; the last three kernels run on blocks of
 // 32 x 8 voxels, the others on one item per thread.  Every kernel covers the
 // whole batch in one launch: a block finds its volume in a block prefix
@@ -39,14 +39,13 @@
 // 4 floats per voxel):
 //   phi2 : H_bar
 //   xs   : x fields (4 Wp H L), then [0, 2N) the valid-layout adjoint pair
-//          and [2N, 4N) e_out, e_in (kappa_bar over e_out); then g_x, g_y in
-//          [0, 2N), later w_x, w_y
-//   ys   : y fields (4 Wp Hv L), then the z-transposed pair [0, 2N), the
-//          y-transposed pair at 2N; later g_z (then w_z), n_x, n_y, n_z
+//          (float2 per voxel) and [2N, 4N) e_out, e_in (w_z over e_out); then
+//          g_x, g_y in [0, 2N)
+//   ys   : y fields (4 Wp Hv L), then the z-transposed pair [0, 2N), the y-
+//          transposed pair at 2N; later g_z, 1/(|g|+1e-6), w_x, w_y
 #include <cuda_runtime.h>
 
-#include "rsf_arith.cuh"
-#include "rsf_internal.h"
+#include "rsf_kernels.cuh"
 
 namespace rsf {
 namespace {
@@ -54,7 +53,8 @@ namespace {
 constexpr int kThreads = 256;
 
 struct AdjConst {
-    float taps[MAXK];
+    float2 taps2[MAXK];  // (g, g) pairs
+    __device__ __forceinline__ unsigned long long tap2(int t) const { return pack2(taps2[t]); }
     int k, r;
     float eps, dt, mu, nu, l1, l2;
     int boundary;    // 0 reference (x = 0 reads the previous linear element), 1 clamp
@@ -85,92 +85,43 @@ __device__ __forceinline__ BlockVol block_vol(const int *__restrict__ pre, int n
     return {lo, (long long)(b - __ldg(pre + lo))};
 }
 
-// The stencil kernels run on blocks of 32 x 8 voxels of kWZ planes (w,
-// gather) or of kPointZ planes (pointwise terms).
+// The stencil kernels run on blocks of 32 x 8 voxels of kWZ planes (gather) or of
+// kPointZ planes (pointwise terms).
 constexpr int kBX = 32, kBY = 8;
-constexpr int kPointZ = 16;
-constexpr int kWZ = 8;  // planes per block of adj_w and adj_gather
+constexpr int kPointZ = 8;
+constexpr int kWZ = 8;  // planes per block of adj_gather
 
-struct Geo {
-    int W, H, L, boundary;
+// The difference rules of a voxel along one axis without branches (a warp that
+// touches a face would otherwise take the general and the inner form one after
+// the other).  D f = (f(i + r) - f(i - l)) / 2 with the offsets r, l; its
+// transpose gathers D^T v = m v(i - s) + c v(i) + p v(i + s) with s the axis
+// stride.  Along x the neighbours are the ones in memory: in the reference
+// boundary mode (kernel.cu:64-67) x = 0 reads the previous linear element, so
+// the last voxel of a row is read by the first one of the next.
+struct Axis {
+    long long s, r, l;
+    float m, c, p;
 };
-
-// Right and left linear indices of the central difference at voxel i.
-__device__ __forceinline__ void nb_x(const Geo &g, long long i, int x, long long &r, long long &l) {
-    r = x + 1 < g.W ? i + 1 : i;
-    if (x > 0) l = i - 1;
-    else l = g.boundary == 0 ? (i > 0 ? i - 1 : 0) : i;
-    if (x == g.W - 1) l = i - 1;
+__device__ __forceinline__ Axis axis_plain(int q, int n, long long s) {
+    const bool lo = q > 0, hi = q + 1 < n;
+    return {s, hi ? s : 0, lo ? s : 0, lo ? 0.5f : 0.0f, (hi ? 0.0f : 0.5f) - (lo ? 0.0f : 0.5f), hi ? -0.5f : 0.0f};
 }
-// y and z: (f[1] - f[0]) / 2 at 0, (f[n-1] - f[n-2]) / 2 at n - 1 (n >= 2).
-__device__ __forceinline__ void nb_axis(long long i, int q, int n, long long stride, long long &r, long long &l) {
-    const int qr = q + 1 < n ? q + 1 : n - 1;
-    const int ql = q > 0 ? q - 1 : 0;
-    r = i + (long long)(qr - q) * stride;
-    l = i + (long long)(ql - q) * stride;
-}
-
-__device__ __forceinline__ float diff_x_at(const Geo &g, const float *f, long long m, int x) {
-    long long r, l;
-    nb_x(g, m, x, r, l);
-    return 0.5f * (f[r] - f[l]);
-}
-__device__ __forceinline__ float diff_axis_at(const float *f, long long m, int q, int n, long long stride) {
-    long long r, l;
-    nb_axis(m, q, n, stride, r, l);
-    return 0.5f * (f[r] - f[l]);
-}
-
-// (D_x^T v)(j): the neighbours j-1, j, j+1 in linear order are the only
-// voxels whose difference reads j.
-// x is j's x coordinate; the linear neighbours of a row's end are the next
-// row's start and vice versa.  Branch-free: an out-of-range candidate is
-// read as j itself with coefficient 0, so that all loads issue together.
-template <class V>
-__device__ __forceinline__ float dT_x(const Geo &g, long long j, int x, long long N, V v) {
-    float acc = 0.0f;
-#pragma unroll
-    for (int d = -1; d <= 1; d++) {
-        const long long m0 = j + d;
-        const bool in = m0 >= 0 && m0 < N;
-        const long long m = in ? m0 : j;
-        const int mx = d == 0 ? x : d < 0 ? (x > 0 ? x - 1 : g.W - 1) : (x + 1 < g.W ? x + 1 : 0);
-        long long r, l;
-        nb_x(g, m, mx, r, l);
-        const float coef = in ? (r == j ? 0.5f : 0.0f) - (l == j ? 0.5f : 0.0f) : 0.0f;
-        acc = fmaf(coef, v(m), acc);
+// x at linear index i of N; i > 0 and i + 1 < N decide at the volume's ends.
+__device__ __forceinline__ Axis axis_x(const AdjVol &a, int boundary, int x, long long i, long long N) {
+    Axis k = axis_plain(x, a.W, 1);
+    if (boundary == 0) {
+        k.l = i > 0 ? 1 : 0;
+        k.c = (x + 1 < a.W ? 0.0f : 0.5f) - (i > 0 ? 0.0f : 0.5f);
+        k.p = i + 1 < N ? -0.5f : 0.0f;
     }
-    return acc;
+    return k;
 }
+// m v(i - s) + c v(i) + p v(i + s), v0 = v(i); a neighbour without weight is
+// not read (it may lie outside the volume).
 template <class V>
-__device__ __forceinline__ float dT_axis(long long j, int q, int n, long long stride, V v) {
-    float acc = 0.0f;
-#pragma unroll
-    for (int d = -1; d <= 1; d++) {
-        const bool in = q + d >= 0 && q + d < n;
-        const int qm = in ? q + d : q;
-        const long long m = j + (long long)(qm - q) * stride;
-        long long r, l;
-        nb_axis(m, qm, n, stride, r, l);
-        const float coef = in ? (r == j ? 0.5f : 0.0f) - (l == j ? 0.5f : 0.0f) : 0.0f;
-        acc = fmaf(coef, v(m), acc);
-    }
-    return acc;
-}
-
-// D_a^T v at a voxel that is neither first nor last along any axis: only
-// j - s (coefficient 1/2) and j + s (-1/2) read j, as in dT_x / dT_axis,
-// whose evaluation order this keeps (the coefficient-0 term of j itself
-// adds nothing to a finite sum).
-template <class V>
-__device__ __forceinline__ float dT_in(long long j, long long s, V v) {
-    return fmaf(-0.5f, v(j + s), 0.5f * v(j - s));
-}
-
-// The voxel is neither first nor last along any axis (the x = 0 and last-index
-// rules of the differences and of their transposes do not apply).
-__device__ __forceinline__ bool inner_voxel(const AdjVol &a, int x, int y, int z) {
-    return x >= 1 && x <= a.W - 2 && y >= 1 && y <= a.H - 2 && z >= 1 && z <= a.L - 2;
+__device__ __forceinline__ float gather3(const Axis &k, long long i, float v0, V v) {
+    const float vm = k.m != 0.0f ? v(i - k.s) : 0.0f, vp = k.p != 0.0f ? v(i + k.s) : 0.0f;
+    return fmaf(k.p, vp, fmaf(k.c, v0, k.m * vm));
 }
 
 // delta(phi) with a fast division: the adjoint needs the derivative's value,
@@ -182,104 +133,114 @@ __device__ __forceinline__ float dirac_fast(float phi, float eps) {
 __device__ __forceinline__ long long nvox(const AdjVol &a) { return (long long)a.W * a.H * a.L; }
 __device__ __forceinline__ long long item(const BlockVol &bv) { return bv.t * kThreads + threadIdx.x; }
 
-// Correlation of NB consecutive outputs start .. start+NB-1 along a strided
-// axis of nin inputs, register-blocked so that each input load feeds up to
-// NB outputs.  Valid: out[o] = sum_t g[t] in[o + t].  Transposed (the
-// adjoint of valid): out[o] = sum_t g[t] in[o - t] over 0 <= o - t < nin.
-template <int NB, bool TRANSPOSED>
-__device__ __forceinline__ void corr_block(const AdjConst &c, const float *__restrict__ col, long long stride,
-                                           int start, int nin, float (&acc)[NB]) {
-#pragma unroll
-    for (int m = 0; m < NB; ++m) acc[m] = 0.0f;
-    const int p0 = TRANSPOSED ? start - c.k + 1 : start;
-    const int p1 = TRANSPOSED ? start + NB : start + NB + c.k - 1;  // exclusive
-    for (int p = max(p0, 0); p < min(p1, nin); ++p) {
-        const float v = col[(long long)p * stride];
-#pragma unroll
-        for (int m = 0; m < NB; ++m) {
-            const int t = TRANSPOSED ? start + m - p : p - start - m;
-            if (t >= 0 && t < c.k) acc[m] = fmaf(v, c.taps[t], acc[m]);
-        }
-    }
-}
-
+// The transposed (full) correlations out[o] = sum_t g[t] in[o - t] over
+// 0 <= o - t < n, both fields of the pair (P, Q) in packed multiply-adds, taps in
+// chunks over a register window (conv_chunks of the forward kernels; the taps
+// are symmetric, so ascending inputs take them in either order).  Inputs
+// outside the range count 0.  4 x 96x112x96 voxels, 21 taps: z 40 -> 14 us, y
+// 55 -> 17, x 85 -> 29 against scalar sums with an index test per multiply-add.
 constexpr int kNB = 8;   // outputs per thread along z
-constexpr int kNBy = 4;  // outputs per thread along y (shorter columns keep more threads in flight)
+constexpr int kNBy = 8;  // and along y
 
-// Transposed (full) correlation along z: xs (Wv, Hv, Lv) -> ys (Wv, Hv, L), two fields.
-__global__ void __launch_bounds__(kThreads) adj_blurT_z(AdjConst c, const AdjVol *__restrict__ vols,
+// z: xs (Wv, Hv, Lv) -> ys (Wv, Hv, L).
+__global__ void __launch_bounds__(kThreads) adj_blurT_z(const __grid_constant__ AdjConst c,
+                                                        const AdjVol *__restrict__ vols,
                                                         const int *__restrict__ pre) {
     const BlockVol bv = block_vol(pre, c.nvol);
     const AdjVol a = vols[bv.v];
-    const long long nin = (long long)a.Wv * a.Hv * a.Lv, n = (long long)a.Wv * a.Hv * a.L;
     const long long plane = (long long)a.Wv * a.Hv;
     const int nzb = (a.L + kNB - 1) / kNB;
     const long long q = item(bv);
     if (q >= plane * nzb) return;
     const long long pxy = q % plane;
-    const int z0 = (int)(q / plane) * kNB;
-    for (int f = 0; f < 2; f++) {
-        float acc[kNB];
-        corr_block<kNB, true>(c, a.xs + f * nin + pxy, plane, z0, a.Lv, acc);
+    const int z0 = (int)(q / plane) * kNB, first = z0 - c.k + 1;
+    const unsigned long long *in = reinterpret_cast<const unsigned long long *>(a.xs) + pxy;
+    unsigned long long u[kNB], *out = reinterpret_cast<unsigned long long *>(a.ys) + z0 * plane + pxy;
+    conv_chunks<kNB>(c, [&](int i) {
+        const int p = first + i;
+        return p >= 0 && p < a.Lv ? __ldg(in + p * plane) : 0ull;
+    }, u);
 #pragma unroll
-        for (int m = 0; m < kNB; ++m)
-            if (z0 + m < a.L) a.ys[f * n + (long long)(z0 + m) * plane + pxy] = acc[m];
-    }
+    for (int m = 0; m < kNB; ++m)
+        if (z0 + m < a.L) out[m * plane] = u[m];
 }
 
-// Transposed correlation along y: ys (Wv, Hv, L) -> ys + 2N (Wv, H, L).
-__global__ void __launch_bounds__(kThreads) adj_blurT_y(AdjConst c, const AdjVol *__restrict__ vols,
+// y: ys (Wv, Hv, L) -> ys + 2N (Wv, H, L).
+__global__ void __launch_bounds__(kThreads) adj_blurT_y(const __grid_constant__ AdjConst c,
+                                                        const AdjVol *__restrict__ vols,
                                                         const int *__restrict__ pre) {
     const BlockVol bv = block_vol(pre, c.nvol);
     const AdjVol a = vols[bv.v];
-    const long long nin = (long long)a.Wv * a.Hv * a.L, n = (long long)a.Wv * a.H * a.L;
     const int nyb = (a.H + kNBy - 1) / kNBy;
     const long long q = item(bv);
     if (q >= (long long)a.Wv * nyb * a.L) return;
     const int xv = (int)(q % a.Wv);
     const long long t1 = q / a.Wv;
-    const int y0 = (int)(t1 % nyb) * kNBy;
+    const int y0 = (int)(t1 % nyb) * kNBy, first = y0 - c.k + 1;
     const int z = (int)(t1 / nyb);
-    float *out = a.ys + 2 * nvox(a);
-    for (int f = 0; f < 2; f++) {
-        float acc[kNBy];
-        corr_block<kNBy, true>(c, a.ys + f * nin + (long long)z * a.Hv * a.Wv + xv, a.Wv, y0, a.Hv, acc);
+    const unsigned long long *in = reinterpret_cast<const unsigned long long *>(a.ys) + (long long)z * a.Hv * a.Wv + xv;
+    unsigned long long u[kNBy], *out = reinterpret_cast<unsigned long long *>(a.ys + 2 * nvox(a)) +
+                                       ((long long)z * a.H + y0) * a.Wv + xv;
+    conv_chunks<kNBy>(c, [&](int i) {
+        const int p = first + i;
+        return p >= 0 && p < a.Hv ? __ldg(in + (long long)p * a.Wv) : 0ull;
+    }, u);
 #pragma unroll
-        for (int m = 0; m < kNBy; ++m)
-            if (y0 + m < a.H) out[f * n + ((long long)z * a.H + y0 + m) * a.Wv + xv] = acc[m];
-    }
+    for (int m = 0; m < kNBy; ++m)
+        if (y0 + m < a.H) out[(long long)m * a.Wv] = u[m];
 }
 
-// Transposed correlation along x and H_bar = I * P~ + Q~ over the volume,
-// into phi2 (0 for a volume without a valid region).
-__global__ void __launch_bounds__(kThreads) adj_blurT_x_hbar(AdjConst c, const AdjVol *__restrict__ vols,
-                                                             const int *__restrict__ pre) {
+// x, and H_bar = I * P~ + Q~ over the volume, into phi2 (0 for a volume without a
+// valid region).  A warp takes a segment of 32 kNBx voxels of one row, whose
+// inputs it stages in shared memory; a lane forms kNBx adjacent outputs (odd, so
+// that the lanes' 64-bit loads fall into distinct banks).
+constexpr int kNBx = 3;
+constexpr int kTxWarps = 8;
+__global__ void __launch_bounds__(32 * kTxWarps) adj_blurT_x_hbar(const __grid_constant__ AdjConst c,
+                                                                  const AdjVol *__restrict__ vols,
+                                                                  const int *__restrict__ pre) {
+    constexpr int XT = 32 * kNBx;
+    __shared__ unsigned long long slab_s[kTxWarps][XT + MAXK + 2 * kNBx];
     const BlockVol bv = block_vol(pre, c.nvol);
     const AdjVol a = vols[bv.v];
-    const long long N = nvox(a);
-    const long long nin = (long long)a.Wv * a.H * a.L;
-    const long long i = item(bv);
-    if (i >= N) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int ntx = (a.W + XT - 1) / XT;
+    const long long row = bv.t / ntx * kTxWarps + w;
+    if (row >= (long long)a.H * a.L) return;  // uniform per warp
+    const int x0 = (int)(bv.t % ntx) * XT;
+    const long long base = row * a.W;
     if (a.Wv == 0) {
-        a.phi2[i] = 0.0f;
+        for (int x = x0 + lane; x < min(x0 + XT, a.W); x += 32) a.phi2[base + x] = 0.0f;
         return;
     }
-    const float *in = a.ys + 2 * N;
-    const int x = (int)(i % a.W);
-    const long long row = i / a.W;
-    const int a0 = max(0, x - a.Wv + 1), a1 = min(c.k - 1, x);
-    float p = 0.0f, q = 0.0f;
-    for (int t = a0; t <= a1; t++) {
-        const long long s = row * a.Wv + (x - t);
-        p = fmaf(in[s], c.taps[t], p);
-        q = fmaf(in[nin + s], c.taps[t], q);
+    // slab[j]: input x0 - (k - 1) + j
+    unsigned long long *slab = slab_s[w];
+    const unsigned long long *in = reinterpret_cast<const unsigned long long *>(a.ys + 2 * nvox(a)) + row * a.Wv;
+    const int first = x0 - c.k + 1, span = XT + c.k - 1;
+    for (int j = lane; j < span; j += 32) {
+        const int p = first + j;
+        slab[j] = p >= 0 && p < a.Wv ? __ldg(in + p) : 0ull;
     }
-    a.phi2[i] = fmaf(img_at(a.img, i, c.img_f32), p, q);
+    __syncwarp();
+    // outputs top, top - 1, ..: input o - t is slab[o - x0 + k - 1 - t]
+    const int top = kNBx * lane + kNBx - 1;
+    unsigned long long u[kNBx];
+    conv_chunks<kNBx>(c, [&](int i) { return slab[max(top + c.k - 1 - i, 0)]; }, u);
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < kNBx; ++m) slab[top - m] = u[m];
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < kNBx; ++m) {
+        const int x = x0 + 32 * m + lane;
+        const float2 pq = unpack2(slab[32 * m + lane]);
+        if (x < a.W) a.phi2[base + x] = fmaf(img_at(a.img, base + x, c.img_f32), pq.x, pq.y);
+    }
 }
 
-// Gradient g = D phi and unit normals n = g / (|g| + 1e-6), stored so that
-// the stencil adjoint reads them at its neighbours instead of recomputing:
-// g_x, g_y to xs, xs + N; g_z, n_x, n_y, n_z to ys .. ys + 3N.
+// Gradient g = D phi and 1 / (|g| + 1e-6), stored so that the kernels after it
+// read them at their neighbours instead of recomputing (the unit normal is the
+// product): g_x, g_y to xs, xs + N; g_z, 1 / (|g| + 1e-6) to ys, ys + N.
 __global__ void __launch_bounds__(kThreads) adj_normals(AdjConst c, const AdjVol *__restrict__ vols,
                                                         const int *__restrict__ pre) {
     const BlockVol bv = block_vol(pre, c.nvol);
@@ -287,29 +248,18 @@ __global__ void __launch_bounds__(kThreads) adj_normals(AdjConst c, const AdjVol
     const long long N = nvox(a);
     const long long i = item(bv);
     if (i >= N) return;
-    const Geo g = {a.W, a.H, a.L, c.boundary};
     const int x = (int)(i % a.W);
     const long long t1 = i / a.W;
     const int y = (int)(t1 % a.H);
     const int z = (int)(t1 / a.H);
-    const long long plane = (long long)a.W * a.H;
-    float gx, gy, gz;
-    if (inner_voxel(a, x, y, z)) {
-        gx = 0.5f * (a.phi[i + 1] - a.phi[i - 1]);
-        gy = 0.5f * (a.phi[i + a.W] - a.phi[i - a.W]);
-        gz = 0.5f * (a.phi[i + plane] - a.phi[i - plane]);
-    } else {
-        gx = diff_x_at(g, a.phi, i, x);
-        gy = diff_axis_at(a.phi, i, y, a.H, a.W);
-        gz = diff_axis_at(a.phi, i, z, a.L, plane);
-    }
-    const float rs = __frcp_rn(sqrtf(gx * gx + gy * gy + gz * gz) + 1e-6f);
+    const Axis ax = axis_x(a, c.boundary, x, i, N), ay = axis_plain(y, a.H, a.W),
+               az = axis_plain(z, a.L, (long long)a.W * a.H);
+    auto diff = [&](const Axis &k) { return 0.5f * (a.phi[i + k.r] - a.phi[i - k.l]); };
+    const float gx = diff(ax), gy = diff(ay), gz = diff(az);
     a.xs[i] = gx;
     a.xs[N + i] = gy;
     a.ys[i] = gz;
-    a.ys[N + i] = gx * rs;
-    a.ys[2 * N + i] = gy * rs;
-    a.ys[3 * N + i] = gz * rs;
+    a.ys[N + i] = __frcp_rn(sqrtf(gx * gx + gy * gy + gz * gz) + 1e-6f);
 }
 
 // The block's 32 x 8 column: x, y of this thread and the first z plane.
@@ -323,59 +273,117 @@ __device__ __forceinline__ Col col_of(const AdjVol &a, long long t, int zdepth) 
             (int)(t1 / nby) * zdepth};
 }
 
-// Pointwise terms and parameter sums:
+// Pointwise terms, parameter sums and the stencil adjoint:
 //   out = u + delta H_bar + delta' u dt (nu kappa - data),
-// with kappa = sum_a D_a n_a and Lap = sum_a D_a g_a from the stored fields.
-// A block covers a 32 x 8 column of kPointZ planes; the parameter sums are
-// reduced in the block and added with one double atomic per parameter and
-// block (the same four addresses for every block, so their number matters).
-// kappa_bar = u dt (nu delta - mu) is written over e_out (read first, by the
-// same thread) for adj_w.
-__global__ void __launch_bounds__(kBX * kBY) adj_point(AdjConst c, const AdjVol *__restrict__ vols,
+// with kappa = sum_a D_a n_a and Lap = sum_a D_a g_a from the stored fields, and
+//   w_a = D_a^T Lap_bar + (n_bar_a - (n_bar . n) g_a/|g|) / (|g| + 1e-6),
+// n_bar = D^T kappa_bar, kappa_bar = u dt (nu delta - mu), Lap_bar = u dt mu, to be
+// gathered by D_a^T: w_x, w_y to ys + 2N, ys + 3N, w_z over e_out (read first, by
+// the same thread).  A block covers a 32 x 8 column of kPointZ planes; kappa_bar
+// of the three planes around the voxel, g_z and the z normals ride in
+// registers, so each is formed once per column, and kappa_bar of the x and y
+// neighbours is formed from phi and u at them (one pass over the fields
+// instead of two with kappa_bar and the normals stored between them).  The
+// parameter sums are reduced in the block and added with one double atomic per
+// parameter and block (the same four addresses for every block, so their
+// number matters).  4 x 96x112x96 voxels: 227 us as two kernels with branches for
+// the face rules, 115 so (8 planes per block and 128 registers: 16 planes 122,
+// 4 planes 127; on one 43x58x67 volume 18.6, 11.2 and 8.0).
+__global__ void __launch_bounds__(kBX * kBY, 2) adj_point(AdjConst c, const AdjVol *__restrict__ vols,
                                                        const int *__restrict__ pre,
                                                        double *grads) {
     const BlockVol bv = block_vol(pre, c.nvol);
     const AdjVol a = vols[bv.v];
     const long long N = nvox(a);
     const long long plane = (long long)a.W * a.H;
-    const Geo g = {a.W, a.H, a.L, c.boundary};
-    const float *gxa = a.xs, *gya = a.xs + N, *gza = a.ys;
-    const float *nx = a.ys + N, *ny = a.ys + 2 * N, *nz = a.ys + 3 * N;
-    float *eo_v = a.xs + 2 * N;
-    const float *ei_v = a.xs + 3 * N;
+    const float *__restrict__ phi = a.phi, *__restrict__ uu = a.u;
+    const float *__restrict__ gxa = a.xs, *__restrict__ gya = a.xs + N, *__restrict__ gza = a.ys, *__restrict__ rsa = a.ys + N;
+    float *ez = a.xs + 2 * N;  // e_out, then w_z
+    const float *__restrict__ ei_v = a.xs + 3 * N;
+    float *__restrict__ wx = a.ys + 2 * N, *__restrict__ wy = a.ys + 3 * N;
+    auto kbar = [&](long long m) { return uu[m] * c.dt * (c.nu * dirac_fast(phi[m], c.eps) - c.mu); };
+    auto lbar = [&](long long m) { return uu[m] * c.dt * c.mu; };
     float s_l1 = 0.0f, s_l2 = 0.0f, s_mu = 0.0f, s_nu = 0.0f;
     const Col cl = col_of(a, bv.t, kPointZ);
     const int x = cl.x, y = cl.y;
     const int z1 = min(cl.z0 + kPointZ, a.L);
-    for (int z = cl.z0; z < z1 && x < a.W && y < a.H; ++z) {
-        const long long i = ((long long)z * a.H + y) * a.W + x;
-        const float ph = a.phi[i], ui = a.u[i];
-        const float I = img_at(a.img, i, c.img_f32);
-        const float delta = dirac_fast(ph, c.eps);
-        const float ddelta = __fdividef(-2.0f * ph * delta, fmaf(ph, ph, c.eps * c.eps));
-        long long rx, lx, ry, ly, rz, lz;
-        nb_x(g, i, x, rx, lx);
-        nb_axis(i, y, a.H, a.W, ry, ly);
-        nb_axis(i, z, a.L, plane, rz, lz);
-        const float kap = 0.5f * (nx[rx] - nx[lx]) + 0.5f * (ny[ry] - ny[ly]) + 0.5f * (nz[rz] - nz[lz]);
-        const float lap = 0.5f * (gxa[rx] - gxa[lx]) + 0.5f * (gya[ry] - gya[ly]) + 0.5f * (gza[rz] - gza[lz]);
-        const bool valid = a.Wv > 0 && x >= c.r && x < c.r + a.Wv && y >= c.r && y < c.r + a.Hv && z >= c.r &&
-                           z < c.r + a.Lv;
-        float eo, ei;
-        if (valid) {
-            eo = eo_v[i];
-            ei = ei_v[i];
-        } else {  // border band: f_out = f_in = 30 / 30
-            eo = ei = (I - 1.0f) * (I - 1.0f);
+    if (x < a.W && y < a.H) {
+        long long i = ((long long)cl.z0 * a.H + y) * a.W + x;
+        const Axis ay = axis_plain(y, a.H, a.W);
+        // of planes z - 1, z: kappa_bar, Lap_bar, g_z and 1/(|g|+1e-6)
+        float k0 = 0.0f, l0 = 0.0f, gz0 = 0.0f, r0 = 0.0f;
+        if (cl.z0 > 0) {
+            k0 = kbar(i - plane);
+            l0 = lbar(i - plane);
+            gz0 = gza[i - plane];
+            r0 = rsa[i - plane];
         }
-        const float data = c.l1 * eo - c.l2 * ei;
-        a.out[i] = ui + delta * a.phi2[i] + ddelta * ui * c.dt * (c.nu * kap - data);
-        const float ud = ui * c.dt, udd = ud * delta;
-        eo_v[i] = ud * (c.nu * delta - c.mu);
-        s_l1 = fmaf(-udd, eo, s_l1);
-        s_l2 = fmaf(udd, ei, s_l2);
-        s_mu = fmaf(ud, lap - kap, s_mu);
-        s_nu = fmaf(udd, kap, s_nu);
+        float k1 = kbar(i), l1 = lbar(i), gz1 = gza[i], r1 = rsa[i];
+        for (int z = cl.z0; z < z1; ++z, i += plane) {
+            float k2 = 0.0f, l2 = 0.0f, gz2 = 0.0f, r2 = 0.0f;
+            if (z + 1 < a.L) {
+                k2 = kbar(i + plane);
+                l2 = lbar(i + plane);
+                gz2 = gza[i + plane];
+                r2 = rsa[i + plane];
+            }
+            const float ph = phi[i], ui = uu[i];
+            const float I = img_at(a.img, i, c.img_f32);
+            const float gx = gxa[i], gy = gya[i];
+            const float delta = dirac_fast(ph, c.eps);
+            const float ddelta = __fdividef(-2.0f * ph * delta, fmaf(ph, ph, c.eps * c.eps));
+            const Axis ax = axis_x(a, c.boundary, x, i, N), az = axis_plain(z, a.L, plane);
+            // curvature and "Laplacian"; the z neighbours are at hand
+            const long long rx = i + ax.r, lx = i - ax.l, ry = i + ay.r, ly = i - ay.l;
+            const float gxr = gxa[rx], gxl = gxa[lx], gyr = gya[ry], gyl = gya[ly];
+            const float gzr = az.r ? gz2 : gz1, gzl = az.l ? gz0 : gz1;
+            const float kap = 0.5f * (gxr * rsa[rx] - gxl * rsa[lx]) + 0.5f * (gyr * rsa[ry] - gyl * rsa[ly]) +
+                              0.5f * (gzr * (az.r ? r2 : r1) - gzl * (az.l ? r0 : r1));
+            const float lap = 0.5f * (gxr - gxl) + 0.5f * (gyr - gyl) + 0.5f * (gzr - gzl);
+            // D^T of kappa_bar and Lap_bar
+            float nbx, nby, lbx, lby;
+            auto both = [&](const Axis &k, float &nb, float &lb) {
+                float um = 0.0f, up = 0.0f, pm = 0.0f, pp = 0.0f;
+                if (k.m != 0.0f) um = uu[i - k.s] * c.dt, pm = phi[i - k.s];
+                if (k.p != 0.0f) up = uu[i + k.s] * c.dt, pp = phi[i + k.s];
+                auto kb = [&](float u, float p) { return u * (c.nu * dirac_fast(p, c.eps) - c.mu); };
+                nb = fmaf(k.p, kb(up, pp), fmaf(k.c, k1, k.m * kb(um, pm)));
+                lb = fmaf(k.p, up * c.mu, fmaf(k.c, l1, k.m * (um * c.mu)));
+            };
+            both(ax, nbx, lbx);
+            both(ay, nby, lby);
+            const float nbz = fmaf(az.p, k2, fmaf(az.c, k1, az.m * k0)), lbz = fmaf(az.p, l2, fmaf(az.c, l1, az.m * l0));
+            const bool valid = a.Wv > 0 && x >= c.r && x < c.r + a.Wv && y >= c.r && y < c.r + a.Hv && z >= c.r &&
+                               z < c.r + a.Lv;
+            float eo, ei;
+            if (valid) {
+                eo = ez[i];
+                ei = ei_v[i];
+            } else {  // border band: f_out = f_in = 30 / 30
+                eo = ei = (I - 1.0f) * (I - 1.0f);
+            }
+            const float data = c.l1 * eo - c.l2 * ei;
+            a.out[i] = ui + delta * a.phi2[i] + ddelta * ui * c.dt * (c.nu * kap - data);
+            const float ud = ui * c.dt, udd = ud * delta;
+            s_l1 = fmaf(-udd, eo, s_l1);
+            s_l2 = fmaf(udd, ei, s_l2);
+            s_mu = fmaf(ud, lap - kap, s_mu);
+            s_nu = fmaf(udd, kap, s_nu);
+            const float mag = sqrtf(gx * gx + gy * gy + gz1 * gz1);
+            const float inv_mag = mag > 0.0f ? __frcp_rn(mag) : 0.0f;
+            const float ndot = nbx * (gx * r1) + nby * (gy * r1) + nbz * (gz1 * r1);
+            wx[i] = lbx + (nbx - ndot * gx * inv_mag) * r1;
+            wy[i] = lby + (nby - ndot * gy * inv_mag) * r1;
+            ez[i] = lbz + (nbz - ndot * gz1 * inv_mag) * r1;
+            k0 = k1;
+            k1 = k2;
+            l0 = l1;
+            l1 = l2;
+            gz0 = gz1;
+            gz1 = gz2;
+            r0 = r1;
+            r1 = r2;
+        }
     }
     if (grads) {  // uniform: every thread reaches the shuffles and the barrier
 #pragma unroll
@@ -401,54 +409,6 @@ __global__ void __launch_bounds__(kBX * kBY) adj_point(AdjConst c, const AdjVol 
     }
 }
 
-// Stencil adjoint: w_a = D_a^T Lap_bar + (n_bar_a - (n_bar . n) g_a/|g|) / (|g| + 1e-6)
-// with n_bar = D^T kappa_bar, to be gathered by D_a^T.  kappa_bar comes from
-// adj_point; Lap_bar = u dt mu.  Each thread reads g and n at its own voxel
-// only, so w is written over g in place.
-__global__ void __launch_bounds__(kBX * kBY) adj_w(AdjConst c, const AdjVol *__restrict__ vols,
-                                                   const int *__restrict__ pre) {
-    const BlockVol bv = block_vol(pre, c.nvol);
-    const AdjVol a = vols[bv.v];
-    const long long N = nvox(a);
-    const long long plane = (long long)a.W * a.H;
-    const Geo g = {a.W, a.H, a.L, c.boundary};
-    const float *kb = a.xs + 2 * N, *u = a.u;
-    auto kbar = [&](long long m) { return kb[m]; };
-    auto lbar = [&](long long m) { return u[m] * c.dt * c.mu; };
-    const Col cl = col_of(a, bv.t, kWZ);
-    const int x = cl.x, y = cl.y;
-    const int z1 = min(cl.z0 + kWZ, a.L);
-    for (int z = cl.z0; z < z1 && x < a.W && y < a.H; ++z) {
-        float *gxa = a.xs, *gya = a.xs + N, *gza = a.ys;
-        const float *nx = a.ys + N, *ny = a.ys + 2 * N, *nz = a.ys + 3 * N;
-        const long long i = ((long long)z * a.H + y) * a.W + x;
-        const float gx = gxa[i], gy = gya[i], gz = gza[i];
-        const float mag = sqrtf(gx * gx + gy * gy + gz * gz);
-        const float rs = __frcp_rn(mag + 1e-6f);
-        const float inv_mag = mag > 0.0f ? __frcp_rn(mag) : 0.0f;
-        float nbx, nby, nbz, lbx, lby, lbz;
-        if (inner_voxel(a, x, y, z)) {
-            nbx = dT_in(i, 1, kbar);
-            nby = dT_in(i, a.W, kbar);
-            nbz = dT_in(i, plane, kbar);
-            lbx = dT_in(i, 1, lbar);
-            lby = dT_in(i, a.W, lbar);
-            lbz = dT_in(i, plane, lbar);
-        } else {
-            nbx = dT_x(g, i, x, N, kbar);
-            nby = dT_axis(i, y, a.H, a.W, kbar);
-            nbz = dT_axis(i, z, a.L, plane, kbar);
-            lbx = dT_x(g, i, x, N, lbar);
-            lby = dT_axis(i, y, a.H, a.W, lbar);
-            lbz = dT_axis(i, z, a.L, plane, lbar);
-        }
-        const float ndot = nbx * nx[i] + nby * ny[i] + nbz * nz[i];
-        gxa[i] = lbx + (nbx - ndot * gx * inv_mag) * rs;
-        gya[i] = lby + (nby - ndot * gy * inv_mag) * rs;
-        gza[i] = lbz + (nbz - ndot * gz * inv_mag) * rs;
-    }
-}
-
 // out += sum_a D_a^T w_a; a non-finite result sets kFlagAdjointNonFinite.
 __global__ void __launch_bounds__(kBX * kBY) adj_gather(AdjConst c, const AdjVol *__restrict__ vols,
                                                         const int *__restrict__ pre, unsigned *flag) {
@@ -456,23 +416,28 @@ __global__ void __launch_bounds__(kBX * kBY) adj_gather(AdjConst c, const AdjVol
     const AdjVol a = vols[bv.v];
     const long long N = nvox(a);
     const long long plane = (long long)a.W * a.H;
-    const Geo g = {a.W, a.H, a.L, c.boundary};
-    const float *wx = a.xs, *wy = a.xs + N, *wz = a.ys;
-    auto vx = [&](long long m) { return wx[m]; };
-    auto vy = [&](long long m) { return wy[m]; };
-    auto vz = [&](long long m) { return wz[m]; };
+    const float *__restrict__ wx = a.ys + 2 * N, *__restrict__ wy = a.ys + 3 * N, *__restrict__ wz = a.xs + 2 * N;
     const Col cl = col_of(a, bv.t, kWZ);
     const int x = cl.x, y = cl.y;
+    if (x >= a.W || y >= a.H) return;
     const int z1 = min(cl.z0 + kWZ, a.L);
-    for (int z = cl.z0; z < z1 && x < a.W && y < a.H; ++z) {
-        const long long i = ((long long)z * a.H + y) * a.W + x;
-        const float d = inner_voxel(a, x, y, z)
-                            ? dT_in(i, 1, vx) + dT_in(i, a.W, vy) + dT_in(i, plane, vz)
-                            : dT_x(g, i, x, N, vx) + dT_axis(i, y, a.H, a.W, vy) + dT_axis(i, z, a.L, plane, vz);
+    const Axis ay = axis_plain(y, a.H, a.W);
+    long long i = ((long long)cl.z0 * a.H + y) * a.W + x;
+    float bad = 0.0f;  // NaN once a result is not finite
+    float z0v = cl.z0 > 0 ? wz[i - plane] : 0.0f, zcv = wz[i];  // w_z of planes z - 1, z
+    for (int z = cl.z0; z < z1; ++z, i += plane) {
+        const float z2v = z + 1 < a.L ? wz[i + plane] : 0.0f;
+        const Axis ax = axis_x(a, c.boundary, x, i, N), az = axis_plain(z, a.L, plane);
+        const float d = gather3(ax, i, wx[i], [&](long long m) { return wx[m]; }) +
+                        gather3(ay, i, wy[i], [&](long long m) { return wy[m]; }) +
+                        fmaf(az.p, z2v, fmaf(az.c, zcv, az.m * z0v));
         const float v = a.out[i] + d;
         a.out[i] = v;
-        if (!isfinite(v) && flag) atomicOr(flag, kFlagAdjointNonFinite);
+        bad = fmaf(v, 0.0f, bad);
+        z0v = zcv;
+        zcv = z2v;
     }
+    if (!isfinite(bad) && flag) atomicOr(flag, kFlagAdjointNonFinite);
 }
 
 long long cdiv(long long a, long long b) { return (a + b - 1) / b; }
@@ -488,10 +453,9 @@ void adjoint_tiles(const AdjVol &v, int tiles[NADJ]) {
         t[ADJ_TZ] = cdiv((long long)v.Wv * v.Hv * cdiv(v.L, kNB), kThreads);
         t[ADJ_TY] = cdiv((long long)v.Wv * cdiv(v.H, kNBy) * v.L, kThreads);
     }
-    t[ADJ_TX] = cdiv(N, kThreads);
+    t[ADJ_TX] = cdiv(v.W, 32 * kNBx) * cdiv((long long)v.H * v.L, kTxWarps);
     t[ADJ_NRM] = cdiv(N, kThreads);
     t[ADJ_PT] = bxy * cdiv(v.L, kPointZ);
-    t[ADJ_W] = bxy * cdiv(v.L, kWZ);
     t[ADJ_G] = bxy * cdiv(v.L, kWZ);
     for (int j = 0; j < NADJ; j++) tiles[j] = t[j] > 0x7fffffffLL ? -1 : (int)t[j];
 }
@@ -499,7 +463,7 @@ void adjoint_tiles(const AdjVol &v, int tiles[NADJ]) {
 cudaError_t launch_step_adjoint(const float *taps, int k, const AdjScalars &s, const AdjVol *vols, const int *pre,
                                 int n, const int *tot, double *grads, unsigned *flag, cudaStream_t st) {
     AdjConst c;
-    for (int t = 0; t < MAXK; t++) c.taps[t] = t < k ? taps[t] : 0.0f;
+    for (int t = 0; t < MAXK; t++) c.taps2[t] = t < k ? make_float2(taps[t], taps[t]) : make_float2(0.0f, 0.0f);
     c.k = k;
     c.r = (k - 1) / 2;
     c.eps = s.eps;
@@ -516,10 +480,9 @@ cudaError_t launch_step_adjoint(const float *taps, int k, const AdjScalars &s, c
     const dim3 b2(kBX, kBY, 1);
     if (tot[ADJ_TZ] > 0) adj_blurT_z<<<tot[ADJ_TZ], kThreads, 0, st>>>(c, vols, P(ADJ_TZ));
     if (tot[ADJ_TY] > 0) adj_blurT_y<<<tot[ADJ_TY], kThreads, 0, st>>>(c, vols, P(ADJ_TY));
-    if (tot[ADJ_TX] > 0) adj_blurT_x_hbar<<<tot[ADJ_TX], kThreads, 0, st>>>(c, vols, P(ADJ_TX));
+    if (tot[ADJ_TX] > 0) adj_blurT_x_hbar<<<tot[ADJ_TX], 32 * kTxWarps, 0, st>>>(c, vols, P(ADJ_TX));
     if (tot[ADJ_NRM] > 0) adj_normals<<<tot[ADJ_NRM], kThreads, 0, st>>>(c, vols, P(ADJ_NRM));
     if (tot[ADJ_PT] > 0) adj_point<<<tot[ADJ_PT], b2, 0, st>>>(c, vols, P(ADJ_PT), grads);
-    if (tot[ADJ_W] > 0) adj_w<<<tot[ADJ_W], b2, 0, st>>>(c, vols, P(ADJ_W));
     if (tot[ADJ_G] > 0) adj_gather<<<tot[ADJ_G], b2, 0, st>>>(c, vols, P(ADJ_G), flag);
     return cudaGetLastError();
 }

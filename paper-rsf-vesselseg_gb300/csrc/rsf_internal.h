@@ -179,10 +179,10 @@ struct AdjVol {
     int Wv, Hv, Lv;    // valid blur extents; all > 0 or all 0
 };
 // Adjoint kernels with a block prefix array each (rsf_adjoint.cu): the
-// transposed blurs z, y, x, normals, pointwise terms, w, gather.  (The recompute
+// transposed blurs z, y, x, gradients, pointwise terms, gather.  (The recompute
 // before them runs in the forward step's kernels.)
-constexpr int NADJ = 7;
-enum AdjKernel { ADJ_TZ, ADJ_TY, ADJ_TX, ADJ_NRM, ADJ_PT, ADJ_W, ADJ_G };
+constexpr int NADJ = 6;
+enum AdjKernel { ADJ_TZ, ADJ_TY, ADJ_TX, ADJ_NRM, ADJ_PT, ADJ_G };
 // Blocks of each adjoint kernel for one volume.
 void adjoint_tiles(const AdjVol &v, int tiles[NADJ]);
 

@@ -348,8 +348,8 @@ __global__ void __launch_bounds__(YP_COLS) ypass_kernel(const SubVolDev *__restr
 // The taps go in chunks of YG_NB over a window of 2 YG_NB inputs in registers,
 // whose upper half is loaded a chunk ahead, so a tap costs YG_NB multiply-adds,
 // one load and no index test.
-template <int NB, class Load>
-__device__ __forceinline__ void conv_chunks(const StepConst &c, Load load, unsigned long long (&u)[NB]) {
+template <int NB, class Const, class Load>
+__device__ __forceinline__ void conv_chunks(const Const &c, Load load, unsigned long long (&u)[NB]) {
     unsigned long long w[2 * NB];
 #pragma unroll
     for (int m = 0; m < NB; ++m) {
@@ -605,7 +605,8 @@ __global__ void __launch_bounds__(ZP_COLS) zpass_chunk_kernel(const SubVolDev *_
 // The adjoint's recompute of the fits (rsf_adjoint.cu): the forward z-pass,
 // emitting at each valid voxel, instead of the data factor,
 //   e_out = (I - f_out)^2 and e_in at the full-volume index, and the pair
-//   (B1_bar - B3_bar, B2_bar - B4_bar) in the valid layout (row stride Wv),
+//   (B1_bar - B3_bar, B2_bar - B4_bar) as a float2 in the valid layout (row
+//   stride Wv),
 // with B1..B4 the blurs of I H, H, I (1-H), 1-H, f_out = B1 / B2,
 // f_in = B3 / B4, and for data_bar = -u dt delta(phi)
 //   f_out_bar = -2 (I - f_out) lambda1 data_bar, f_in_bar = 2 (I - f_in) lambda2 data_bar,
@@ -647,8 +648,8 @@ __global__ void __launch_bounds__(ZP_COLS, zpass_blocks(K)) zpass_adjoint_kernel
     const size_t esz = c.img_f32 ? 4 : 1, plane = (size_t)s.W * s.H;
     size_t v = ((size_t)(z.o0 + c.r) * s.H + (z.y + c.r)) * s.W + (z.x + c.r);  // the next load's voxel
     float *eo = a.xs + 2 * plane * s.L + v, *ei = eo + plane * s.L;
-    const size_t nv = (size_t)s.Wv * s.Hv * s.Lv, vplane = (size_t)s.Wv * s.Hv;
-    float *pq = a.xs + (size_t)z.o0 * vplane + (size_t)z.y * s.Wv + z.x;
+    const size_t vplane = (size_t)s.Wv * s.Hv;
+    float2 *pq = reinterpret_cast<float2 *>(a.xs) + (size_t)z.o0 * vplane + (size_t)z.y * s.Wv + z.x;
     struct In {
         unsigned i;
         float phi, u;
@@ -673,8 +674,7 @@ __global__ void __launch_bounds__(ZP_COLS, zpass_blocks(K)) zpass_adjoint_kernel
                    const AdjFits f = adjoint_fits(c, I, ph, uo, h, ih);
                    *eo = f.eo;
                    *ei = f.ei;
-                   pq[0] = f.p;
-                   pq[nv] = f.q;
+                   *pq = make_float2(f.p, f.q);
                    eo += plane;
                    ei += plane;
                    pq += vplane;
@@ -694,15 +694,14 @@ __global__ void __launch_bounds__(ZP_COLS) zchunk_adjoint_kernel(const SubVolDev
     if (!z.live) return;
     const size_t plane = (size_t)s.W * s.H, n = plane * s.L;
     const size_t v0 = ((size_t)(z.o0 + c.r) * s.H + (z.y + c.r)) * s.W + (z.x + c.r);
-    const size_t nv = (size_t)s.Wv * s.Hv * s.Lv, vplane = (size_t)s.Wv * s.Hv;
-    float *pq = a.xs + (size_t)z.o0 * vplane + (size_t)z.y * s.Wv + z.x;
+    const size_t vplane = (size_t)s.Wv * s.Hv;
+    float2 *pq = reinterpret_cast<float2 *>(a.xs) + (size_t)z.o0 * vplane + (size_t)z.y * s.Wv + z.x;
     zchunk<NB>(s, c, z, [&](int m, float2 h, float2 ih) {
         const size_t v = v0 + (size_t)m * plane;
         const AdjFits f = adjoint_fits(c, load_img(s.img, v, c.img_f32), __ldg(a.phi + v), __ldg(a.u + v), h, ih);
         a.xs[2 * n + v] = f.eo;
         a.xs[3 * n + v] = f.ei;
-        pq[(size_t)m * vplane] = f.p;
-        pq[nv + (size_t)m * vplane] = f.q;
+        pq[(size_t)m * vplane] = make_float2(f.p, f.q);
     });
 }
 
