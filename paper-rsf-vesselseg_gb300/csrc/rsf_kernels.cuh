@@ -80,59 +80,64 @@ __device__ __forceinline__ float load_img(const void *img, size_t i, int f32) {
                : (float)__ldg(static_cast<const unsigned char *>(img) + i);
 }
 
-// Valid correlation of XB consecutive outputs of one packed field pair:
-// src points at the lane's first input, consecutive inputs are two float2
-// apart (the shared slab holds float4 (H, 1-H, I H, I (1-H)) per element).
-// With a run-time tap count the taps go in chunks of XB over a window of 2 XB
-// inputs (which may read up to 2 XB elements past the slab; the slabs are
-// followed by more shared memory, and no tap uses those).
+// Valid correlation of XB consecutive outputs of both field pairs: src points at
+// the lane's first input in the shared slab of float4 (H, 1-H, I H, I (1-H)) per
+// element; one 128-bit load feeds both pairs.  With a run-time tap count the
+// taps go in chunks of XB over a window of 2 XB inputs (which may read up to
+// 2 XB elements past the slab; they lie in the next slab or the padding after the
+// last, and no tap uses them).
 template <int K, int XB>
-__device__ __forceinline__ void xconv_pair(const float2 *src, const StepConst &c, int k, float2 (&acc)[XB]) {
-    const unsigned long long *in = reinterpret_cast<const unsigned long long *>(src);
-    unsigned long long u[XB];
+__device__ __forceinline__ void xconv(const float4 *src, const StepConst &c, int k, unsigned long long (&u)[XB],
+                                      unsigned long long (&v)[XB]) {
+    const ulonglong2 *in = reinterpret_cast<const ulonglong2 *>(src);
     if constexpr (K > 0) {
 #pragma unroll
         for (int q = 0; q < XB + K - 1; ++q) {
-            const unsigned long long v = in[2 * q];
+            const ulonglong2 w = in[q];
 #pragma unroll
             for (int m = 0; m < XB; ++m) {
                 const int tt = q - m;
-                if (tt >= 0 && tt < K) u[m] = fma2(v, c.tap2(tt), tt == 0 ? 0ull : u[m]);
+                if (tt < 0 || tt >= K) continue;
+                u[m] = fma2(w.x, c.tap2(tt), tt == 0 ? 0ull : u[m]);
+                v[m] = fma2(w.y, c.tap2(tt), tt == 0 ? 0ull : v[m]);
             }
         }
     } else {
-        unsigned long long w[2 * XB];
+        // one pair after the other: the window of both at once takes 76
+        // registers instead of 48 and measured 181 against 171 us
+        auto pair = [&](const unsigned long long *in1, unsigned long long (&o)[XB]) {
+            unsigned long long w[2 * XB];
 #pragma unroll
-        for (int m = 0; m < XB; ++m) {
-            u[m] = 0ull;
-            w[m] = in[2 * m];
-        }
-        for (int t0 = 0; t0 < k; t0 += XB) {
-#pragma unroll
-            for (int m = 0; m < XB; ++m) w[XB + m] = in[2 * (t0 + XB + m)];
-#pragma unroll
-            for (int j = 0; j < XB; ++j) {
-                if (t0 + j >= k) break;
-                const unsigned long long g = c.tap2(t0 + j);
-#pragma unroll
-                for (int m = 0; m < XB; ++m) u[m] = fma2(w[m + j], g, u[m]);
+            for (int m = 0; m < XB; ++m) {
+                o[m] = 0ull;
+                w[m] = in1[2 * m];
             }
+            for (int t0 = 0; t0 < k; t0 += XB) {
 #pragma unroll
-            for (int m = 0; m < XB; ++m) w[m] = w[XB + m];
-        }
+                for (int m = 0; m < XB; ++m) w[XB + m] = in1[2 * (t0 + XB + m)];
+#pragma unroll
+                for (int j = 0; j < XB; ++j) {
+                    if (t0 + j >= k) break;
+                    const unsigned long long g = c.tap2(t0 + j);
+#pragma unroll
+                    for (int m = 0; m < XB; ++m) o[m] = fma2(w[m + j], g, o[m]);
+                }
+#pragma unroll
+                for (int m = 0; m < XB; ++m) w[m] = w[XB + m];
+            }
+        };
+        pair(reinterpret_cast<const unsigned long long *>(src), u);
+        pair(reinterpret_cast<const unsigned long long *>(src) + 1, v);
     }
-#pragma unroll
-    for (int m = 0; m < XB; ++m) acc[m] = unpack2(u[m]);
 }
 
 // ---------------------------------------------------------------------------
 // x-pass.  One warp per row segment of 32*XB outputs.  The four fields of
 // the segment's inputs sit in shared memory as float4 (H, 1-H, I H, I (1-H));
-// a lane produces XB consecutive outputs of one packed field pair at a time
-// (XB odd, so the lanes' 64-bit loads fall in distinct banks), the results
-// are staged in shared memory and written as float4 rows.
-// Shared memory: XP_ROWS * span float4 inputs, XP_ROWS * XT float2 of pair-0
-// staging.
+// a lane produces XB consecutive outputs of both pairs (XB odd, so the lanes'
+// 128-bit loads fall in distinct banks).  Besides issue, the kernel is bound by
+// shared-memory wavefronts (73 % of peak at 21 taps).
+// Shared memory: XP_ROWS * span float4 inputs and 2 * XB float4 of padding.
 // ---------------------------------------------------------------------------
 template <int K, int XB, Arith A>
 __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__restrict__ svs,
@@ -155,6 +160,22 @@ __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__
     float4 *in = sm4 + warp * span;
     const int x0 = tx * XT;
     pdl_wait();
+    // The warp's next row into L2: lanes 0 .. 7 its phi lines, 8 and 9 its image
+    // lines.  A row's loads are waited for at once, and from memory they took
+    // most of its time: 5.30 ms per launch on the 48 sub-volumes without this,
+    // 4.68 with it; two rows ahead 4.76.  Float images gained nothing (865
+    // against 888 us on 195 M voxels, 29 taps) and go without.
+    auto prefetch_next = [&](int j, int y, size_t row) {
+        if (c.img_f32 || j + 1 >= c.xrpw || y + XP_ROWS >= s.H) return;
+        const size_t next = row + (size_t)XP_ROWS * s.W;
+        const int xp = x0 + 32 * lane, xi = x0 + 128 * (lane - 8);
+        if (lane < 8) {
+            if (xp < s.W && 32 * lane < span)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"((parity ? s.phi[1] : s.phi[0]) + next + xp));
+        } else if (lane < 10 && xi < s.W) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const unsigned char *>(s.img) + next + xi));
+        }
+    };
     // c.xrpw rows per warp, XP_ROWS apart: the block setup above is paid
     // once per c.xrpw row segments
     for (int j = 0; j < c.xrpw; ++j) {
@@ -163,6 +184,7 @@ __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__
         if (j > 0) __syncwarp();  // the previous row's stores have read the slab
         const size_t row = ((size_t)z * s.H + y) * s.W;
         const float *phi = (parity ? s.phi[1] : s.phi[0]) + row;
+        prefetch_next(j, y, row);
         if constexpr (K > 0) {
             // all of the lane's loads first, so that they are in flight together
             constexpr int NE = ((XT + K - 1 + 31) / 32 + 1) & ~1;
@@ -198,26 +220,19 @@ __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__
             }
         }
         __syncwarp();
-        // Pair 0 (H, 1-H) is staged in its own slab, pair 1 (I H, I (1-H)) in
-        // the input slab once every lane has finished reading it.
-        float2 *s01 = reinterpret_cast<float2 *>(sm4 + XP_ROWS * span) + warp * XT;
-        float2 *s23 = reinterpret_cast<float2 *>(in);
-        const float2 *src = reinterpret_cast<const float2 *>(in + XB * lane);
-        float2 acc[XB];
-        xconv_pair<K, XB>(src, c, k, acc);
-#pragma unroll
-        for (int m = 0; m < XB; ++m) s01[XB * lane + m] = acc[m];
-        xconv_pair<K, XB>(src + 1, c, k, acc);
+        unsigned long long u[XB], v[XB];
+        xconv<K, XB>(in + XB * lane, c, k, u, v);
+        // staged in the slab, once every lane has finished reading it, so that
+        // the rows go out coalesced
         __syncwarp();
 #pragma unroll
-        for (int m = 0; m < XB; ++m) s23[XB * lane + m] = acc[m];
+        for (int m = 0; m < XB; ++m) reinterpret_cast<ulonglong2 *>(in)[XB * lane + m] = make_ulonglong2(u[m], v[m]);
         __syncwarp();
         float4 *dst = reinterpret_cast<float4 *>(s.xb) + ((size_t)z * s.H + y) * s.Wp + x0;
 #pragma unroll
         for (int q = 0; q < XB; ++q) {
             const int e = lane + 32 * q;
-            const float2 a = s01[e], b = s23[e];
-            if (x0 + e < s.Wv) dst[e] = make_float4(a.x, a.y, b.x, b.y);
+            if (x0 + e < s.Wv) dst[e] = in[e];
         }
     }
 }

@@ -13,7 +13,7 @@ namespace rsf {
 
 static size_t xpass_smem(int k, int xb) {
     const int span = 32 * xb + k - 1;
-    return sizeof(float4) * (size_t)XP_ROWS * span + sizeof(float2) * XP_ROWS * 32 * xb;
+    return sizeof(float4) * ((size_t)XP_ROWS * span + 2 * xb);
 }
 
 template <int XB, Arith A>
