@@ -49,6 +49,10 @@ struct rsf_workspace {
     int device = -1;
     int64_t max_voxels = 0;
     int32_t max_subvols = 0;
+    // One device and one pinned allocation hold everything below but pool_g and
+    // the host-buffer staging (a dozen separate ones cost most of creating and
+    // destroying a workspace).
+    void *device_arena = nullptr, *host_arena = nullptr;
     float *pool_phi2 = nullptr;  // second level-set buffer, max_voxels
     float *pool_x = nullptr;     // x-pass fields, 4 * max_voxels
     float *pool_y = nullptr;     // y-pass fields, 4 * max_voxels
@@ -110,6 +114,18 @@ struct rsf_workspace {
 };
 
 namespace {
+// Lays parts out one after the other, each on a 256-byte boundary: without a
+// base for the size, with one for the addresses.
+struct Arena {
+    unsigned char *base = nullptr;
+    size_t used = 0;
+    template <class T>
+    void take(T *&p, size_t count) {
+        if (base) p = reinterpret_cast<T *>(base + used);
+        used = (used + count * sizeof(T) + 255) & ~(size_t)255;
+    }
+};
+
 // The address through which the device reads or writes `ptr`: the pointer
 // itself for device or managed memory, the mapped address for pinned or
 // registered host memory, null for pageable host memory.
@@ -211,23 +227,11 @@ static void ws_free(rsf_workspace *ws) {
     if (ws->device >= 0) cudaSetDevice(ws->device);
     for (cudaEvent_t ev : ws->table_ev)
         if (ev) cudaEventSynchronize(ev);
-    cudaFree(ws->pool_phi2);
-    cudaFree(ws->pool_x);
-    cudaFree(ws->pool_y);
+    cudaFree(ws->device_arena);
     cudaFree(ws->pool_g);
-    cudaFree(ws->d_svs);
-    cudaFree(ws->d_pre);
-    cudaFree(ws->d_maps);
-    cudaFree(ws->d_adj);
-    cudaFree(ws->d_adj_pre);
-    cudaFree(ws->d_flag);
     cudaFree(ws->stage_img);
     cudaFree(ws->stage_phi);
-    cudaFreeHost(ws->h_svs);
-    cudaFreeHost(ws->h_pre);
-    cudaFreeHost(ws->h_maps);
-    cudaFreeHost(ws->h_adj);
-    cudaFreeHost(ws->h_adj_pre);
+    cudaFreeHost(ws->host_arena);
     for (cudaEvent_t ev : ws->table_ev)
         if (ev) cudaEventDestroy(ev);
     for (cudaEvent_t ev : ws->events) cudaEventDestroy(ev);
@@ -250,27 +254,40 @@ rsf_status rsf_workspace_create(int64_t max_voxels, int32_t max_subvols, rsf_wor
     ws->max_voxels = max_voxels;
     ws->max_subvols = max_subvols;
     const size_t v = (size_t)max_voxels;
-    cudaError_t e = cudaSuccess;
-    auto alloc = [&](void **p, size_t bytes) {
-        if (e == cudaSuccess) e = cudaMalloc(p, bytes);
+    if (max_voxels > (int64_t)1 << 48) {
+        delete ws;
+        return fail(RSF_ERR_NO_MEMORY, "workspace allocation failed");
+    }
+    const size_t n = (size_t)max_subvols, n1 = n + 1, ns = rsf_workspace::kStages;
+    auto device_parts = [&](Arena &a) {
+        a.take(ws->pool_phi2, v);
+        a.take(ws->pool_x, 4 * v);
+        a.take(ws->pool_y, 4 * v);
+        a.take(ws->d_svs, n);
+        a.take(ws->d_pre, rsf::NPRE * n1);
+        a.take(ws->d_maps, n * rsf::TMAP_BYTES);
+        a.take(ws->d_adj, n);
+        a.take(ws->d_adj_pre, rsf::NADJ * n1);
+        a.take(ws->d_flag, 64);
     };
-    alloc((void **)&ws->pool_phi2, v * sizeof(float));
-    alloc((void **)&ws->pool_x, 4 * v * sizeof(float));
-    alloc((void **)&ws->pool_y, 4 * v * sizeof(float));
-    alloc((void **)&ws->d_svs, (size_t)max_subvols * sizeof(SubVolDev));
-    alloc((void **)&ws->d_pre, rsf::NPRE * ((size_t)max_subvols + 1) * sizeof(int));
-    alloc((void **)&ws->d_maps, (size_t)max_subvols * rsf::TMAP_BYTES);
-    alloc((void **)&ws->d_adj, (size_t)max_subvols * sizeof(rsf::AdjVol));
-    alloc((void **)&ws->d_adj_pre, rsf::NADJ * ((size_t)max_subvols + 1) * sizeof(int));
-    alloc((void **)&ws->d_flag, 256);
-    const size_t ns = rsf_workspace::kStages;
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&ws->h_svs, ns * (size_t)max_subvols * sizeof(SubVolDev));
-    if (e == cudaSuccess)
-        e = cudaMallocHost((void **)&ws->h_pre, ns * rsf::NPRE * ((size_t)max_subvols + 1) * sizeof(int));
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&ws->h_maps, ns * (size_t)max_subvols * rsf::TMAP_BYTES);
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&ws->h_adj, ns * (size_t)max_subvols * sizeof(rsf::AdjVol));
-    if (e == cudaSuccess)
-        e = cudaMallocHost((void **)&ws->h_adj_pre, ns * rsf::NADJ * ((size_t)max_subvols + 1) * sizeof(int));
+    auto host_parts = [&](Arena &a) {
+        a.take(ws->h_svs, ns * n);
+        a.take(ws->h_pre, ns * rsf::NPRE * n1);
+        a.take(ws->h_maps, ns * n * rsf::TMAP_BYTES);
+        a.take(ws->h_adj, ns * n);
+        a.take(ws->h_adj_pre, ns * rsf::NADJ * n1);
+    };
+    Arena dev, host;
+    device_parts(dev);
+    host_parts(host);
+    cudaError_t e = cudaMalloc(&ws->device_arena, dev.used);
+    if (e == cudaSuccess) e = cudaMallocHost(&ws->host_arena, host.used);
+    if (e == cudaSuccess) {
+        dev = Arena{static_cast<unsigned char *>(ws->device_arena), 0};
+        host = Arena{static_cast<unsigned char *>(ws->host_arena), 0};
+        device_parts(dev);
+        host_parts(host);
+    }
     for (size_t i = 0; i < ns && e == cudaSuccess; i++)
         e = cudaEventCreateWithFlags(&ws->table_ev[i], cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ws->capture_stream, cudaStreamNonBlocking);
