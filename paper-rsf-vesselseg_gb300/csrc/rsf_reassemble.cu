@@ -13,7 +13,7 @@
 //                   blend; the weight of a sub-volume is the product over the
 //                   axes and the output is sum(w phi) / sum(w).  Two volumes
 //                   overlapping along one axis give the reference's blend.
-// One thread per output voxel, x fastest, so reads of each sub-volume row and
+// Neighbouring threads take neighbouring x, so reads of each sub-volume row and
 // the output writes are coalesced; the grid geometry rides in the kernel
 // parameters and the sub-volume table in device memory.
 #include <cuda_runtime.h>
@@ -23,7 +23,7 @@
 namespace rsf {
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 64;  // small, so that ragged rows leave few threads idle
 
 struct ReasmConst {
     int n[3];                        // cells per axis (x, y, z)
@@ -64,14 +64,27 @@ __device__ __forceinline__ float axis_weight(const ReasmConst &c, int a, int ci,
     return w;
 }
 
-__global__ void __launch_bounds__(kThreads) reassemble_kernel(ReasmConst c, const TileDev *tiles, float *out) {
-    const long long N = (long long)c.ext[0] * c.ext[1] * c.ext[2];
-    for (long long i = (long long)blockIdx.x * kThreads + threadIdx.x; i < N; i += (long long)gridDim.x * kThreads) {
-        const int x = (int)(i % c.ext[0]);
-        const long long r = i / c.ext[0];
-        const int y = (int)(r % c.ext[1]);
-        const int z = (int)(r / c.ext[1]);
-        const int ix = cell_of(c, 0, x), iy = cell_of(c, 1, y), iz = cell_of(c, 2, z);
+// A block takes kThreads voxels of one output row after another (grid y strides
+// over the rows), so the y and z cells and weights are found once per row and a
+// voxel is left with its x cells: 190x333x290 voxels of 18 blended tiles took
+// 414 us with a flat index per voxel (three divisions and searches each), 281 so
+// (289 with 256 threads, 311 with four voxels per thread).
+__global__ void __launch_bounds__(kThreads) reassemble_kernel(const __grid_constant__ ReasmConst c,
+                                                              const TileDev *__restrict__ tiles, float *out) {
+    const int x = blockIdx.x * kThreads + threadIdx.x;
+    if (x >= c.ext[0]) return;
+    const long long rows = (long long)c.ext[1] * c.ext[2];
+    const int ix = cell_of(c, 0, x);
+    float wx[3] = {0.0f, 0.0f, 0.0f};
+    if (c.mode != 0) {
+#pragma unroll
+        for (int dx = -1; dx <= 1; dx++)
+            if (ix + dx >= 0 && ix + dx < c.n[0]) wx[dx + 1] = axis_weight(c, 0, ix + dx, x);
+    }
+    for (long long row = blockIdx.y; row < rows; row += gridDim.y) {
+        const int z = (int)(row / c.ext[1]), y = (int)(row - (long long)z * c.ext[1]);
+        const int iy = cell_of(c, 1, y), iz = cell_of(c, 2, z);
+        const long long i = row * c.ext[0] + x;
         if (c.mode == 0) {
             out[i] = tile_at(tiles[((long long)iz * c.n[1] + iy) * c.n[0] + ix], x, y, z);
             continue;
@@ -87,13 +100,11 @@ __global__ void __launch_bounds__(kThreads) reassemble_kernel(ReasmConst c, cons
                 if (cy < 0 || cy >= c.n[1]) continue;
                 const float wy = axis_weight(c, 1, cy, y);
                 if (wy == 0.0f) continue;
+#pragma unroll
                 for (int dx = -1; dx <= 1; dx++) {
-                    const int cx = ix + dx;
-                    if (cx < 0 || cx >= c.n[0]) continue;
-                    const float wx = axis_weight(c, 0, cx, x);
-                    if (wx == 0.0f) continue;
-                    const float w = wz * wy * wx;
-                    acc = fmaf(w, tile_at(tiles[((long long)cz * c.n[1] + cy) * c.n[0] + cx], x, y, z), acc);
+                    if (wx[dx + 1] == 0.0f) continue;
+                    const float w = wz * wy * wx[dx + 1];
+                    acc = fmaf(w, tile_at(tiles[((long long)cz * c.n[1] + cy) * c.n[0] + ix + dx], x, y, z), acc);
                     wsum += w;
                 }
             }
@@ -119,10 +130,10 @@ cudaError_t launch_reassemble(const TileDev *d_tiles, const int n[3], const int 
             c.hi[a][j] = j < n[a] ? hi[a][j] : 0;
         }
     }
-    const long long N = (long long)W * H * L;
-    long long blocks = (N + kThreads - 1) / kThreads;
-    if (blocks > 32LL * sm_count()) blocks = 32LL * sm_count();
-    reassemble_kernel<<<(unsigned)blocks, kThreads, 0, st>>>(c, d_tiles, out);
+    const unsigned ntx = (unsigned)((W + kThreads - 1) / kThreads);
+    const long long rows = (long long)H * L, want = (64LL * sm_count() + ntx - 1) / ntx;
+    const unsigned ny = (unsigned)(rows < want ? rows : want < 65535 ? want : 65535);
+    reassemble_kernel<<<dim3(ntx, ny), kThreads, 0, st>>>(c, d_tiles, out);
     return cudaGetLastError();
 }
 
