@@ -922,7 +922,7 @@ __device__ __forceinline__ float border_data(const unsigned char *ip, const Step
 // and rounded to float.  f(c) comes from the z-pass in the valid region and
 // is 30/30 = 1 in the border band.  Writes the data factor of every voxel;
 // runs on the stencil's tiling (lanes 1..30 x warps 1..14 x c.zc planes), a
-// grid row per BOX_Z of the planes.
+// grid row per BOX_Z of the planes or fewer.
 //
 // Double precision is what bounds the sum in its own terms (four operations
 // and six conversions per neighbour on a pipe with 1/64 of the FP32 rate), so
@@ -962,7 +962,8 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 2) box_kernel(const SubVolDev *
     const int tz = t / nty;
     const int x = tx * ST_OX - 1 + lane, y = ty * ST_OY - 1 + w;
     if (lane < 1 || lane > ST_OX || w < 1 || w > ST_OY || x >= s.W || y >= s.H) return;
-    const int z0 = tz * c.zc + (int)blockIdx.y * BOX_Z, z1 = min(min(z0 + BOX_Z, tz * c.zc + c.zc), s.L);
+    const int zb = (c.zc + (int)gridDim.y - 1) / (int)gridDim.y;  // planes per grid row
+    const int z0 = tz * c.zc + (int)blockIdx.y * zb, z1 = min(min(z0 + zb, tz * c.zc + c.zc), s.L);
     const int bs = c.box, r = c.r;
     const double wt = 1.0 / (double)((2 * bs + 1) * (2 * bs + 1));
     const float2 wh = dup2((float)wt), wl = dup2((float)(wt - (double)(float)wt));

@@ -62,14 +62,16 @@ int choose_xb(const int *Wv, int n) {
 // planes one after another, each behind a barrier, so a small volume wants many
 // shallow ones.  The candidate with the lowest modelled time is taken.  A block
 // takes its planes, the two before them and about three of set-up as steps; a
-// step costs 0.45 (us) of an SM's issue per block sharing it and at least the
-// 0.9 of its own latency chain, and the last wave is three quarters empty.
+// step is mostly latency: measured 1.09 us with two blocks on an SM (128^3) and
+// 1.18 with three (320^3), so 0.9 + 0.095 per block; beyond three blocks the
+// waves follow one another and the last one costs a quarter of a block's steps
+// (three quarters made it prefer shallow blocks: 248 against 209 us on 18 tiles of
+// 150x263x333).
 int choose_zc(const int *whl, int n) {
-    const double issue = 0.45, chain = 0.9;
     const int sms = sm_count(), setup = 5;
     int best = ST_ZC_MAX;
     double best_t = -1.0;
-    for (int zc : {ST_ZC_MAX, 96, ST_ZC, 48, ST_ZC / 2, 24, 16, 12, 8, 6, 4}) {
+    for (int zc : {ST_ZC_MAX, 96, ST_ZC, 48, ST_ZC / 2, 24, 20, 16, 14, 12, 10, 8, 6, 5, 4, 3, 2}) {
         long long blocks = 0;
         double steps = 0.0;
         int deepest = 0;
@@ -80,13 +82,10 @@ int choose_zc(const int *whl, int n) {
             steps += (double)cols * (L + setup * chunks);
             if (L < zc ? L > deepest : zc > deepest) deepest = L < zc ? L : zc;
         }
-        double t = 0.0;
-        if (blocks <= 3LL * sms) {
-            const double step = issue * (double)((blocks + sms - 1) / sms);
-            t = (deepest + setup) * (step > chain ? step : chain);
-        } else {
-            t = issue * (steps / sms + 0.75 * (deepest + setup));
-        }
+        const double per = blocks <= 3LL * sms ? (double)((blocks + sms - 1) / sms) : 3.0;
+        double rounds = deepest + setup;
+        if (blocks > 3LL * sms) rounds = steps / (3.0 * sms) + 0.25 * (deepest + setup);
+        const double t = rounds * (0.9 + 0.095 * per);
         if (best_t < 0.0 || t < best_t) {
             best_t = t;
             best = zc;
