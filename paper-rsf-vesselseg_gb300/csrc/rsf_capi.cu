@@ -472,6 +472,7 @@ StepConst make_const(const rsf_params *p, int k, const float *taps, rsf_dtype dt
     c.nsv = n;
     c.xb_w = sh.xb_w;
     c.xrpw = sh.xrpw;
+    c.yout = sh.yout;
     c.zout = sh.zout;
     c.zc = sh.zc;
     c.ymaps = sh.zt ? maps : nullptr;

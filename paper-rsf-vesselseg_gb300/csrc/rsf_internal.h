@@ -72,6 +72,7 @@ struct StepConst {
     int nsv;        // number of sub-volumes in the table
     int xb_w;       // x-pass outputs per lane for this launch
     int xrpw;       // x-pass rows per warp for this launch
+    int yout;       // y-pass outputs per block for this launch (specialised tap counts)
     int zout;       // z-pass output planes per block for this launch
     int zc;         // stencil planes per block for this launch
     int box;        // e-term box radius (int)sigma2; 0: e = (I - f)^2
@@ -128,6 +129,7 @@ constexpr int BOX_Z = 8;    // most planes per block of the box e-term
 struct LaunchShape {
     int xb_w;   // x-pass outputs per lane
     int xrpw;   // x-pass rows per warp (1, 2, 4 or XP_RPW)
+    int yout;   // y-pass outputs per block (specialised tap counts)
     int zout;   // z-pass output planes per block
     int zt;     // 1: the z-pass loads planes with TMA (needs a map per sub-volume)
     int zc;     // stencil planes per block

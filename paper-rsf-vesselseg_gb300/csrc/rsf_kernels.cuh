@@ -334,7 +334,7 @@ __device__ __forceinline__ void conv_block_rt(const float *__restrict__ base, si
 // ---------------------------------------------------------------------------
 // y-pass.  One thread streams one column of one pair (every other float2 of
 // the interleaved fields): the 2 Wp float2 columns of a z plane, over all
-// planes, are numbered consecutively.
+// planes, are numbered consecutively, and each is cut into c.yout outputs.
 // ---------------------------------------------------------------------------
 template <int K>
 __global__ void __launch_bounds__(YP_COLS) ypass_kernel(const SubVolDev *__restrict__ svs,
@@ -343,18 +343,20 @@ __global__ void __launch_bounds__(YP_COLS) ypass_kernel(const SubVolDev *__restr
     const int b = blockIdx.x;
     const int sv = find_sv(pre, c.nsv, b);
     const SubVolDev s = svs[sv];
-    pdl_wait();
-    const long long q = (long long)(b - __ldg(pre + sv)) * YP_COLS + threadIdx.x;
-    const int row = 2 * s.Wp;
+    const int row = 2 * s.Wp, t = b - __ldg(pre + sv);
+    const int ntq = (int)(((long long)row * s.L + YP_COLS - 1) / YP_COLS);
+    const long long q = (long long)(t % ntq) * YP_COLS + threadIdx.x;
+    const int y0 = (t / ntq) * c.yout;
     const int z = (int)(q / row), x = (int)(q - (long long)z * row);
     __shared__ float2 ring[RING * YP_COLS];
+    pdl_wait();
     if (z >= s.L || x >= 2 * s.Wv) return;
-    const float *src = s.xb + 2 * ((size_t)z * s.H * row + x);
-    float2 *dst = reinterpret_cast<float2 *>(s.yb) + (size_t)z * s.Hv * row + x;
+    const float *src = s.xb + 2 * (((size_t)z * s.H + y0) * row + x);
+    float2 *dst = reinterpret_cast<float2 *>(s.yb) + ((size_t)z * s.Hv + y0) * row + x;
     // The y-pass is bound by HBM bandwidth: it keeps the deeper 8-slot ring
     // (more loads in flight) rather than the compile-time-slot ring.
     auto emit = [&](int o, float2 v, int) { dst[(size_t)o * row] = v; };
-    const Ring rg = {ring + threadIdx.x, YP_COLS, src, 2 * (size_t)row, s.H, true};
+    const Ring rg = {ring + threadIdx.x, YP_COLS, src, 2 * (size_t)row, min(c.yout, s.Hv - y0) + K - 1, true};
     stream_axis<K>(rg, c, emit);
     pdl_launch();
 }

@@ -163,6 +163,7 @@ extern "C" rsf_status rsf_evolve_noalloc(const rsf_params *p, const void *image,
     c.nsv = 1;
     c.xb_w = sh.xb_w;
     c.xrpw = sh.xrpw;
+    c.yout = sh.yout;
     c.zout = sh.zout;
     c.zc = sh.zc;
     rsf::set_pair_const(c.pk, c.eps, c.dt, c.nu, c.mu);

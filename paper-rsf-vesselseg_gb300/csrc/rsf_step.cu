@@ -112,24 +112,23 @@ int choose_xrpw(const int *whl, int n, int k, int xb_w) {
     return rpw;
 }
 
-// Output planes per z-pass block.  A block streams its outputs and the K - 1
-// planes before them, so cutting a column costs K - 1 steps per cut and pays
-// only where the batch leaves the SMs short of warps: the fewest cuts that give
-// every SM its resident blocks, as long as a cut is no shorter than the taps.
-int choose_zout(const int *whl, int n, int k) {
-    const long long want = (long long)zpass_blocks(k) * sm_count();
-    int deepest = 1;
-    for (int i = 0; i < n; i++) deepest = whl[3 * i + 2] > deepest ? whl[3 * i + 2] : deepest;
+// Outputs along a streamed axis per y- or z-pass block.  A block streams its
+// outputs and the k - 1 inputs before them, so cutting a column costs k - 1 steps
+// per cut and pays only where the batch leaves the SMs short of warps: the
+// fewest cuts that give `want` blocks, as long as a cut is no shorter than the
+// taps.  cols(i): a volume's columns of one block each; ext(i): its extent along
+// the axis.
+template <class Cols, class Ext>
+static int choose_cut(int n, int k, long long want, Cols cols, Ext ext) {
+    int deepest = 0;
+    for (int i = 0; i < n; i++) deepest = ext(i) - k + 1 > deepest ? ext(i) - k + 1 : deepest;
+    if (deepest < 1) return 1;
     for (int cuts = 1;; cuts++) {
-        const int zout = (deepest - k + cuts) / cuts;
+        const int out = (deepest + cuts - 1) / cuts;
         long long blocks = 0;
-        for (int i = 0; i < n; i++) {
-            int Wv, Hv, Lv, Wp;
-            valid_extents(whl[3 * i], whl[3 * i + 1], whl[3 * i + 2], k, Wv, Hv, Lv, Wp);
-            if (Wv > 0) blocks += (((long long)Wp * Hv + ZP_COLS - 1) / ZP_COLS) * ((Lv + zout - 1) / (zout > 0 ? zout : 1));
-        }
-        if (zout < 1) return 1;
-        if (blocks >= want || (deepest - k + cuts + 1) / (cuts + 1) < k) return zout;
+        for (int i = 0; i < n; i++)
+            if (cols(i) > 0) blocks += cols(i) * ((ext(i) - k + out) / out);
+        if (blocks >= want || (deepest + cuts) / (cuts + 1) < k) return out;
     }
 }
 
@@ -145,7 +144,26 @@ LaunchShape choose_shape(const int *whl, int n, int k, int kspec, int gauss) {
     sh.xrpw = choose_xrpw(whl, n, k, sh.xb_w);
     sh.zt = tma_z(kspec) && tma_z_requested() && tensor_maps_available() ? 1 : 0;
     sh.zc = choose_zc(whl, n);
-    sh.zout = kspec > 0 ? choose_zout(whl, n, k) : ZG_NB;
+    sh.yout = YG_NB;
+    sh.zout = ZG_NB;
+    if (kspec > 0) {
+        auto valid = [&](int i, int e[4]) {
+            valid_extents(whl[3 * i], whl[3 * i + 1], whl[3 * i + 2], k, e[0], e[1], e[2], e[3]);
+            return e[0] > 0;
+        };
+        int e[4];
+        // y: three blocks per SM (61x187x203, 35 taps: 4.10 -> 3.75 ms per 30
+        // iterations; with six, 21 taps lose 8 % on 4 x 96x112x96); z: its
+        // resident ones
+        sh.yout = choose_cut(
+            n, k, 3LL * sm_count(),
+            [&](int i) { return valid(i, e) ? (2LL * e[3] * whl[3 * i + 2] + YP_COLS - 1) / YP_COLS : 0LL; },
+            [&](int i) { return whl[3 * i + 1]; });
+        sh.zout = choose_cut(
+            n, k, (long long)zpass_blocks(k) * sm_count(),
+            [&](int i) { return valid(i, e) ? ((long long)e[3] * e[1] + ZP_COLS - 1) / ZP_COLS : 0LL; },
+            [&](int i) { return whl[3 * i + 2]; });
+    }
     sh.gauss = gauss;
     return sh;
 }
@@ -205,7 +223,7 @@ void tile_counts(const SubVolDev &d, int kspec, const LaunchShape &sh, int tiles
     tiles[0] = valid ? ((d.Wv + xt - 1) / xt) * ((d.H + xr - 1) / xr) * d.L : 0;
     if (!valid) tiles[1] = 0;
     else tiles[1] = (int)((2LL * d.Wp * d.L + YP_COLS - 1) / YP_COLS);  // one column of one pair per thread
-    if (kspec == 0) tiles[1] *= (d.Hv + YG_NB - 1) / YG_NB;
+    if (valid) tiles[1] *= (d.Hv + sh.yout - 1) / sh.yout;
     if (!valid) tiles[2] = 0;
     else if (sh.zt) tiles[2] = ((d.Wv + ZT_X - 1) / ZT_X) * ((d.Hv + ZT_Y - 1) / ZT_Y);
     else tiles[2] = (int)(((long long)d.Wp * d.Hv + ZP_COLS - 1) / ZP_COLS) * ((d.Lv + sh.zout - 1) / sh.zout);
