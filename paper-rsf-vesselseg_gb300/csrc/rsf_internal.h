@@ -123,7 +123,7 @@ inline int kernel_k(int k, int arith, bool debug, int box = 0, int gauss = 0) {
 // ring depth divides k).
 inline bool tma_z(int kspec) { return kspec == 21 || kspec == 35; }
 constexpr int MAX_BOX = 8;  // largest e-term box radius
-constexpr int BOX_Z = 8;    // most planes per block of the box e-term
+constexpr int BOX_Z = 3;    // most planes per block of the box e-term
 
 // Per-launch tile shapes of a batch.
 struct LaunchShape {
