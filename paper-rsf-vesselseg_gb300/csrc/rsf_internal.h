@@ -219,7 +219,7 @@ cudaError_t config_ztpass_35();
 cudaError_t launch_ztpass_21(const SubVolDev *, const int *, int, const StepConst &, unsigned *flag, cudaStream_t);
 cudaError_t launch_ztpass_35(const SubVolDev *, const int *, int, const StepConst &, unsigned *flag, cudaStream_t);
 cudaError_t launch_stencil(const SubVolDev *, const int *, int, const StepConst &, int parity, int arith,
-                           unsigned *flag, const DebugOut *dbg, cudaStream_t);
+                           bool dependent, unsigned *flag, const DebugOut *dbg, cudaStream_t);
 // Expanded data term (c.gauss): its four kernels after the z-pass; pre holds
 // NPRE prefix arrays of n1 entries, tot their totals.
 cudaError_t launch_gauss(const SubVolDev *, const int *pre, int n1, const int *tot, const StepConst &,

@@ -4,14 +4,14 @@
 namespace rsf {
 
 cudaError_t launch_stencil(const SubVolDev *svs, const int *pre, int blocks, const StepConst &c, int parity,
-                           int arith, unsigned *flag, const DebugOut *dbg, cudaStream_t st) {
+                           int arith, bool dependent, unsigned *flag, const DebugOut *dbg, cudaStream_t st) {
     if (dbg) {
         constexpr int T = ST_WARPS * 32;
         if (arith == 1) stencil_debug_kernel<Arith::Reference><<<blocks, T, 0, st>>>(svs, pre, c, parity, flag, *dbg);
         else stencil_debug_kernel<Arith::Portable><<<blocks, T, 0, st>>>(svs, pre, c, parity, flag, *dbg);
     } else {
         constexpr int T = SP_WARPS * 32;
-        return launch_dependent(true, arith == 1 ? stencil_pair_kernel<Arith::Reference> : stencil_pair_kernel<Arith::Portable>,
+        return launch_dependent(dependent, arith == 1 ? stencil_pair_kernel<Arith::Reference> : stencil_pair_kernel<Arith::Portable>,
                                 (unsigned)blocks, T, 0, st, svs, pre, c, parity, flag);
     }
     return cudaGetLastError();

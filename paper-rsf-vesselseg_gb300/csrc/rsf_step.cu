@@ -330,7 +330,8 @@ cudaError_t launch_step(const SubVolDev *svs, const int *pre, const int *tot, co
         if (e != cudaSuccess) return e;
     }
     if ((e = mark(3)) != cudaSuccess) return e;
-    if (tot[3] > 0) e = launch_stencil(svs, pre + 3 * n1, tot[3], c, parity, arith, flag, dbg, st);
+    // (the stencil is the first kernel where no volume has a valid region)
+    if (tot[3] > 0) e = launch_stencil(svs, pre + 3 * n1, tot[3], c, parity, arith, !(first && tot[0] == 0), flag, dbg, st);
     if (e == cudaSuccess) e = mark(4);
     return e;
 }
