@@ -18,10 +18,13 @@
 //
 // Summation order is the reference's: each blurred value is accumulated with
 // fused multiply-adds from +0 over ascending taps, x first, then y, then z.
-// The y and z correlations stream along their axis with K rotating
-// accumulators per column (the accumulator of output o is slot o mod K), so
-// every input is loaded once; two adjacent columns share one thread and one
-// packed f32x2 multiply-add, which rounds each lane exactly like fmaf.
+// Two values share one packed f32x2 multiply-add, which rounds each lane exactly
+// like fmaf.  The fields lie interleaved, a float4 per voxel.  The y and z
+// correlations stream along their axis with K rotating accumulators per column
+// (the accumulator of output o is slot o mod K), so every input is loaded once:
+// a y-pass thread owns one pair of fields of a column, a z-pass thread all four
+// (its fits and data factor then need no exchange).  Tap counts that are not
+// compiled in run in chunks over a register window.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -908,14 +911,6 @@ __device__ __forceinline__ void stencil_step(const StencilCtx &k, const StepCons
     S.DT[C1] = dn;  // plane rel+1
 }
 
-// Border-band data factor (f_out = f_in = 30/30 = 1) from the image at ip.
-__device__ __forceinline__ float border_data(const unsigned char *ip, const StepConst &c) {
-    const float I = c.img_f32 ? __ldg(reinterpret_cast<const float *>(ip)) : (float)__ldg(ip);
-    const float d = __fsub_rn(I, 1.0f);
-    const float e = __fmul_rn(d, d);
-    return data_factor(e, e, c.l1, c.l2, c.lam_equal != 0);
-}
-
 // ---------------------------------------------------------------------------
 // Box e-term, CUDA_RSF/kernel.cu:25-55 with s = (int)sigma2 >= 1: for every
 // voxel c, e = sum over the neighbours n of the (2s+1)^3 box that lie inside
@@ -934,7 +929,7 @@ __device__ __forceinline__ float border_data(const unsigned char *ip, const Step
 // double sequence is within 2^-52; where the two ends of a 2^-43 margin round
 // to the same float, that float is the reference's.  Elsewhere (one term in
 // 2^18) the z column is redone in double.  72x100x131 voxels, s = 1: 809 us per
-// launch in double, BOX_MEASURED so.
+// launch in double, 60 so (67 with a grid row per plane).
 // ---------------------------------------------------------------------------
 // One z column of the box in double, from the sums before it.
 static __device__ __noinline__ float2 box_column_double(const void *img, size_t i, size_t step, int n, int f32,
