@@ -557,7 +557,7 @@ rsf_status timing_events(rsf_workspace *ws, int iters, const int tot[rsf::NKERN]
 }
 
 rsf_status run(rsf_workspace *ws, const rsf_params *p, rsf_dtype dtype, const rsf_subvol *svs, int32_t n,
-               int32_t iters, cudaStream_t st, bool use_graph) {
+               int32_t iters, cudaStream_t st, bool batched) {
     if (!ws) return fail(RSF_ERR_INVALID_ARGUMENT, "workspace is null");
     if (iters < 0) return fail(RSF_ERR_INVALID_ARGUMENT, "iters must be >= 0");
     float taps[rsf::MAXK];
@@ -582,7 +582,14 @@ rsf_status run(rsf_workspace *ws, const rsf_params *p, rsf_dtype dtype, const rs
         return rsf::launch_step(ws->d_svs, ws->d_pre, tot, c, it & 1, p->arith, it == 0, ws->d_flag, nullptr, on, ev);
     };
     cudaError_t e = cudaSuccess;
-    if (!use_graph) {
+    if (batched && iters < kGraphFrom) {
+        // a graph launch is refused on a capturing stream: so are the launches in its place
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        e = cudaStreamIsCapturing(st, &cap);
+        if (e == cudaSuccess && cap != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
+        if (e != cudaSuccess) return cuda_fail(e, "graph");
+    }
+    if (!batched || iters < kGraphFrom) {
         for (int it = 0; it < iters && e == cudaSuccess; it++) e = step(it, st);
         if (e != cudaSuccess) return cuda_fail(e, "step launch");
     } else {
@@ -633,7 +640,7 @@ rsf_status rsf_evolve(rsf_workspace *ws, const rsf_params *p, const void *image,
 rsf_status rsf_evolve_batched(rsf_workspace *ws, const rsf_params *p, rsf_dtype dtype, const rsf_subvol *subvols,
                               int32_t n, int32_t iters, void *stream) {
     if (!subvols) return fail(RSF_ERR_INVALID_ARGUMENT, "subvols is null");
-    return run(ws, p, dtype, subvols, n, iters, (cudaStream_t)stream, iters >= kGraphFrom);
+    return run(ws, p, dtype, subvols, n, iters, (cudaStream_t)stream, true);
 }
 
 rsf_status rsf_evolve_host(rsf_workspace *ws, const rsf_params *p, const void *image_host, rsf_dtype dtype,

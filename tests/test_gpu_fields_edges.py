@@ -2,6 +2,10 @@
 at the edges of their tiles: valid regions of one voxel and of ragged rows,
 columns cut along z, and images at the ends of the packed quotient's range.
 Bit for bit against the oracle (a NaN's payload is the platform's own)."""
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -88,3 +92,30 @@ def test_box_term_in_float_pairs(sigma2, kind, orc, cuda, rsflib):
         got = t.cpu().numpy()
     same = (got.view(np.uint32) == want.view(np.uint32)) | (np.isnan(got) & np.isnan(want))
     assert same.all(), f"{int((~same).sum())} voxels differ"
+
+
+@pytest.mark.parametrize("iters", [2, 5])
+def test_batched_is_refused_on_a_capturing_stream(iters, cuda, rsflib):
+    """With and without a graph of its own (a refused capture spoils the process's next call: a child process)."""
+    code = f"""
+import os, torch
+from rsf_gb300 import Params, RsfError, Workspace
+img, phi = torch.zeros((24, 24, 24), dtype=torch.uint8, device="cuda"), torch.randn((24, 24, 24), device="cuda")
+ws = Workspace(phi.numel())
+ws.evolve_batched([(img, phi)], Params(sigma=1.0), {iters})
+torch.cuda.synchronize()
+answer = "accepted"
+try:
+    with torch.cuda.graph(torch.cuda.CUDAGraph()):
+        try:
+            ws.evolve_batched([(img, phi)], Params(sigma=1.0), {iters})
+        except RsfError:
+            answer = "refused"
+except RuntimeError:
+    pass
+print(answer, flush=True)
+os._exit(0)
+"""
+    pkg = Path(__file__).resolve().parent.parent / "paper-rsf-vesselseg_gb300"
+    r = subprocess.run([sys.executable, "-c", code], cwd=str(pkg), capture_output=True, text=True, timeout=300)
+    assert r.stdout.split() == ["refused"], r.stdout + r.stderr
