@@ -838,18 +838,24 @@ rsf_status rsf_step_adjoint_batched(rsf_workspace *ws, const rsf_params *p, rsf_
         const int *pre = ws->d_pre;
         const int f1 = n + 1;
         if (ftot[0] > 0) switch (kspec) {
+                case 11: e = rsf::launch_xpass_11(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, false, st); break;
+                case 15: e = rsf::launch_xpass_15(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, false, st); break;
                 case 21: e = rsf::launch_xpass_21(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, false, st); break;
                 case 29: e = rsf::launch_xpass_29(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, false, st); break;
                 case 35: e = rsf::launch_xpass_35(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, false, st); break;
                 default: e = rsf::launch_xpass_0(svs, pre, ftot[0], c, 0, RSF_ARITH_PORTABLE, false, st); break;
             }
         if (e == cudaSuccess && ftot[1] > 0) switch (kspec) {
+                case 11: e = rsf::launch_ypass_11(svs, pre + f1, ftot[1], c, st); break;
+                case 15: e = rsf::launch_ypass_15(svs, pre + f1, ftot[1], c, st); break;
                 case 21: e = rsf::launch_ypass_21(svs, pre + f1, ftot[1], c, st); break;
                 case 29: e = rsf::launch_ypass_29(svs, pre + f1, ftot[1], c, st); break;
                 case 35: e = rsf::launch_ypass_35(svs, pre + f1, ftot[1], c, st); break;
                 default: e = rsf::launch_ypass_0(svs, pre + f1, ftot[1], c, st); break;
             }
         if (e == cudaSuccess && ftot[2] > 0) switch (kspec) {
+                case 11: e = rsf::launch_zpass_adjoint_11(svs, pre + 2 * f1, ftot[2], c, ws->d_adj, st); break;
+                case 15: e = rsf::launch_zpass_adjoint_15(svs, pre + 2 * f1, ftot[2], c, ws->d_adj, st); break;
                 case 21: e = rsf::launch_zpass_adjoint_21(svs, pre + 2 * f1, ftot[2], c, ws->d_adj, st); break;
                 case 29: e = rsf::launch_zpass_adjoint_29(svs, pre + 2 * f1, ftot[2], c, ws->d_adj, st); break;
                 case 35: e = rsf::launch_zpass_adjoint_35(svs, pre + 2 * f1, ftot[2], c, ws->d_adj, st); break;

@@ -20,7 +20,8 @@ constexpr int ZP_COLS = 128;   // z-pass: columns per block
 // z-pass: resident blocks per SM that its 4 K accumulator registers leave room
 // for (21 taps: 3.70 ms per launch on the 48-sub-volume batch with 4, 4.17 with
 // 3; 29 and 35 taps spill with 3: 771 against 1061 us on a 195 M voxel batch,
-// 1.02 against 1.45 ms on 512^3)
+// 1.02 against 1.45 ms on 512^3; 11 and 15 taps spill with 5, 3345 against 3313 us
+// on a batch of 15 taps)
 constexpr int zpass_blocks(int K) { return K <= 21 ? 4 : 2; }
 constexpr int YG_NB = 16;      // run-time-k y-pass: outputs per thread
 constexpr int ZG_NB = 8;       // run-time-k z-pass: outputs per thread
@@ -112,10 +113,13 @@ constexpr unsigned kFlagNonFinite = 1u;  // a non-finite value was written to ph
 constexpr unsigned kFlagTimeout = 2u;    // a barrier wait gave up (a TMA copy did not complete)
 constexpr unsigned kFlagAdjointNonFinite = 4u;  // rsf_step_adjoint produced a non-finite dL/dphi
 
-// Tap counts with streaming (compile-time K) kernels.  Other tap counts, the
-// debug step, the reference arithmetic and the box e-term use the
-// run-time-k kernels.
-inline bool is_specialised(int k) { return k == 21 || k == 29 || k == 35; }
+// Tap counts with streaming (compile-time K) kernels: sigma 1.5, 2, 3, 4 and 5.
+// They load each input once and keep K accumulators, where the run-time-k kernels
+// run over a window per chunk of outputs: 256^3 voxels take 397 against 550 us per
+// iteration with 11 taps, 405 against 550 with 15; at 64^3 (25 us, latency) the two
+// are level.  Other tap counts, the debug step, the reference arithmetic and
+// the box e-term use the run-time-k kernels.
+inline bool is_specialised(int k) { return k == 11 || k == 15 || k == 21 || k == 29 || k == 35; }
 inline int kernel_k(int k, int arith, bool debug, int box = 0, int gauss = 0) {
     return (is_specialised(k) && arith == 0 && !debug && box == 0 && gauss == 0) ? k : 0;
 }
@@ -197,6 +201,8 @@ void adjoint_tiles(const AdjVol &v, int tiles[NADJ]);
                                  cudaStream_t);                                                                \
     cudaError_t config_zpass_##K();
 RSF_DECLARE_K(0)
+RSF_DECLARE_K(11)
+RSF_DECLARE_K(15)
 RSF_DECLARE_K(21)
 RSF_DECLARE_K(29)
 RSF_DECLARE_K(35)
@@ -205,6 +211,12 @@ RSF_DECLARE_K(35)
 // sub-volume i of the table is volume i of `vols`.
 cudaError_t launch_zpass_adjoint_0(const SubVolDev *, const int *, int, const StepConst &, const AdjVol *vols,
                                    cudaStream_t);
+cudaError_t config_zpass_adjoint_11();
+cudaError_t launch_zpass_adjoint_11(const SubVolDev *, const int *, int, const StepConst &, const AdjVol *vols,
+                                    cudaStream_t);
+cudaError_t config_zpass_adjoint_15();
+cudaError_t launch_zpass_adjoint_15(const SubVolDev *, const int *, int, const StepConst &, const AdjVol *vols,
+                                    cudaStream_t);
 cudaError_t config_zpass_adjoint_21();
 cudaError_t launch_zpass_adjoint_21(const SubVolDev *, const int *, int, const StepConst &, const AdjVol *vols,
                                     cudaStream_t);

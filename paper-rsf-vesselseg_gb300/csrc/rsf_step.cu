@@ -240,9 +240,13 @@ void tile_counts(const SubVolDev &d, int kspec, const LaunchShape &sh, int tiles
 // current device; called once per workspace, outside any stream capture.
 cudaError_t configure_device() {
     cudaError_t e = config_xpass_0();
+    if (e == cudaSuccess) e = config_xpass_11();
+    if (e == cudaSuccess) e = config_xpass_15();
     if (e == cudaSuccess) e = config_xpass_21();
     if (e == cudaSuccess) e = config_xpass_29();
     if (e == cudaSuccess) e = config_xpass_35();
+    if (e == cudaSuccess) e = config_zpass_11();
+    if (e == cudaSuccess) e = config_zpass_15();
     if (e == cudaSuccess) e = config_zpass_21();
     if (e == cudaSuccess) e = config_zpass_29();
     if (e == cudaSuccess) e = config_zpass_35();
@@ -290,6 +294,8 @@ cudaError_t launch_step(const SubVolDev *svs, const int *pre, const int *tot, co
     if ((e = mark(0)) != cudaSuccess) return e;
     if (tot[0] > 0) {
         switch (kspec) {
+            case 11: e = launch_xpass_11(svs, pre, tot[0], c, parity, arith, !first, st); break;
+            case 15: e = launch_xpass_15(svs, pre, tot[0], c, parity, arith, !first, st); break;
             case 21: e = launch_xpass_21(svs, pre, tot[0], c, parity, arith, !first, st); break;
             case 29: e = launch_xpass_29(svs, pre, tot[0], c, parity, arith, !first, st); break;
             case 35: e = launch_xpass_35(svs, pre, tot[0], c, parity, arith, !first, st); break;
@@ -300,6 +306,8 @@ cudaError_t launch_step(const SubVolDev *svs, const int *pre, const int *tot, co
     if ((e = mark(1)) != cudaSuccess) return e;
     if (tot[1] > 0) {
         switch (kspec) {
+            case 11: e = launch_ypass_11(svs, pre + n1, tot[1], c, st); break;
+            case 15: e = launch_ypass_15(svs, pre + n1, tot[1], c, st); break;
             case 21: e = launch_ypass_21(svs, pre + n1, tot[1], c, st); break;
             case 29: e = launch_ypass_29(svs, pre + n1, tot[1], c, st); break;
             case 35: e = launch_ypass_35(svs, pre + n1, tot[1], c, st); break;
@@ -314,6 +322,8 @@ cudaError_t launch_step(const SubVolDev *svs, const int *pre, const int *tot, co
         if (e != cudaSuccess) return e;
     } else if (tot[2] > 0) {
         switch (kspec) {
+            case 11: e = launch_zpass_11(svs, pre + 2 * n1, tot[2], c, dbg, st); break;
+            case 15: e = launch_zpass_15(svs, pre + 2 * n1, tot[2], c, dbg, st); break;
             case 21: e = launch_zpass_21(svs, pre + 2 * n1, tot[2], c, dbg, st); break;
             case 29: e = launch_zpass_29(svs, pre + 2 * n1, tot[2], c, dbg, st); break;
             case 35: e = launch_zpass_35(svs, pre + 2 * n1, tot[2], c, dbg, st); break;

@@ -119,3 +119,32 @@ os._exit(0)
     pkg = Path(__file__).resolve().parent.parent / "paper-rsf-vesselseg_gb300"
     r = subprocess.run([sys.executable, "-c", code], cwd=str(pkg), capture_output=True, text=True, timeout=300)
     assert r.stdout.split() == ["refused"], r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("sigma,k", [(1.5, 11), (2.0, 15)])
+@pytest.mark.parametrize("extra", [(0, 0, 0), (1, 2, 3), (2, 0, 40), (75, 3, 9), (130, 1, 1), (14, 15, 150)])
+def test_valid_region_edges_of_short_taps(sigma, k, extra, orc, cuda, rsflib):
+    """The compiled tap counts below 21, as test_valid_region_edges."""
+    assert len(orc.taps(sigma)) == k
+    test_valid_region_edges(sigma, k, extra, orc, cuda, rsflib)
+
+
+@pytest.mark.parametrize("shape", [(15, 15, 15), (16, 18, 20), (34, 31, 45)])
+def test_step_adjoint_of_15_taps(shape, orc, cuda, rsflib):
+    """Against float64 autograd, at the tolerance of the other tap counts (test_gpu_adjoint.py)."""
+    from test_adjoint_ref_cpu import smooth_case
+    from test_gpu_adjoint import _params, _rel, _vjp_fp64
+    from rsf_gb300 import Workspace
+
+    img, phi, _ = smooth_case(shape)
+    p = _params(sigma=2.0, lambda2=0.7)
+    u = np.random.default_rng(sum(shape)).standard_normal(shape).astype(np.float32)
+    g = torch.zeros(4, dtype=torch.float64, device="cuda")
+    with Workspace(phi.size) as ws:
+        got = ws.step_adjoint(torch.from_numpy(img).cuda(), torch.from_numpy(phi).cuda(), torch.from_numpy(u).cuda(), p,
+                              param_grads=g).cpu().numpy()
+    want, want_p = _vjp_fp64(orc, phi, img, u, p, "reference")
+    assert _rel(got, want) <= 1e-4
+    gp = g.cpu().numpy()
+    for k in range(4):
+        assert abs(gp[k] - want_p[k]) <= 1e-4 * max(abs(want_p[k]), 1e-3 * np.abs(want_p).max()), k
