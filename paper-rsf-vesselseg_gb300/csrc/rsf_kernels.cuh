@@ -56,7 +56,10 @@ __device__ __forceinline__ int find_sv(const int *__restrict__ pre, int n, int b
 // Every thread of every block waits, also those without work: a grid that
 // finished before its predecessor would let its own successor through.  The
 // first kernel after a table upload is launched the ordinary way: its tables'
-// writes are only visible behind a full dependency.  (The x-pass lets its
+// writes are only visible behind a full dependency.  What a kernel of the chain
+// writes (level set, blurred fields, data factor) is read with ordinary loads or
+// cp.async: __ldg wants memory that nothing writes while the reading kernel is
+// resident, which holds for the image and the tables alone.  (The x-pass lets its
 // dependents go by ending: an explicit call after its row loop takes it from 56
 // to 182 registers at 35 taps.)
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -196,7 +199,7 @@ __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__
             for (int q = 0; q < NE; ++q) {
                 const int e = lane + 32 * q, x = x0 + e;
                 const bool ok = e < span && x < s.W;
-                ph[q] = ok ? __ldg(phi + x) : 0.0f;
+                ph[q] = ok ? phi[x] : 0.0f;
                 im[q] = ok ? load_img(s.img, row + x, c.img_f32) : 0.0f;
             }
             // (elements past the row feed only outputs past Wv)
@@ -213,7 +216,7 @@ __global__ void __launch_bounds__(XP_ROWS * 32) xpass_kernel(const SubVolDev *__
             for (int e = lane; e < span; e += 64) {
                 const int x = x0 + e;
                 const bool ok0 = x < s.W, ok1 = e + 32 < span && x + 32 < s.W;
-                const float p0 = ok0 ? __ldg(phi + x) : 0.0f, p1 = ok1 ? __ldg(phi + x + 32) : 0.0f;
+                const float p0 = ok0 ? phi[x] : 0.0f, p1 = ok1 ? phi[x + 32] : 0.0f;
                 const float i0 = ok0 ? load_img(s.img, row + x, c.img_f32) : 0.0f;
                 const float i1 = ok1 ? load_img(s.img, row + x + 32, c.img_f32) : 0.0f;
                 const float2 h = heaviside2<A>(make_float2(p0, p1), c.eps, c.pk);
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(YP_COLS) ypass_chunk_kernel(const SubVolDev *_
     unsigned long long *dst = reinterpret_cast<unsigned long long *>(s.yb) + ((size_t)z * s.Hv + y0) * row + x;
     const int have = min(s.H - y0, NB + c.k - 1);
     unsigned long long u[NB];
-    conv_chunks<NB>(c, [&](int i) { return i < have ? __ldg(src + (size_t)i * row) : 0ull; }, u);
+    conv_chunks<NB>(c, [&](int i) { return i < have ? src[(size_t)i * row] : 0ull; }, u);
 #pragma unroll
     for (int m = 0; m < NB; ++m)
         if (y0 + m < s.Hv) dst[(size_t)m * row] = u[m];
@@ -560,7 +563,7 @@ __device__ __forceinline__ void zchunk(const SubVolDev &s, const StepConst &c, c
     const int have = min(s.L - z.o0, NB + c.k - 1);
     ulonglong2 w[2 * NB];
     unsigned long long a[NB], b[NB];
-    auto load = [&](int i) { return i < have ? __ldg(src + (size_t)i * z.plane) : make_ulonglong2(0ull, 0ull); };
+    auto load = [&](int i) { return i < have ? src[(size_t)i * z.plane] : make_ulonglong2(0ull, 0ull); };
 #pragma unroll
     for (int m = 0; m < NB; ++m) {
         a[m] = b[m] = 0ull;

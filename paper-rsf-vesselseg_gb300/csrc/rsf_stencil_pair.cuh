@@ -132,13 +132,13 @@ __device__ __forceinline__ void pair_step(const PairCtx &k, const StepConst &c, 
     // data factor of plane sc + 1, or the image in the border band
     float2 dn = make_float2(0.0f, 0.0f);
     if (INSIDE) {
-        if (k.out0) dn.x = __ldg(q.d);
-        if (k.out1) dn.y = __ldg(q.d + k.dstep);
+        if (k.out0) dn.x = *q.d;
+        if (k.out1) dn.y = q.d[k.dstep];
     } else if (!EDGE || (sc + 1 >= k.z0 && sc + 1 < k.z1)) {
         const bool zin = sc + 1 >= k.rz && sc + 1 < k.L - k.rz;
-        if (zin && k.val0) dn.x = __ldg(q.d);
+        if (zin && k.val0) dn.x = *q.d;
         else if (k.out0) dn.x = border_word(q.i, c.img_f32);
-        if (zin && k.val1) dn.y = __ldg(q.d + k.dstep);
+        if (zin && k.val1) dn.y = q.d[k.dstep];
         else if (k.out1) dn.y = border_word(q.i + k.istep, c.img_f32);
     }
     q.d += k.dplane;
