@@ -23,7 +23,7 @@
 namespace rsf {
 namespace {
 
-constexpr int kThreads = 64;  // small, so that ragged rows leave few threads idle
+constexpr int kThreads = 64;  // per block: small, so that ragged rows leave few threads idle
 
 struct ReasmConst {
     int n[3];                        // cells per axis (x, y, z)
@@ -64,15 +64,20 @@ __device__ __forceinline__ float axis_weight(const ReasmConst &c, int a, int ci,
     return w;
 }
 
-// A block takes kThreads voxels of one output row after another (grid y strides
-// over the rows), so the y and z cells and weights are found once per row and a
-// voxel is left with its x cells: 190x333x290 voxels of 18 blended tiles took
-// 414 us with a flat index per voxel (three divisions and searches each), 281 so
-// (289 with 256 threads, 311 with four voxels per thread).
+// A block of BX x (kThreads / BX) threads takes BX voxels of that many output rows at
+// a time (grid y strides over the rows), so the y and z cells and weights are found
+// once per row and a voxel is left with its x cells: 190x333x290 voxels of 18
+// blended tiles took 414 us with a flat index per voxel (three divisions and
+// searches each), 281 so (289 with 256 threads, 311 with four voxels per thread).
+// BX (launch_rows) follows the width: with 64 for every width 2000x2000x3 voxels
+// took 1185 us (cores) and 2418 us (blend), the flat index 153 and 235, this 145 and
+// 219.
+template <int BX>
 __global__ void __launch_bounds__(kThreads) reassemble_kernel(const __grid_constant__ ReasmConst c,
                                                               const TileDev *__restrict__ tiles, float *out) {
-    const int x = blockIdx.x * kThreads + threadIdx.x;
+    const int x = blockIdx.x * BX + threadIdx.x % BX;
     if (x >= c.ext[0]) return;
+    constexpr int BY = kThreads / BX;
     const long long rows = (long long)c.ext[1] * c.ext[2];
     const int ix = cell_of(c, 0, x);
     float wx[3] = {0.0f, 0.0f, 0.0f};
@@ -81,7 +86,7 @@ __global__ void __launch_bounds__(kThreads) reassemble_kernel(const __grid_const
         for (int dx = -1; dx <= 1; dx++)
             if (ix + dx >= 0 && ix + dx < c.n[0]) wx[dx + 1] = axis_weight(c, 0, ix + dx, x);
     }
-    for (long long row = blockIdx.y; row < rows; row += gridDim.y) {
+    for (long long row = blockIdx.y * BY + threadIdx.x / BX; row < rows; row += gridDim.y * BY) {
         const int z = (int)(row / c.ext[1]), y = (int)(row - (long long)z * c.ext[1]);
         const int iy = cell_of(c, 1, y), iz = cell_of(c, 2, z);
         const long long i = row * c.ext[0] + x;
@@ -113,6 +118,22 @@ __global__ void __launch_bounds__(kThreads) reassemble_kernel(const __grid_const
     }
 }
 
+// The most threads along a row (powers of two, so that a warp writes whole pieces of
+// rows) that leave at most a tenth of a row's threads without a voxel: 2000x2000x33
+// voxels (cores) take 863 us with a quarter allowed, 798 so (the flat index 777); with
+// a sixteenth 190x333x290 loses its rows of 64 (376 -> 400 us, blend).
+template <int BX = kThreads>
+void launch_rows(const ReasmConst &c, const TileDev *tiles, float *out, cudaStream_t st) {
+    const int W = c.ext[0], ntx = (W + BX - 1) / BX;
+    if constexpr (BX > 1) {
+        if (10 * (ntx * BX - W) > ntx * BX) return launch_rows<BX / 2>(c, tiles, out, st);
+    }
+    constexpr int BY = kThreads / BX;
+    const long long groups = ((long long)c.ext[1] * c.ext[2] + BY - 1) / BY, want = (64LL * sm_count() + ntx - 1) / ntx;
+    const unsigned ny = (unsigned)(groups < want ? groups : want < 65535 ? want : 65535);
+    reassemble_kernel<BX><<<dim3((unsigned)ntx, ny), kThreads, 0, st>>>(c, tiles, out);
+}
+
 }  // namespace
 
 cudaError_t launch_reassemble(const TileDev *d_tiles, const int n[3], const int *const cb[3], const int *const lo[3],
@@ -130,10 +151,7 @@ cudaError_t launch_reassemble(const TileDev *d_tiles, const int n[3], const int 
             c.hi[a][j] = j < n[a] ? hi[a][j] : 0;
         }
     }
-    const unsigned ntx = (unsigned)((W + kThreads - 1) / kThreads);
-    const long long rows = (long long)H * L, want = (64LL * sm_count() + ntx - 1) / ntx;
-    const unsigned ny = (unsigned)(rows < want ? rows : want < 65535 ? want : 65535);
-    reassemble_kernel<<<dim3(ntx, ny), kThreads, 0, st>>>(c, d_tiles, out);
+    launch_rows(c, d_tiles, out, st);
     return cudaGetLastError();
 }
 
