@@ -25,13 +25,18 @@
 // Columns of up to kTileMax voxels take the tiled kernels instead: both
 // classes at once (a voxel needs its distance to the other class only, so one
 // signed value per voxel carries both transforms), a block holding 32 whole
-// columns in shared memory and every voxel searching outwards from itself.
-// The envelope is a serial chain of dependent loads per column, with one thread
-// per column; the search has a thread per four voxels and stops at the
-// distance found, and beyond kFine rows it skips blocks of 16 rows whose
-// smallest value cannot improve on it, so that sparse seeds stay cheap.
-// 256 x 448 x 512 voxels, a tenth of them inside:
-// 3.90 ms with the envelopes, 0.80 ms here.
+// columns in shared memory and a thread per four rows.  The envelope is a serial
+// chain of dependent loads per column, with one thread per column; here a
+// thread searches outwards a few rows, which ends most voxels near a surface, and
+// the others go by halving: for one class the nearest row's index grows with
+// the voxel's (Aggarwal et al., "Geometric applications of a matrix-searching
+// algorithm", Algorithmica 2, 1987), so a group of rows between two finished
+// groups searches only the rows between their results.  That bounds the work per
+// voxel whatever the seeds are, as the envelope's is.  256 x 448 x 512 voxels:
+// winding vessels 3.84 ms with the envelopes, 0.87 here; an empty seed 2.04 and
+// 1.38; a slanted plane 2.70 and 1.48 (3.94 with the search alone, blocks of 16 rows
+// skipped where their smallest value cannot improve; on 500^3 9.5 ms, 4.7 with the
+// envelopes, 3.7 here); sparse noise (1e-3) 2.65 and 1.36.
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -182,9 +187,8 @@ __global__ void __launch_bounds__(kColThreads) sdf_cols(ColArgs a) {
 // Tiled path.  Values are signed: positive inside, negative outside, the
 // magnitude the distance to the other class so far.
 // ---------------------------------------------------------------------------
-constexpr int kTileMax = 1408;          // column length: 32 columns of 32-bit values and their block minima in shared memory
-constexpr int kFine = 24;               // rows searched one by one to either side
-constexpr int kSkip = 16;               // rows per skipped block beyond
+constexpr int kTileMax = 1408;          // column length: 32 columns of 32-bit values and their groups' results in shared memory
+constexpr int kShortMax = 144;          // columns up to here search more rows one by one (see launch_tile)
 constexpr short kNone16 = 32767;        // no voxel of the other class in the row
 constexpr int kNone = 1 << 28;          // nor in the plane; plus any squared offset it stays above every distance
 
@@ -239,26 +243,31 @@ struct TileArgs {
     const void *in;     // signed row distances (int16), or squared plane distances (int32) for FINAL
     int *out;           // squared plane distances, signed
     float *phi;         // FINAL
-    int W, n, ntx;
-    long long plane;    // element offset of a column group's outer index
+    int W, n, ncols;    // columns are numbered c = a * W + x
+    long long plane;    // element offset of a column: (c / W) * plane + c % W
     long long stride;   // element step along the column
     float fill;
 };
 
+// A group's state: the row that is nearest to its first row, or one of these.
+constexpr unsigned short kNear = 0xffff;  // found within FINE rows
+constexpr unsigned short kFar = 0xfffe;   // not found yet
+
 // Squared distance along a strided axis added to the values in `in`, for 32
-// columns per block.  A thread takes four consecutive rows, which share every
-// value they read: rows y0 - t and y0 + 3 + t lie t .. t + 3 rows from them.
-template <bool FINAL, int T>
+// columns per block (one per lane).  A thread takes groups of four consecutive
+// rows, which share every value they read: rows y0 - t and y0 + 3 + t lie
+// t .. t + 3 rows from them.  Every voxel searches TRY rows to either side, and FINE
+// if its distance so far is at most one row more.
+template <bool FINAL, int T, int TRY, int FINE>
 __global__ void __launch_bounds__(T) sdf_cols_tile(TileArgs a) {
     extern __shared__ int sdf_sm[];
-    int *v = sdf_sm;                                // [n][32]
-    const int nb = (a.n + kSkip - 1) / kSkip;
-    int *mo = v + 32 * a.n, *mi = mo + 32 * nb;     // block minima of the distance to outside / inside
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     constexpr int NW = T / 32;
-    const int x = (blockIdx.x % a.ntx) * 32 + lane;
-    const bool have = x < a.W;
-    const size_t base = (size_t)(blockIdx.x / a.ntx) * (size_t)a.plane + x;
+    int *v = sdf_sm + lane;  // the lane's column: row r at v[32 r]
+    unsigned short *state = reinterpret_cast<unsigned short *>(sdf_sm + 32 * a.n) + lane;  // group g at state[32 g]
+    const int col = blockIdx.x * 32 + lane;
+    const bool have = col < a.ncols;
+    const size_t base = (size_t)(col / a.W) * (size_t)a.plane + (size_t)(col % a.W);
     for (int r = w; r < a.n; r += NW) {
         int q = 1;
         if (have) {
@@ -271,70 +280,22 @@ __global__ void __launch_bounds__(T) sdf_cols_tile(TileArgs a) {
                 q = d > 0 ? m : -m;
             }
         }
-        v[32 * r + lane] = q;
+        v[32 * r] = q;
     }
     __syncthreads();
-    for (int b = w; b < nb; b += NW) {
-        int so = kNone, si = kNone;
-        for (int r = kSkip * b; r < min(kSkip * (b + 1), a.n); ++r) {
-            const int q = v[32 * r + lane];
-            so = min(so, max(q, 0));
-            si = min(si, max(-q, 0));
-        }
-        mo[32 * b + lane] = so;
-        mi[32 * b + lane] = si;
-    }
-    __syncthreads();
-    for (int y0 = 4 * w; y0 < a.n; y0 += 4 * NW) {
-        int s[4], best[4];
+    int s[4], best[4];
+    // a voxel of the other class counts 0, one of the same class its own distance
+    auto take = [&](int q, int j, int d2) { best[j] = min(best[j], max(s[j] * q + d2, d2)); };
+    auto worst = [&] { return max(max(best[0], best[1]), max(best[2], best[3])); };
+    auto own = [&](int y0) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int q = v[32 * min(y0 + j, a.n - 1) + lane];
+            const int q = v[32 * min(y0 + j, a.n - 1)];
             s[j] = q > 0 ? 1 : -1;
             best[j] = abs(q);
         }
-        // a voxel of the other class counts 0, one of the same class its own distance
-        auto take = [&](int q, int j, int d2) { best[j] = min(best[j], max(s[j] * q + d2, d2)); };
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int q = v[32 * min(y0 + i, a.n - 1) + lane];
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (i != j) take(q, j, (i - j) * (i - j));
-        }
-        auto worst = [&] { return max(max(best[0], best[1]), max(best[2], best[3])); };
-        // rows past an end repeat the last one at a larger offset, which never wins
-        int t = 1;
-        for (; t <= kFine && __any_sync(0xffffffffu, t * t < worst()); ++t) {
-            const int ql = v[32 * max(y0 - t, 0) + lane], qr = v[32 * min(y0 + 3 + t, a.n - 1) + lane];
-            const int t0 = t * t, t1 = t0 + 2 * t + 1, t2 = t0 + 4 * t + 4, t3 = t0 + 6 * t + 9;
-            take(ql, 0, t0);
-            take(ql, 1, t1);
-            take(ql, 2, t2);
-            take(ql, 3, t3);
-            take(qr, 3, t0);
-            take(qr, 2, t1);
-            take(qr, 1, t2);
-            take(qr, 0, t3);
-        }
-        if (t > kFine && __any_sync(0xffffffffu, t * t < worst())) {
-            // (a lane that gets here has four voxels of one class: mixed ones found each other)
-            const int *m = s[0] > 0 ? mo : mi;
-            for (int side = 0; side < 2; ++side) {
-                const int step = side ? 1 : -1;
-                for (int b = side ? min(y0 + 3 + t, a.n - 1) / kSkip : max(y0 - t, 0) / kSkip; b >= 0 && b < nb; b += step) {
-                    const int gap = max(side ? kSkip * b - (y0 + 3) : y0 - (kSkip * b + kSkip - 1), 0);
-                    const int wst = worst();
-                    if (!__any_sync(0xffffffffu, gap * gap < wst)) break;
-                    if (!__any_sync(0xffffffffu, gap * gap + m[32 * b + lane] < wst)) continue;
-                    for (int r = kSkip * b; r < min(kSkip * (b + 1), a.n); ++r) {
-                        const int q = v[32 * r + lane];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) take(q, j, (r - y0 - j) * (r - y0 - j));
-                    }
-                }
-            }
-        }
+    };
+    auto store = [&](int y0) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             if (!have || y0 + j >= a.n) continue;
@@ -346,25 +307,127 @@ __global__ void __launch_bounds__(T) sdf_cols_tile(TileArgs a) {
                 a.out[i] = s[j] * best[j];
             }
         }
+    };
+    bool far = false;
+    for (int y0 = 4 * w; y0 < a.n; y0 += 4 * NW) {
+        own(y0);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int q = v[32 * min(y0 + i, a.n - 1)];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (i != j) take(q, j, (i - j) * (i - j));
+        }
+        // rows past an end repeat the last one at a larger offset, which never wins
+        auto go_on = [&](int t) {
+            const int wst = worst();
+            return t * t < wst && (t <= TRY || wst <= (FINE + 1) * (FINE + 1));
+        };
+        for (int t = 1; t <= FINE && __any_sync(0xffffffffu, go_on(t)); ++t) {
+            const int ql = v[32 * max(y0 - t, 0)], qr = v[32 * min(y0 + 3 + t, a.n - 1)];
+            const int t0 = t * t, t1 = t0 + 2 * t + 1, t2 = t0 + 4 * t + 4, t3 = t0 + 6 * t + 9;
+            take(ql, 0, t0);
+            take(ql, 1, t1);
+            take(ql, 2, t2);
+            take(ql, 3, t3);
+            take(qr, 3, t0);
+            take(qr, 2, t1);
+            take(qr, 1, t2);
+            take(qr, 0, t3);
+        }
+        // (a far lane has four voxels of one class: mixed ones found each other)
+        const bool fin = worst() <= (FINE + 1) * (FINE + 1);
+        state[8 * y0] = fin ? kNear : kFar;
+        if (fin) store(y0);
+        else far = true;
+    }
+    if (!__syncthreads_or(far)) return;
+    // The far groups by halving: groups are numbered from 1, those that are odd
+    // multiples of `step` lie between two multiples of 2 step, which are finished (0
+    // and numbers past the last stand for the column's ends).
+    const int groups = (a.n + 3) / 4;
+    int step = 1;
+    while (2 * step <= groups) step *= 2;
+    for (; step > 0; step /= 2) {
+        for (int i = w;; i += NW) {
+            const int below = 2 * step * i, above = below + 2 * step, g = below + step;
+            if (g > groups) break;
+            const bool todo = state[32 * (g - 1)] == kFar;
+            if (!__any_sync(0xffffffffu, todo)) continue;
+            const int y0 = 4 * (g - 1);
+            int lo = y0, hi = y0, at = y0;
+            if (todo) {
+                own(y0);
+                lo = 0;
+                hi = a.n - 1;
+                // a group found near lies at most FINE + 1 rows from its result; one of
+                // the other class is its own
+                if (below > 0) {
+                    const int yn = 4 * (below - 1);
+                    const unsigned short sn = state[8 * yn];
+                    lo = sn == kNear ? max(yn + 2 - FINE, 0) : s[0] * v[32 * yn] > 0 ? sn : yn + 3;
+                }
+                if (above <= groups) {
+                    const int yn = 4 * (above - 1);
+                    const unsigned short sn = state[8 * yn];
+                    hi = sn == kNear ? min(yn + FINE + 1, hi) : s[0] * v[32 * yn] > 0 ? sn : yn;
+                }
+            }
+            // row r: its distance to the group's first row, and to all four
+            auto row = [&](int r) {
+                const int q = max(s[0] * v[32 * r], 0), d = r - y0, c = q + d * d;
+                if (c < best[0]) {
+                    best[0] = c;
+                    at = r;
+                }
+                best[1] = min(best[1], c - 2 * d + 1);
+                best[2] = min(best[2], c - 4 * d + 4);
+                best[3] = min(best[3], c - 6 * d + 9);
+            };
+            if (todo) {
+                row(lo);
+                row(hi);
+                // rows further away than the worst distance so far cannot improve any
+                const int reach = (int)sqrtf((float)worst()) + 1;
+                lo = max(lo, y0 - reach);
+                hi = min(hi, y0 + 3 + reach);
+            }
+            const int last = __reduce_max_sync(0xffffffffu, hi - lo);
+            if (todo) {
+                for (int i = 0; i <= last; i += 4) {
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) row(min(lo + i + m, hi));
+                }
+                state[8 * y0] = (unsigned short)at;
+                store(y0);
+            }
+        }
+        __syncthreads();
     }
 }
 
-size_t tile_smem(int n) { return 128 * ((size_t)n + 2 * ((n + kSkip - 1) / kSkip)); }
+size_t tile_smem(int n) { return 128 * (size_t)n + 64 * ((size_t)(n + 3) / 4); }
 
 // 256 threads share an SM three or more times up to about 500 rows; longer
 // columns leave one or two blocks, which then bring 512.
 constexpr int kWideFrom = 560;
 
+// TRY and FINE, by winding vessels (the first figure) and planes (the second): 4 and 24
+// take 0.87 and 1.45 ms on 256 x 448 x 512 voxels, 8 and 48 0.86 and 1.72.  In short
+// columns the halving's levels, one after the other, are latency: 128^3 takes 76 and
+// 125 us with 4 and 24, 69 and 177 with 8 and 48, 96^3 54 and 75, 49 and 94.
 template <bool FINAL>
-void launch_tile(const TileArgs &a, long long groups, cudaStream_t st) {
-    const unsigned blocks = (unsigned)(groups * a.ntx);
-    if (a.n >= kWideFrom) sdf_cols_tile<FINAL, 512><<<blocks, 512, tile_smem(a.n), st>>>(a);
-    else sdf_cols_tile<FINAL, 256><<<blocks, 256, tile_smem(a.n), st>>>(a);
+void launch_tile(const TileArgs &a, cudaStream_t st) {
+    const unsigned blocks = (unsigned)((a.ncols + 31) / 32);
+    const size_t sm = tile_smem(a.n);
+    if (a.n >= kWideFrom) sdf_cols_tile<FINAL, 512, 4, 24><<<blocks, 512, sm, st>>>(a);
+    else if (a.n > kShortMax) sdf_cols_tile<FINAL, 256, 4, 24><<<blocks, 256, sm, st>>>(a);
+    else sdf_cols_tile<FINAL, 256, 8, 48><<<blocks, 256, sm, st>>>(a);
 }
 
 template <bool FINAL, int T>
 cudaError_t allow_tile() {
-    return cudaFuncSetAttribute(sdf_cols_tile<FINAL, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(sdf_cols_tile<FINAL, T, 4, 24>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)tile_smem(T == 512 ? kTileMax : kWideFrom));
 }
 
@@ -389,9 +452,8 @@ cudaError_t launch_signed_distance(const void *seed, int f32, float thr, float *
         int *dxy = reinterpret_cast<int *>(scratch);
         sdf_rows_tile<<<(unsigned)((rows + kRowWarps - 1) / kRowWarps), 32 * kRowWarps, 0, st>>>(seed, f32, thr, dx, W,
                                                                                                 rows);
-        const int ntx = (W + 31) / 32;
-        launch_tile<false>(TileArgs{dx, dxy, nullptr, W, H, ntx, (long long)W * H, W, fill}, L, st);
-        launch_tile<true>(TileArgs{dxy, nullptr, phi, W, L, ntx, W, (long long)W * H, fill}, H, st);
+        launch_tile<false>(TileArgs{dx, dxy, nullptr, W, H, W * L, (long long)W * H, W, fill}, st);
+        launch_tile<true>(TileArgs{dxy, nullptr, phi, W, L, W * H, W, (long long)W * H, fill}, st);
         return cudaGetLastError();
     }
     for (int feat_inside = 0; feat_inside < 2; feat_inside++) {
