@@ -85,7 +85,7 @@ def _time_plan(tiles: Sequence[Tile], params: Params, dtype, iters: int, device)
             img = (torch.randint(0, 256, t.shape, generator=gen, device=device, dtype=torch.uint8)
                    if dtype == "u8" else torch.rand(t.shape, generator=gen, device=device))
             pairs.append((img, smooth_phi(t.shape, device)))
-        ws.evolve_batched(pairs, params, 1)  # warm-up (graph capture, table upload)
+        ws.evolve_batched(pairs, params, 1)  # warm-up
         torch.cuda.synchronize(device)
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record()
@@ -121,13 +121,17 @@ def tune_cores(shape: Sequence[int], params: Params, halo: int = 32, dtype: str 
 # Kernel launch shapes.  The kernels take three shape choices per launch: the
 # x-pass lane width (5 or 9 outputs per lane: which wastes fewer outputs past
 # the valid width depends on the batch's row lengths), the stencil's planes
-# per block (128 or 64, or 32 for batches too small to fill the GPU several
-# times)
-# and, for 21 and 35 taps, whether the z-pass takes its planes through TMA.
-# The workspace picks them by heuristics; `tune_launch_shape` times every
-# combination on the caller's batch and keeps the fastest.
+# per block (0: the workspace's own choice from the batch's shapes, which goes
+# down to 2 planes for small volumes; 128 and 64 for batches that fill the GPU
+# several times) and, for 21 and 35 taps, whether the z-pass takes its planes
+# through TMA.  The workspace picks them by heuristics; `tune_launch_shape`
+# times every combination on the caller's batch and keeps the fastest.
 # ---------------------------------------------------------------------------
-LAUNCH_CANDIDATES = tuple((xb, zc, zt) for xb in (5, 9) for zc in (128, 64, 32) for zt in (0, 1))
+LAUNCH_CANDIDATES = tuple((xb, zc, zt) for xb in (5, 9) for zc in (0, 128, 64) for zt in (0, 1))
+
+# Iterations from which a batched evolution runs as a captured graph: shorter
+# timed runs would measure the direct launches instead.
+GRAPH_FROM = 4
 
 
 @dataclass
@@ -149,9 +153,9 @@ def pick_launch_shape(measurements: Sequence[Tuple[Tuple[int, int, int], float]]
 def tune_launch_shape(ws: Workspace, pairs, params: Params, iters: int = 4,
                       candidates: Sequence[Tuple[int, int, int]] = LAUNCH_CANDIDATES,
                       timer: Optional[Callable[[Tuple[int, int, int]], float]] = None) -> LaunchShape:
-    """Times `iters` batched iterations of `pairs` (image, phi) for every
-    launch shape, restoring each phi between the runs, sets the fastest on
-    `ws` and returns it.  `timer(shape) -> ms per iteration` replaces the
+    """Times `iters` (at least GRAPH_FROM) batched iterations of `pairs` (image,
+    phi) for every launch shape, restoring each phi between the runs, sets the
+    fastest on `ws` and returns it.  `timer(shape) -> ms per iteration` replaces the
     device measurement (for tests)."""
     meas = []
     if timer is not None:
@@ -160,11 +164,12 @@ def tune_launch_shape(ws: Workspace, pairs, params: Params, iters: int = 4,
     else:
         import torch
 
+        iters = max(iters, GRAPH_FROM)
         starts = [phi.clone() for _, phi in pairs]
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         for shape in candidates:
             ws.set_launch_shape(*shape)
-            ws.evolve_batched(pairs, params, 1)  # graph capture and table upload
+            ws.evolve_batched(pairs, params, 1)  # warm-up
             for (_, phi), s0 in zip(pairs, starts):
                 phi.copy_(s0)
             torch.cuda.synchronize()
