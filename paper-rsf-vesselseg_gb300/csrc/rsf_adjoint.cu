@@ -93,35 +93,36 @@ constexpr int kWZ = 8;  // planes per block of adj_gather
 
 // The difference rules of a voxel along one axis without branches (a warp that
 // touches a face would otherwise take the general and the inner form one after
-// the other).  D f = (f(i + r) - f(i - l)) / 2 with the offsets r, l; its
-// transpose gathers D^T v = m v(i - s) + c v(i) + p v(i + s) with s the axis
-// stride.  Along x the neighbours are the ones in memory: in the reference
-// boundary mode (kernel.cu:64-67) x = 0 reads the previous linear element, so
-// the last voxel of a row is read by the first one of the next.
+// the other).  D f = (f(i + r) - f(i - l)) / 2 with the offsets r, l.  Its
+// transpose gathers D^T v = m v(i - l) + p v(i + r) with the same offsets: where a
+// neighbour is missing the voxel's own value takes its place.  A value has no
+// other part in it, so that an infinite one stays out of results that do not
+// depend on it.
 struct Axis {
-    long long s, r, l;
-    float m, c, p;
+    long long r, l;
+    float m, p;
 };
 __device__ __forceinline__ Axis axis_plain(int q, int n, long long s) {
     const bool lo = q > 0, hi = q + 1 < n;
-    return {s, hi ? s : 0, lo ? s : 0, lo ? 0.5f : 0.0f, (hi ? 0.0f : 0.5f) - (lo ? 0.0f : 0.5f), hi ? -0.5f : 0.0f};
+    return {hi ? s : 0, lo ? s : 0, lo ? 0.5f : -0.5f, hi ? -0.5f : 0.5f};
 }
-// x at linear index i of N; i > 0 and i + 1 < N decide at the volume's ends.
-__device__ __forceinline__ Axis axis_x(const AdjVol &a, int boundary, int x, long long i, long long N) {
-    Axis k = axis_plain(x, a.W, 1);
-    if (boundary == 0) {
-        k.l = i > 0 ? 1 : 0;
-        k.c = (x + 1 < a.W ? 0.0f : 0.5f) - (i > 0 ? 0.0f : 0.5f);
-        k.p = i + 1 < N ? -0.5f : 0.0f;
-    }
-    return k;
+// Along x the neighbours are the ones in memory: in the reference boundary mode
+// (kernel.cu:64-67) x = 0 reads the previous linear element, so the last voxel
+// of a row is read by the first one of the next and, being its own right
+// neighbour, by itself.  D^T v = m v(i - 1) + c v(i) + p v(i + 1), i > 0 and
+// i + 1 < N decide at the volume's ends.
+struct AxisX {
+    int r, l;
+    float m, c, p;
+};
+__device__ __forceinline__ AxisX axis_x(const AdjVol &a, int boundary, int x, long long i, long long N) {
+    const bool lo = x > 0, hi = x + 1 < a.W;
+    const bool left = boundary == 0 ? i > 0 : lo, right = boundary == 0 ? i + 1 < N : hi;
+    return {hi, left, lo ? 0.5f : 0.0f, (hi ? 0.0f : 0.5f) - (left ? 0.0f : 0.5f), right ? -0.5f : 0.0f};
 }
-// m v(i - s) + c v(i) + p v(i + s), v0 = v(i); a neighbour without weight is
-// not read (it may lie outside the volume).
-template <class V>
-__device__ __forceinline__ float gather3(const Axis &k, long long i, float v0, V v) {
-    const float vm = k.m != 0.0f ? v(i - k.s) : 0.0f, vp = k.p != 0.0f ? v(i + k.s) : 0.0f;
-    return fmaf(k.p, vp, fmaf(k.c, v0, k.m * vm));
+// The sum from the neighbours' values (0 where they have no weight) and the own.
+__device__ __forceinline__ float gather_x(const AxisX &k, float vm, float v0, float vp) {
+    return fmaf(k.p, vp, fmaf(k.c, k.c != 0.0f ? v0 : 0.0f, k.m * vm));
 }
 
 // delta(phi) with a fast division: the adjoint needs the derivative's value,
@@ -283,10 +284,10 @@ __global__ void __launch_bounds__(kThreads) adj_normals(AdjConst c, const AdjVol
     const long long t1 = i / a.W;
     const int y = (int)(t1 % a.H);
     const int z = (int)(t1 / a.H);
-    const Axis ax = axis_x(a, c.boundary, x, i, N), ay = axis_plain(y, a.H, a.W),
-               az = axis_plain(z, a.L, (long long)a.W * a.H);
-    auto diff = [&](const Axis &k) { return 0.5f * (a.phi[i + k.r] - a.phi[i - k.l]); };
-    const float gx = diff(ax), gy = diff(ay), gz = diff(az);
+    const AxisX ax = axis_x(a, c.boundary, x, i, N);
+    const Axis ay = axis_plain(y, a.H, a.W), az = axis_plain(z, a.L, (long long)a.W * a.H);
+    auto diff = [&](long long r, long long l) { return 0.5f * (a.phi[i + r] - a.phi[i - l]); };
+    const float gx = diff(ax.r, ax.l), gy = diff(ay.r, ay.l), gz = diff(az.r, az.l);
     a.xs[i] = gx;
     a.xs[N + i] = gy;
     a.ys[i] = gz;
@@ -341,17 +342,18 @@ __global__ void __launch_bounds__(kBX * kBY, 2) adj_point(AdjConst c, const AdjV
     if (x < a.W && y < a.H) {
         long long i = ((long long)cl.z0 * a.H + y) * a.W + x;
         const Axis ay = axis_plain(y, a.H, a.W);
-        // of planes z - 1, z: kappa_bar, Lap_bar, g_z and 1/(|g|+1e-6)
-        float k0 = 0.0f, l0 = 0.0f, gz0 = 0.0f, r0 = 0.0f;
+        // of planes z - 1, z, z + 1: kappa_bar, Lap_bar, g_z and 1/(|g|+1e-6); the
+        // voxel's own where there is no such plane
+        float k1 = kbar(i), l1 = lbar(i), gz1 = gza[i], r1 = rsa[i];
+        float k0 = k1, l0 = l1, gz0 = gz1, r0 = r1;
         if (cl.z0 > 0) {
             k0 = kbar(i - plane);
             l0 = lbar(i - plane);
             gz0 = gza[i - plane];
             r0 = rsa[i - plane];
         }
-        float k1 = kbar(i), l1 = lbar(i), gz1 = gza[i], r1 = rsa[i];
         for (int z = cl.z0; z < z1; ++z, i += plane) {
-            float k2 = 0.0f, l2 = 0.0f, gz2 = 0.0f, r2 = 0.0f;
+            float k2 = k1, l2 = l1, gz2 = gz1, r2 = r1;
             if (z + 1 < a.L) {
                 k2 = kbar(i + plane);
                 l2 = lbar(i + plane);
@@ -363,31 +365,27 @@ __global__ void __launch_bounds__(kBX * kBY, 2) adj_point(AdjConst c, const AdjV
             const float gx = gxa[i], gy = gya[i];
             const float delta = dirac_fast(ph, c.eps);
             const float ddelta = __fdividef(-2.0f * ph * delta, fmaf(ph, ph, c.eps * c.eps));
-            const Axis ax = axis_x(a, c.boundary, x, i, N), az = axis_plain(z, a.L, plane);
+            const AxisX ax = axis_x(a, c.boundary, x, i, N);
+            const Axis az = axis_plain(z, a.L, plane);
             // curvature and "Laplacian"; the z neighbours are at hand
             const long long rx = i + ax.r, lx = i - ax.l, ry = i + ay.r, ly = i - ay.l;
             const float gxr = gxa[rx], gxl = gxa[lx], gyr = gya[ry], gyl = gya[ly];
-            const float gzr = az.r ? gz2 : gz1, gzl = az.l ? gz0 : gz1;
             // The normals are rounded before they are subtracted, so that equal
             // neighbours cancel (a contracted multiply-add would leave the rounding
             // of one product, times u).
             const float kap = 0.5f * (__fmul_rn(gxr, rsa[rx]) - __fmul_rn(gxl, rsa[lx])) +
                               0.5f * (__fmul_rn(gyr, rsa[ry]) - __fmul_rn(gyl, rsa[ly])) +
-                              0.5f * (__fmul_rn(gzr, az.r ? r2 : r1) - __fmul_rn(gzl, az.l ? r0 : r1));
-            const float lap = 0.5f * (gxr - gxl) + 0.5f * (gyr - gyl) + 0.5f * (gzr - gzl);
+                              0.5f * (__fmul_rn(gz2, r2) - __fmul_rn(gz0, r0));
+            const float lap = 0.5f * (gxr - gxl) + 0.5f * (gyr - gyl) + 0.5f * (gz2 - gz0);
             // D^T of kappa_bar and Lap_bar
-            float nbx, nby, lbx, lby;
-            auto both = [&](const Axis &k, float &nb, float &lb) {
-                float um = 0.0f, up = 0.0f, pm = 0.0f, pp = 0.0f;
-                if (k.m != 0.0f) um = uu[i - k.s] * c.dt, pm = phi[i - k.s];
-                if (k.p != 0.0f) up = uu[i + k.s] * c.dt, pp = phi[i + k.s];
-                auto kb = [&](float u, float p) { return u * (c.nu * dirac_fast(p, c.eps) - c.mu); };
-                nb = fmaf(k.p, kb(up, pp), fmaf(k.c, k1, k.m * kb(um, pm)));
-                lb = fmaf(k.p, up * c.mu, fmaf(k.c, l1, k.m * (um * c.mu)));
-            };
-            both(ax, nbx, lbx);
-            both(ay, nby, lby);
-            const float nbz = fmaf(az.p, k2, fmaf(az.c, k1, az.m * k0)), lbz = fmaf(az.p, l2, fmaf(az.c, l1, az.m * l0));
+            auto kb = [&](float u, float p) { return u * (c.nu * dirac_fast(p, c.eps) - c.mu); };
+            float um = 0.0f, up = 0.0f, pm = 0.0f, pp = 0.0f;
+            if (ax.m != 0.0f) um = uu[i - 1] * c.dt, pm = phi[i - 1];
+            if (ax.p != 0.0f) up = uu[i + 1] * c.dt, pp = phi[i + 1];
+            const float nbx = gather_x(ax, kb(um, pm), k1, kb(up, pp)), lbx = gather_x(ax, um * c.mu, l1, up * c.mu);
+            const float vm = uu[ly] * c.dt, vp = uu[ry] * c.dt;
+            const float nby = fmaf(ay.p, kb(vp, phi[ry]), ay.m * kb(vm, phi[ly])), lby = fmaf(ay.p, vp * c.mu, ay.m * (vm * c.mu));
+            const float nbz = fmaf(az.p, k2, az.m * k0), lbz = fmaf(az.p, l2, az.m * l0);
             const bool valid = a.Wv > 0 && x >= c.r && x < c.r + a.Wv && y >= c.r && y < c.r + a.Hv && z >= c.r &&
                                z < c.r + a.Lv;
             float eo, ei;
@@ -458,13 +456,13 @@ __global__ void __launch_bounds__(kBX * kBY) adj_gather(AdjConst c, const AdjVol
     const Axis ay = axis_plain(y, a.H, a.W);
     long long i = ((long long)cl.z0 * a.H + y) * a.W + x;
     float bad = 0.0f;  // NaN once a result is not finite
-    float z0v = cl.z0 > 0 ? wz[i - plane] : 0.0f, zcv = wz[i];  // w_z of planes z - 1, z
+    float zcv = wz[i], z0v = cl.z0 > 0 ? wz[i - plane] : zcv;  // w_z of planes z, z - 1
     for (int z = cl.z0; z < z1; ++z, i += plane) {
-        const float z2v = z + 1 < a.L ? wz[i + plane] : 0.0f;
-        const Axis ax = axis_x(a, c.boundary, x, i, N), az = axis_plain(z, a.L, plane);
-        const float d = gather3(ax, i, wx[i], [&](long long m) { return wx[m]; }) +
-                        gather3(ay, i, wy[i], [&](long long m) { return wy[m]; }) +
-                        fmaf(az.p, z2v, fmaf(az.c, zcv, az.m * z0v));
+        const float z2v = z + 1 < a.L ? wz[i + plane] : zcv;
+        const AxisX ax = axis_x(a, c.boundary, x, i, N);
+        const Axis az = axis_plain(z, a.L, plane);
+        const float d = gather_x(ax, ax.m != 0.0f ? wx[i - 1] : 0.0f, wx[i], ax.p != 0.0f ? wx[i + 1] : 0.0f) +
+                        fmaf(ay.p, wy[i + ay.r], ay.m * wy[i - ay.l]) + fmaf(az.p, z2v, az.m * z0v);
         const float v = a.out[i] + d;
         a.out[i] = v;
         bad = fmaf(v, 0.0f, bad);
