@@ -161,8 +161,9 @@ rsf_status rsf_evolve(rsf_workspace *ws, const rsf_params *p, const void *image,
                       float *phi, int64_t W, int64_t H, int64_t L, int32_t iters, void *stream);
 
 /* Evolves `n` independent sub-volumes of (possibly) different shapes in one
- * launch sequence per iteration, the iteration loop captured once into a
- * CUDA graph and replayed.  Replaces the one-process-per-sub-volume batch
+ * launch sequence per iteration; from four iterations on the loop is
+ * captured once into a CUDA graph and replayed.  Refused on a capturing
+ * stream.  Replaces the one-process-per-sub-volume batch
  * driver described at README.md:56 (rsfbatch.py, not in the reference). */
 rsf_status rsf_evolve_batched(rsf_workspace *ws, const rsf_params *p, rsf_dtype dtype,
                               const rsf_subvol *subvols, int32_t n, int32_t iters, void *stream);
