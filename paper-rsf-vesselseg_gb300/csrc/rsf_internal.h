@@ -30,8 +30,8 @@ constexpr int ZB_ZB = 16;      // and outputs per thread
 constexpr int ST_OX = 30;      // stencil: output columns per warp (lanes 1..30)
 constexpr int ST_OY = 14;      // stencil: output rows per block (warps 1..14)
 constexpr int ST_WARPS = ST_OY + 2;
-constexpr int ST_ZC = 64;      // stencil: planes per block (chosen per launch: 32, 64 or ST_ZC_MAX)
-constexpr int ST_ZC_MAX = 128;
+constexpr int ST_ZC_MAX = 128; // stencil: most planes per block (chosen per launch, choose_zc)
+constexpr int ST_ZC = 64;      // forced ones: ST_ZC / 2, ST_ZC or ST_ZC_MAX
 
 // The x-pass lane width (outputs per lane) is chosen per launch from these.
 constexpr int XB_CHOICES[2] = {5, 9};
@@ -113,12 +113,15 @@ constexpr unsigned kFlagNonFinite = 1u;  // a non-finite value was written to ph
 constexpr unsigned kFlagTimeout = 2u;    // a barrier wait gave up (a TMA copy did not complete)
 constexpr unsigned kFlagAdjointNonFinite = 4u;  // rsf_step_adjoint produced a non-finite dL/dphi
 
-// Tap counts with streaming (compile-time K) kernels: sigma 1.5, 2, 3, 4 and 5.
-// They load each input once and keep K accumulators, where the run-time-k kernels
-// run over a window per chunk of outputs: 256^3 voxels take 397 against 550 us per
-// iteration with 11 taps, 405 against 550 with 15; at 64^3 (25 us, latency) the two
-// are level.  Other tap counts, the debug step, the reference arithmetic and
-// the box e-term use the run-time-k kernels.
+// Tap counts with streaming (compile-time K) kernels: sigma 1.5, 2, 3, 4 and 5, the
+// blur widths of the configurations, the command line's default and the tests, each
+// with the range of sigma that gives the same count.  They load each input once and
+// keep K accumulators, where the run-time-k kernels run over a window per chunk of
+// outputs: 256^3 voxels take 397 against 550 us per iteration with 11 taps, 405
+// against 550 with 15; at 64^3 (25 us, latency) the two are level.  Any other odd
+// count up to 35 would gain as much; each costs four units of compile time.  The
+// debug step, the reference arithmetic, the box e-term and the Gaussian data term
+// use the run-time-k kernels for every count.
 inline bool is_specialised(int k) { return k == 11 || k == 15 || k == 21 || k == 29 || k == 35; }
 inline int kernel_k(int k, int arith, bool debug, int box = 0, int gauss = 0) {
     return (is_specialised(k) && arith == 0 && !debug && box == 0 && gauss == 0) ? k : 0;
@@ -157,8 +160,9 @@ constexpr size_t UPLOAD_BYTES = 2048;
 cudaError_t launch_upload(void *dst0, const void *src0, size_t bytes0, void *dst1, const void *src1, size_t bytes1,
                           cudaStream_t st);
 
-// One iteration; `first`: the tables may have been uploaded just before.  With `ev` (NKERN + 1 events) the events are recorded before
-// the first and after every kernel, for per-kernel device times.
+// One iteration; `first`: the tables may have been uploaded just before.  With
+// `ev` (NKERN + 1 events) the events are recorded before the first and after every
+// kernel, for per-kernel device times.
 cudaError_t launch_step(const SubVolDev *d_svs, const int *d_pre, const int *h_tot, const StepConst &c,
                         int parity, int arith, bool first, unsigned *d_flag, const DebugOut *dbg, cudaStream_t st,
                         cudaEvent_t *ev = nullptr);

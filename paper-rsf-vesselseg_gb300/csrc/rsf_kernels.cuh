@@ -35,8 +35,6 @@
 
 namespace rsf {
 
-enum { F_H = 0, F_HI = 1, F_IH = 2, F_IHI = 3 };  // field order in the x/y buffers
-
 __device__ __forceinline__ int find_sv(const int *__restrict__ pre, int n, int b) {
     int lo = 0, hi = n;
     while (hi - lo > 1) {
@@ -930,9 +928,15 @@ __device__ __forceinline__ void stencil_step(const StencilCtx &k, const StepCons
 // the sum by Knuth's two-sum), e_out and e_in in the two lanes of packed
 // instructions.  That gives the sum to within 2^-45 of its size, while the
 // double sequence is within 2^-52; where the two ends of a 2^-43 margin round
-// to the same float, that float is the reference's.  Elsewhere (one term in
-// 2^18) the z column is redone in double.  72x100x131 voxels, s = 1: 809 us per
-// launch in double, 60 so (67 with a grid row per plane).
+// to the same float, that float is the reference's.  Elsewhere the z column is
+// redone in double.  For s = 1 that is one column in 3000 to 4000 with fractional
+// fits (random values, restated on the CPU), but one in 15 where f = 1 meets an integer
+// image, in the border band: w d^2 is then whole for every third d, and most warps
+// go there.  With equal weights and a byte image the border needs no sum.
+// 72x100x131 voxels, half of them border, s = 1, a whole iteration: 1259 us with
+// the sums in double, 118 for bytes and equal weights (box kernel 60; 67 with a grid
+// row per plane), 377 with unequal weights or a float image of integers, 162 with a
+// fractional one.
 // ---------------------------------------------------------------------------
 // One z column of the box in double, from the sums before it.
 static __device__ __noinline__ float2 box_column_double(const void *img, size_t i, size_t step, int n, int f32,
