@@ -319,8 +319,10 @@ __device__ __forceinline__ Col col_of(const AdjVol &a, long long t, int zdepth) 
 // parameter sums are reduced in the block and added with one double atomic per
 // parameter and block (the same four addresses for every block, so their
 // number matters).  4 x 96x112x96 voxels: 227 us as two kernels with branches for
-// the face rules, 115 so (8 planes per block and 128 registers: 16 planes 122,
-// 4 planes 127; on one 43x58x67 volume 18.6, 11.2 and 8.0).
+// the face rules, 115 with three weights per axis, 100 so (the own value in a missing
+// neighbour's place along y and z; the gather after it 21 and 26).  Planes per block,
+// with three weights: 8 115 us, 16 122, 4 127; on one 43x58x67 volume 11.2, 18.6 and 8.0
+// (9.4 with 8 now).
 __global__ void __launch_bounds__(kBX * kBY, 2) adj_point(AdjConst c, const AdjVol *__restrict__ vols,
                                                        const int *__restrict__ pre,
                                                        double *grads) {

@@ -18,7 +18,7 @@ constexpr int YB_TX = 128;     // expanded data term's y kernel: columns per blo
 constexpr int YB_YB = 16;      // and outputs per thread
 constexpr int ZP_COLS = 128;   // z-pass: columns per block
 // z-pass: resident blocks per SM that its 4 K accumulator registers leave room
-// for (21 taps: 3.70 ms per launch on the 48-sub-volume batch with 4, 4.17 with
+// for (21 taps: 3.72 ms per launch on the 48-sub-volume batch with 4, 4.17 with
 // 3; 29 and 35 taps spill with 3: 771 against 1061 us on a 195 M voxel batch,
 // 1.02 against 1.45 ms on 512^3; 11 and 15 taps spill with 5, 3345 against 3313 us
 // on a batch of 15 taps)

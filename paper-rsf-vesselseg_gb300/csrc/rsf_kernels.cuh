@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(YP_COLS) ypass_chunk_kernel(const SubVolDev *_
 // cp.async.  The kernel is bound by instruction issue, and everything but the
 // multiply-adds is paid once per voxel this way (with the two pairs on
 // different lanes it took 186 thread instructions per voxel, 21 taps, and
-// 6.78 ms per launch on the 48 sub-volumes of 946 M voxels; now 3.70 ms).
+// 6.78 ms per launch on the 48 sub-volumes of 946 M voxels; now 3.72 ms).
 // The ring's depth divides the taps (7 for 21 and 35; K for 11, 15 and 29), so every
 // slot index of a K-element block is a constant; element i is commit group i,
 // and iteration i refills the slot of element i-1 with element i-1+RD before it

@@ -20,10 +20,10 @@
 //
 // Measured per launch on the 48 sub-volumes cut from 512 x 1024 x 1024 voxels:
 // 8.22 ms with one voxel per thread (32 warps per SM, 237 thread instructions
-// per voxel, 67 % issue), 5.64 ms here (24 warps, 80 registers, 160 and 67 %).
-// With phi loaded into registers one plane ahead it took 6.89 ms (long
-// scoreboard stalls behind every barrier), with four rows per thread and 16
-// warps 8.80 ms, with 64 registers and 32 warps 6.75 ms (spills).
+// per voxel, 67 % issue), 5.48 ms here (24 warps, 80 registers, 160 and 66 %).
+// With phi loaded into registers one plane ahead its first form (5.64 ms) took
+// 6.89 ms (long scoreboard stalls behind every barrier), with four rows per thread
+// and 16 warps 8.80 ms, with 64 registers and 32 warps 6.75 ms (spills).
 #pragma once
 #include "rsf_kernels.cuh"
 
@@ -129,16 +129,17 @@ __device__ __forceinline__ void pair_step(const PairCtx &k, const StepConst &c, 
     pair_fill<EDGE, FACE>(k, q, sc + SP_RING, C + half);
     q.a += k.WH;
     if (k.hwarp) q.h += k.WH;
-    // data factor of plane sc + 1, or the image in the border band
+    // data factor of plane sc + 1 (read once, so from L2: 5.48 ms per launch on the 48
+    // sub-volumes, 5.53 through L1), or the image in the border band
     float2 dn = make_float2(0.0f, 0.0f);
     if (INSIDE) {
-        if (k.out0) dn.x = *q.d;
-        if (k.out1) dn.y = q.d[k.dstep];
+        if (k.out0) dn.x = __ldcg(q.d);
+        if (k.out1) dn.y = __ldcg(q.d + k.dstep);
     } else if (!EDGE || (sc + 1 >= k.z0 && sc + 1 < k.z1)) {
         const bool zin = sc + 1 >= k.rz && sc + 1 < k.L - k.rz;
-        if (zin && k.val0) dn.x = *q.d;
+        if (zin && k.val0) dn.x = __ldcg(q.d);
         else if (k.out0) dn.x = border_word(q.i, c.img_f32);
-        if (zin && k.val1) dn.y = q.d[k.dstep];
+        if (zin && k.val1) dn.y = __ldcg(q.d + k.dstep);
         else if (k.out1) dn.y = border_word(q.i + k.istep, c.img_f32);
     }
     q.d += k.dplane;
