@@ -120,8 +120,9 @@ int choose_xrpw(const int *whl, int n, int k, int xb_w) {
 // the axis.
 template <class Cols, class Ext>
 static int choose_cut(int n, int k, long long want, Cols cols, Ext ext) {
-    int deepest = 0;
-    for (int i = 0; i < n; i++) deepest = ext(i) - k + 1 > deepest ? ext(i) - k + 1 : deepest;
+    int deepest = 0;  // of the volumes that have columns
+    for (int i = 0; i < n; i++)
+        if (cols(i) > 0 && ext(i) - k + 1 > deepest) deepest = ext(i) - k + 1;
     if (deepest < 1) return 1;
     for (int cuts = 1;; cuts++) {
         const int out = (deepest + cuts - 1) / cuts;
