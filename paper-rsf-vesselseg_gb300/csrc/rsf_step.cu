@@ -117,7 +117,9 @@ int choose_xrpw(const int *whl, int n, int k, int xb_w) {
 // per cut and pays only where the batch leaves the SMs short of warps: the
 // fewest cuts that give `want` blocks, as long as a cut is no shorter than the
 // taps.  cols(i): a volume's columns of one block each; ext(i): its extent along
-// the axis.
+// the axis.  Volumes without columns take no part: they never add blocks, and the
+// extent of a long thin one kept the search going (2^20 x 2 x 2 voxels, 21 taps: 0.23
+// ms of host time per call, 0.87 beside a small valid volume; 0.014 and 0.019 so).
 template <class Cols, class Ext>
 static int choose_cut(int n, int k, long long want, Cols cols, Ext ext) {
     int deepest = 0;  // of the volumes that have columns
