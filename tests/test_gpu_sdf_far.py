@@ -71,14 +71,17 @@ def _time(ws, seed, reps=7):
     return min(times)
 
 
-@pytest.mark.parametrize("kind", ["zy", "zyx", "one", "z"])
-def test_time_does_not_follow_the_distance(kind, cuda, rsflib):
-    """A plane far away took 14 times as long as noise where the search went on row by row."""
+@pytest.mark.parametrize("axes", ["zy", "zyx"])
+def test_time_does_not_follow_the_distance(axes, cuda, rsflib):
+    """A volume cut in two by a slanted plane against noise, whose every voxel is near: 3 times its time; 5 (zy) and
+    7 times (zyx) where the search went on row by row."""
     from rsf_gb300 import Workspace
 
-    shape = (320, 320, 320)
-    near = (torch.rand(shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)) < 0.5)
-    far = torch.from_numpy(_inside(kind, shape)).cuda()
-    with Workspace(near.numel()) as ws:
-        t = [_time(ws, (m.to(torch.uint8) * 200)) for m in (near, far)]
-    assert t[1] <= 6.0 * t[0], t
+    n = 500
+    at = torch.arange(n, device="cuda", dtype=torch.int16)
+    far = at[:, None, None] + at[None, :, None] + (at[None, None, :] if axes == "zyx" else at[None, None, :] * 0)
+    far = (far < n * len(axes) // 2).to(torch.uint8).mul_(200)
+    near = (torch.rand((n, n, n), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)) < 0.5)
+    with Workspace(n ** 3) as ws:
+        t = [_time(ws, m) for m in (near.to(torch.uint8).mul_(200), far)]
+    assert t[1] <= 4.5 * t[0], t
