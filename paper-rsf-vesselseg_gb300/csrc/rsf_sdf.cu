@@ -33,10 +33,10 @@
 // algorithm", Algorithmica 2, 1987), so a group of rows between two finished
 // groups searches only the rows between their results.  That bounds the work per
 // voxel whatever the seeds are, as the envelope's is.  256 x 448 x 512 voxels:
-// winding vessels 3.84 ms with the envelopes, 0.87 here; an empty seed 2.04 and
-// 1.38; a slanted plane 2.70 and 1.48 (3.94 with the search alone, blocks of 16 rows
+// winding vessels 3.84 ms with the envelopes, 0.82 here; an empty seed 2.04 and
+// 1.32; a slanted plane 2.70 and 1.40 (3.94 with the search alone, blocks of 16 rows
 // skipped where their smallest value cannot improve; on 500^3 9.5 ms, 4.7 with the
-// envelopes, 3.7 here); sparse noise (1e-3) 2.65 and 1.36.
+// envelopes, 3.3 here); sparse noise (1e-3) 2.65 and 1.27.
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -408,12 +408,16 @@ __global__ void __launch_bounds__(T) sdf_cols_tile(TileArgs a) {
 
 size_t tile_smem(int n) { return 128 * (size_t)n + 64 * ((size_t)(n + 3) / 4); }
 
-// 256 threads share an SM three or more times up to about 500 rows; longer
-// columns leave one or two blocks, which then bring 512.
-constexpr int kWideFrom = 560;
+// Threads per block.  Three blocks share an SM at about 500 rows, and with 256
+// threads leave it half of its warps: 256 x 448 x 512 voxels of winding vessels take 874
+// us with 256 threads for the 448 rows, 818 with 512; 500^3 1897 and 1737, a single
+// corner voxel there 3605 and 3396.  At 300 rows and below eight or more blocks of
+// 256 fill it, and 512 threads share too few groups: 256^3 cut by a slanted plane 427 us
+// and 486.
+constexpr int kWideFrom = 400;
 
-// TRY and FINE, by winding vessels (the first figure) and planes (the second): 4 and 24
-// take 0.87 and 1.45 ms on 256 x 448 x 512 voxels, 8 and 48 0.86 and 1.72.  In short
+// TRY and FINE, by winding vessels (the first figure) and planes (the second), with 256
+// threads: 4 and 24 take 0.87 and 1.45 ms on 256 x 448 x 512 voxels, 8 and 48 0.86 and 1.72.  In short
 // columns the halving's levels, one after the other, are latency: 128^3 takes 76 and
 // 125 us with 4 and 24, 69 and 177 with 8 and 48, 96^3 54 and 75, 49 and 94.
 template <bool FINAL>
